@@ -26,34 +26,34 @@ from meshhashing_gb300 import scene as scenes
 from meshhashing_gb300.pose import left_update
 
 TV_LAMBDA = 0.1
-WINDOW = 8          # frames a fusing case cycles through once its map is built
 
 
 # ------------------------------------------------------------------ the cases
 
 def listed():
+    # A scan is a whole pass of a scanner from an empty map: every frame through the chain (denoising, allocation,
+    # fusion, meshing, garbage collection, the model's image), then the counts that the program looks at.
     return [
         # a small plain-TSDF sensor (a robot's ToF camera): launches and latency
-        dict(name="fuse_tsdf_160", kind="fuse", mode="tsdf", plan=False, width=160, height=120, voxel=0.008, fused=30,
+        dict(name="scan_tsdf_160", kind="scan", mode="tsdf", plan=False, width=160, height=120, voxel=0.008, frames=15,
              tv=0, host=False, maps="depth"),
-        # the smallest camera of the batched-fusion workload, alone
-        dict(name="fuse_psdf_160", kind="fuse", mode="psdf", plan=False, width=160, height=120, voxel=0.006, fused=48,
-             tv=20, host=False, maps="depth"),
-        # a ragged image from host memory, every map read back to the host
-        dict(name="fuse_psdf_322_host", kind="fuse", mode="psdf", plan=False, width=322, height=238, voxel=0.006,
-             fused=64, tv=20, host=True, maps="all"),
-        # the PSDF workload's frame: 640x480, 4 mm, frames in device memory
-        dict(name="fuse_psdf_640", kind="fuse", mode="psdf", plan=False, width=640, height=480, voxel=0.004, fused=96,
+        # the plain TSDF workload: 320x240, the circle, 8 mm
+        dict(name="scan_tsdf_320", kind="scan", mode="tsdf", plan=False, width=320, height=240, voxel=0.008, frames=45,
+             tv=0, host=False, maps="all"),
+        # a ragged image from host memory, every map read back to the host, long enough for the surfaces to be meshed
+        dict(name="scan_psdf_322_host", kind="scan", mode="psdf", plan=False, width=322, height=238, voxel=0.008,
+             frames=60, tv=20, host=True, maps="all"),
+        # the PSDF workload: 640x480, 4 mm, frames in device memory
+        dict(name="scan_psdf_640", kind="scan", mode="psdf", plan=False, width=640, height=480, voxel=0.004, frames=48,
              tv=20, host=False, maps="all"),
         # the streaming walk through a floor plan, frames from and depth to pinned host memory
-        dict(name="fuse_plan_640_host", kind="fuse", mode="psdf", plan=True, width=640, height=480, voxel=0.005,
-             fused=64, tv=20, host=True, maps="depth"),
-        # a whole short scan from an empty map: the plain TSDF workload (320x240, circle, 8 mm)
-        dict(name="scan_tsdf_320", kind="scan", width=320, height=240, voxel=0.008, frames=40),
-        # many small and middling scenes advanced together
-        dict(name="batch_16", kind="batch", scenes=16, fused=8, tv=20),
-        # a viewer: the map of a 640x480 sequence from poses off its path
+        dict(name="scan_plan_640_host", kind="scan", mode="psdf", plan=True, width=640, height=480, voxel=0.005,
+             frames=32, tv=20, host=True, maps="depth"),
+        # many small and middling scenes advanced together, from empty maps
+        dict(name="batch_16", kind="batch", scenes=16, frames=12, tv=20),
+        # a viewer: the map of a 640x480 sequence from poses off its path, and a thumbnail of one
         dict(name="render_640", kind="render", width=640, height=480, voxel=0.004, fused=40),
+        dict(name="render_161", kind="render", width=161, height=119, voxel=0.008, fused=30),
         # pose and voxel gradients through the renderer, forward and backward
         dict(name="gradient_320", kind="gradient", width=320, height=240, voxel=0.008, fused=24),
         # frame-to-model tracking: 10 Gauss-Newton iterations from a perturbed pose
@@ -70,24 +70,23 @@ def _log(rng, lo, hi):
 
 
 def draw(rng):
-    kind = rng.choice(("fuse", "fuse", "fuse", "scan", "batch", "render", "gradient", "track", "smooth", "denoise"))
+    kind = rng.choice(("scan", "scan", "scan", "scan", "batch", "render", "render", "gradient", "track", "smooth",
+                       "denoise"))
     width = int(_log(rng, 96, 641))
     height = max(72, min(480, int(width * rng.uniform(0.6, 0.8))))
     # 4 mm at every size; coarser voxels up to 8 mm
     voxel = round(_log(rng, 0.004, 0.008), 5)
-    if kind == "fuse":
+    if kind == "scan":
         mode = rng.choice(("psdf", "psdf", "tsdf"))
         host = rng.random() < 0.4
         if host:                # host images have even sides
             width, height = width - width % 2, height - height % 2
         return dict(kind=kind, mode=mode, plan=mode == "psdf" and rng.random() < 0.3, width=width, height=height,
-                    voxel=voxel, fused=rng.randint(8, 80), tv=rng.choice((0, 5, 20, 23)) if mode == "psdf" else 0,
-                    host=host, maps=rng.choice(("depth", "all")))
-    if kind == "scan":
-        return dict(kind=kind, width=min(width, 321), height=min(height, 241), voxel=max(voxel, 0.006),
-                    frames=rng.randint(12, 40))
+                    voxel=voxel if mode == "psdf" else max(voxel, 0.006), frames=rng.randint(6, 40),
+                    tv=rng.choice((0, 5, 20, 23)) if mode == "psdf" else 0, host=host,
+                    maps=rng.choice(("depth", "all")))
     if kind == "batch":
-        return dict(kind=kind, scenes=rng.randint(3, 16), fused=rng.randint(3, 8), tv=rng.choice((0, 20)))
+        return dict(kind=kind, scenes=rng.randint(3, 16), frames=rng.randint(4, 12), tv=rng.choice((0, 20)))
     if kind == "denoise":
         return dict(kind=kind, width=width, height=height, iterations=rng.randint(3, 30))
     case = dict(kind=kind, width=width, height=height, voxel=max(voxel, 0.006) if kind != "render" else voxel,
@@ -101,24 +100,27 @@ def work(case):
     """Bytes that a pass cannot do without.  Blocks in view are estimated from
     the view's volume and the share of it that the outliers have allocated."""
     if case["kind"] == "batch":
-        parts = [work(dict(kind="fuse", mode="psdf", maps="all", fused=case["fused"], **s)) for s in _mix(case["scenes"])]
+        parts = [work(dict(kind="scan", mode="psdf", maps="all", frames=case["frames"], **c)) for c in _mix(case["scenes"])]
         return {k: sum(p[k] for p in parts) for k in ("bytes", "flops")}
     px = case["width"] * case["height"]
     if case["kind"] == "denoise":
         return {"bytes": 8.0 * px, "flops": 30.0 * px * case["iterations"]}
-    tsdf = case["kind"] == "scan" or case.get("mode") == "tsdf"
-    frames = case.get("fused", 1)
+    tsdf = case.get("mode") == "tsdf"
     block = (8 * case["voxel"]) ** 3
     surface = 6.0 * 3 / (8 * case["voxel"]) ** 2
     volume = 7.0 / block                  # between the camera and the surface
-    blocks = surface if tsdf else surface + volume * (1.0 - math.exp(-frames * 0.05 * px / volume))
-    fuse = blocks * 512 * (16 if tsdf else 32) + px * 8
+
+    def seen(frames):
+        return surface if tsdf else surface + volume * (1.0 - math.exp(-frames * 0.05 * px / volume))
+
     images = px * (4 if case.get("maps") == "depth" else 36)
     look = surface * (2048 + 16)          # the blocks at the surface that an image shows
-    if case["kind"] == "fuse":
-        return {"bytes": fuse + look + images, "flops": blocks * 512 * 60.0 + px * 2000.0}
     if case["kind"] == "scan":
-        return {"bytes": case["frames"] * (fuse + look + px * 4.0), "flops": case["frames"] * (blocks * 30720.0 + px * 500.0)}
+        n = case["frames"]
+        blocks = sum(seen(k + 1) for k in range(n))
+        return {"bytes": blocks * 512 * (16 if tsdf else 32) + n * (px * 8 + look + images),
+                "flops": blocks * 512 * 60.0 + n * px * 2000.0}
+    blocks = seen(case["fused"])
     if case["kind"] == "render":
         return {"bytes": look + images, "flops": px * 2000.0}
     if case["kind"] == "gradient":
@@ -127,8 +129,8 @@ def work(case):
         n = case["iterations"] + 1
         return {"bytes": n * (look + px * 4.0), "flops": n * px * 2000.0}
     # smooth: per observed voxel and iteration sdf, sdf_bar and the dual, read and written, the weight and sdf0 read
-    seen = blocks * 512
-    return {"bytes": case["iterations"] * seen * 48.0 + look + images, "flops": case["iterations"] * seen * 60.0}
+    voxels = blocks * 512
+    return {"bytes": case["iterations"] * voxels * 48.0 + look + images, "flops": case["iterations"] * voxels * 60.0}
 
 
 # ------------------------------------------------------------------ inputs
@@ -183,7 +185,7 @@ def _camera(width, height):
 def _sequence(case, seed, n):
     """n frames (on the device) and their poses; a TSDF case's camera goes round a circle of 60 frames."""
     cam = _camera(case["width"], case["height"])
-    if case["kind"] == "scan" or case.get("mode") == "tsdf":
+    if case.get("mode") == "tsdf":
         sc, poses = scenes.room_scene(seed), scenes.circle_trajectory(60)
         first = seed % 60
         poses = [poses[(first + i) % 60] for i in range(n)]
@@ -200,11 +202,11 @@ def _sequence(case, seed, n):
 def _volume(case, cam, frames):
     """A volume whose pools hold what `frames` frames of this size allocate (with a margin)."""
     v = case["voxel"]
-    if case["kind"] == "scan" or case.get("mode") == "tsdf":
+    if case.get("mode") == "tsdf":
         cap = int(2 ** 17 * max(1.0, (0.008 / v) ** 2))
         return Volume(config.make_params(cam.width, cam.height, cam.fx, cam.fy, cam.cx, cam.cy, voxel_size=v,
                                          truncation=3 * v, bayesian=False, bucket_count=1 << 18, value_capacity=cap,
-                                         weight_sample=200, max_vertex_count=1 << 21, max_triangle_count=1 << 21))
+                                         weight_sample=200, max_vertex_count=1 << 21, max_triangle_count=1 << 22))
     k = 53108.0 * (cam.width * cam.height / 307200.0) ** 0.62 * (0.004 / v) ** 1.4
     cap = int(1.8 * k * frames ** 0.62) // 1024 * 1024 + 8192
     buckets = 1 << max(14, (cap - 1).bit_length())
@@ -263,20 +265,16 @@ def _inverse(T):
 def prepare(case, seed):
     kind = case["kind"]
     rng = np.random.default_rng(seed)
-    if kind == "fuse":
-        s = _fused(case, seed, WINDOW)
-        s.host = case["host"]
-        s.images = _images(case, s.cam, s.host)
-        s.frames = [f.cpu().pin_memory() if s.host else f for f in s.frames]
-        s.at = 0
-    elif kind == "scan":
+    if kind == "scan":
         s = State()
-        s.cam, s.frames, s.poses = _sequence(case, seed, case["frames"])
+        s.cam, frames, s.poses = _sequence(case, seed, case["frames"])
         s.vol = _volume(case, s.cam, case["frames"])
-        s.images = _images(dict(maps="all"), s.cam, False)
+        s.host, s.tv = case["host"], case["tv"]
+        s.images = _images(case, s.cam, s.host)
+        s.frames = [f.cpu().pin_memory() if s.host else f for f in frames]
     elif kind == "batch":
         s = State()
-        n, total = case["scenes"], case["fused"] + 4
+        n, total = case["scenes"], case["frames"]
         vols, s.frames, s.poses = [], [], []
         for i, spec in enumerate(_mix(n)):
             c = dict(kind="batch", **spec)
@@ -290,9 +288,7 @@ def prepare(case, seed):
             shapes = ((v.RH, v.RW), (v.RH, v.RW, 4), (v.RH, v.RW, 4))
             s.views.append([torch.as_tensor(_View(s.batch, p, sh), device="cuda")
                             for p, sh in zip(s.batch.outputs(i), shapes)])
-        s.tv, s.at, s.first = case["tv"], 0, case["fused"]
-        for k in range(case["fused"]):
-            _step(s, k)
+        s.tv, s.count = case["tv"], total
     elif kind == "render":
         s = _fused(case, seed)
         # off the path by a few centimetres and degrees
@@ -339,29 +335,21 @@ def prepare(case, seed):
 
 # ------------------------------------------------------------------ one pass
 
-def _step(s, k):
-    s.batch.step([f[k] for f in s.frames], [p[k] for p in s.poses], on_device=True, tv_iterations=s.tv,
-                 tv_lambda=TV_LAMBDA, use_graph=True)
-
-
 def run(s):
-    if s.kind == "fuse":
-        k = s.at % WINDOW
-        s.at += 1
-        s.vol.integrate_frame(s.frames[k], s.poses[k], on_device=not s.host, tv_iterations=s.tv, tv_lambda=TV_LAMBDA,
-                              outputs_on_device=not s.host, **s.images)
-        return s.images
     if s.kind == "scan":
         s.vol.reset()
         for f, T in zip(s.frames, s.poses):
-            s.vol.integrate_frame(f, T, on_device=True, outputs_on_device=True, **s.images)
+            s.vol.integrate_frame(f, T, on_device=not s.host, tv_iterations=s.tv, tv_lambda=TV_LAMBDA,
+                                  outputs_on_device=not s.host, **s.images)
         st = s.vol.stats()
         return dict(s.images, blocks=st["blocks_allocated"], vertices=st["vertices_allocated"],
                     triangles=st["triangles_allocated"], error=st["error"])
     if s.kind == "batch":
-        k = s.first + s.at % 4
-        s.at += 1
-        _step(s, k)
+        for v in s.batch.volumes:
+            v.reset()
+        for k in range(s.count):
+            s.batch.step([f[k] for f in s.frames], [p[k] for p in s.poses], on_device=True, tv_iterations=s.tv,
+                         tv_lambda=TV_LAMBDA, use_graph=True)
         return s.views
     if s.kind == "render":
         im = s.images
@@ -558,7 +546,7 @@ def _picture(cam, ray, x, last=None):
 
 
 def exact(case, seed):
-    """Fused frames and tracked poses have no such value: they follow from a long chain of single-precision decisions."""
+    """Scans and tracked poses have no such value: they follow from a long chain of single-precision decisions."""
     if case["kind"] in ("render", "gradient"):
         s = prepare(case, seed)
         mp = _Map(s.vol, ("sdf",))
