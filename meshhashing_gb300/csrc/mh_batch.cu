@@ -135,6 +135,7 @@ static int enqueue(mh_batch *b, int p, bool host_depth, int tv_it, float lambda,
   if ((r = launch_batch_gc_recycle(t, n, 0, s)) != MH_OK) return r;
   mark(MH_STAGE_RAYCAST);
   if (b->raycast) {
+    if ((r = launch_batch_ray_grid(t, n, s)) != MH_OK) return r;
     if (timed) cudaEventRecord(b->ev[2], s);
     if ((r = launch_raycast_batch(t, n, b->ray_tiles(b->tune.ray_tile_shape, nullptr), b->tune.ray_tile_shape, s)) !=
         MH_OK)
@@ -315,7 +316,6 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
     const bool act = !active || active[i];
     sc.d = v->d;
     sc.d.fc = d_fc + i;
-    sc.d.cellok = nullptr;  // the batched raycast runs without the per-block cell flags
     sc.tv = v->tv;
     sc.ray_depth = b->out_depth[i];
     sc.ray_vert = reinterpret_cast<float4 *>(b->out_vert[i]);
@@ -347,6 +347,7 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
     inverse4(fc.rc_cTw, fc.rc_wTc);
     v->fc_host = fc;
     v->has_frame = true;
+    if (b->raycast) sc.d.grid = ray_grid_for(v->hp, fc.rc_wTc, v->grid);
   }
   const bool host_depth = !depth_on_device;
   if (use_graph && !tuning) {

@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(256) k_pd_primal(Dev d, PD pd, const int *nbt,
     s = (s + lam * tau * s0) / (1.0f + lam * tau);
     if (w > 2.0f) s = s0;
     d.sdf[g] = s;
-    const int dpos = sdf_nonneg(s) - sdf_nonneg(prev);
-    if (dpos) atomicAdd(d.nnc + blk, dpos);
+    if (!sdf_nonneg(s) && sdf_nonneg(prev))
+      atomicOr(d.neg + blk, 1ull << (((li >> 1) & 3) | ((li >> 2) & 12) | ((li >> 3) & 48)));
     pd.bar[g] = 2.0f * s - prev;
   }
 }

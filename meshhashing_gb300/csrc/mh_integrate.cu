@@ -59,6 +59,13 @@ __device__ __forceinline__ void note_wmax(const Dev &d, int blk, float w) {
   if ((int)lane_id() == __ffs(act) - 1 && m) atomicMax(reinterpret_cast<unsigned *>(d.wmax + blk), m);
 }
 
+// The block's mask (neg) for the two z layers that this warp of a 128-thread
+// CTA holds: 16 bits of its own, so no other warp's bits are written.
+__device__ __forceinline__ void note_neg(const Dev &d, int blk, const float4 &S) {
+  const unsigned bits = neg_bits(S);
+  if (lane_id() == 0) reinterpret_cast<uint16_t *>(d.neg + blk)[threadIdx.x >> 5] = (uint16_t)bits;
+}
+
 }  // namespace
 
 // UpdateBlocksSimpleKernel + Voxel::Update (core/voxel.h:107-115)
@@ -99,24 +106,26 @@ __device__ __forceinline__ void integrate_simple_body(const Dev &d) {
       act[k] = true;
       any = true;
     }
-    if (!any) continue;
+    // a warp that updates anything reads all its sdf: the block's mask of
+    // voxels that are not non-negative is rewritten for its two layers
+    if (!__any_sync(0xffffffffu, any)) continue;
     const size_t base = (size_t)cb.w * MH_BLOCK_VOXELS + t * 4;
     float4 S = *reinterpret_cast<const float4 *>(d.sdf + base);
-    float4 W = *reinterpret_cast<const float4 *>(d.w + base);
-    int dpos = 0;
+    if (any) {
+      float4 W = *reinterpret_cast<const float4 *>(d.w + base);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!act[k]) continue;
-      const float s0 = get(S, k), w0 = get(W, k);
-      const float s1 = (s0 * w0 + sdf_new[k] * w_new[k]) / (w0 + w_new[k]);
-      dpos += sdf_nonneg(s1) - sdf_nonneg(s0);
-      put(S, k, s1);
-      put(W, k, w0 + w_new[k]);
+      for (int k = 0; k < 4; ++k) {
+        if (!act[k]) continue;
+        const float s0 = get(S, k), w0 = get(W, k);
+        put(S, k, (s0 * w0 + sdf_new[k] * w_new[k]) / (w0 + w_new[k]));
+        put(W, k, w0 + w_new[k]);
+      }
+      *reinterpret_cast<float4 *>(d.sdf + base) = S;
+      *reinterpret_cast<float4 *>(d.w + base) = W;
+      note_wmax(d, cb.w, fmaxf(fmaxf(W.x, W.y), fmaxf(W.z, W.w)));
     }
-    *reinterpret_cast<float4 *>(d.sdf + base) = S;
-    *reinterpret_cast<float4 *>(d.w + base) = W;
-    note_wmax(d, cb.w, fmaxf(fmaxf(W.x, W.y), fmaxf(W.z, W.w)));
-    note_nnc(d, cb.w, dpos);
+    __syncwarp();
+    note_neg(d, cb.w, S);
   }
 }
 __global__ void __launch_bounds__(128) k_integrate_simple(Dev d) { integrate_simple_body(d); }
@@ -160,93 +169,95 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
       act[k] = true;
       any = true;
     }
-    if (!any) continue;
+    if (!__any_sync(0xffffffffu, any)) continue;
     const size_t base = (size_t)cb.w * MH_BLOCK_VOXELS + t * 4;
     float4 S = *reinterpret_cast<const float4 *>(d.sdf + base);
-    float4 W = *reinterpret_cast<const float4 *>(d.w + base);
-    float4 A = *reinterpret_cast<const float4 *>(d.a + base);
-    float4 B = *reinterpret_cast<const float4 *>(d.b + base);
-    const int pos_before = sdf_nonneg(S.x) + sdf_nonneg(S.y) + sdf_nonneg(S.z) + sdf_nonneg(S.w);
+    if (any) {
+      float4 W = *reinterpret_cast<const float4 *>(d.w + base);
+      float4 A = *reinterpret_cast<const float4 *>(d.a + base);
+      float4 B = *reinterpret_cast<const float4 *>(d.b + base);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!act[k]) continue;
-      const float x = xs[k], r = rho[k], dd = dep[k];
-      const float tau = (dd - 0.4f) * 0.012f + 0.019f;
-      const float w0 = get(W, k);
-      if (w0 == 0.0f) {
-        put(S, k, x);
-        put(W, k, 1.0f / (tau * tau));
-        put(A, k, r * 10.0f);
-        put(B, k, (1.0f - r) * 10.0f);
-        continue;
+      for (int k = 0; k < 4; ++k) {
+        if (!act[k]) continue;
+        const float x = xs[k], r = rho[k], dd = dep[k];
+        const float tau = (dd - 0.4f) * 0.012f + 0.019f;
+        const float w0 = get(W, k);
+        if (w0 == 0.0f) {
+          put(S, k, x);
+          put(W, k, 1.0f / (tau * tau));
+          put(A, k, r * 10.0f);
+          put(B, k, (1.0f - r) * 10.0f);
+          continue;
+        }
+        const float mu = get(S, k);
+        const float a = get(A, k), b = get(B, k);
+        const float t2 = tau * tau;
+        const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
+        if (p.compat) {
+          // the reference's expressions as written (update_bayesian.cu:140-180);
+          // sqrt(2 pi) is a double there, so the product and the reciprocal of
+          // gaussian() are double (geometry_helper.h:30-34)
+          const float s2 = 1.0f / w0;
+          const float ss2 = 1.0f / (1.0f / s2 + 1.0f / t2);
+          const float m = ss2 * (mu / s2 + x / t2);
+          const float sv = s2 + t2;
+          const double g = 1.0 / (2.5066282746310002 * (double)sqrtf(sv)) * (double)expf(-((x - mu) * (x - mu)) / sv);
+          float C1 = (float)((double)r * g);
+          float C2 = in_range ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : 1.0f;
+          const float sum = C1 + C2;
+          C1 /= sum;
+          C2 /= sum;
+          const float f = C1 * (a + 1) / (a + b + 1) + C2 * a / (a + b + 1);
+          const float e =
+              C1 * (a + 1) * (a + 2) / ((a + b + 1) * (a + b + 2)) + C2 * a * (a + 1) / ((a + b + 1) * (a + b + 2));
+          const float nsdf = C1 * m + C2 * mu;
+          const float var = C1 * (ss2 + m * m) + C2 * (s2 + mu * mu) - nsdf * nsdf;
+          put(S, k, nsdf);
+          put(W, k, 1.0f / var);
+          const float na = (e - f) / (f - e / f);
+          put(A, k, na);
+          put(B, k, na * (1.0f - f) / f);
+          continue;
+        }
+        // The same update with 4 divisions instead of 21.  With the stored
+        // weight w0 = 1/s^2 and u = w0 sigma^2, q = 1/(1 + u):
+        //   the product's variance s~^2 = sigma^2 q, its mean m = q (mu u + x),
+        //   1/(s^2 + sigma^2) = w0 q, so gaussian() = exp(-dx^2 w0 q) sqrt(w0 q) / sqrt(2 pi);
+        //   c = C1 / (C1 + C2) is the normalised inlier weight, 1 - c the outlier's;
+        //   sdf' = mu + c (m - mu);
+        //   the variance c s~^2 + (1 - c) s^2 + c (1 - c)(m - mu)^2 (the
+        //   reference's C1 (s~^2 + m^2) + C2 (s^2 + mu^2) - sdf'^2 without its
+        //   cancellation) gives w' = w0 / (c u q + (1 - c) + c (1 - c)(m - mu)^2 w0);
+        //   the Beta moments f, e of the reference give a' = f (e - f) / (f^2 - e)
+        //   = (a + c) k and b' = a' (1 - f) / f = (b + 1 - c) k with
+        //   k = (c (a - b) - a (b + 1)) / (c^2 (a + b + 2) - (a + 2c)(b + 1)),
+        //   which cancels far less than f^2 - e.
+        const float u = w0 * t2;
+        const float q = 1.0f / (1.0f + u);
+        const float m = q * (mu * u + x);
+        const float isv = w0 * q;
+        const float dx = x - mu;
+        const float g = mh_expf(-(dx * dx) * isv) * sqrtf(isv) * 0.398942280401432678f;
+        const float C1 = r * g;
+        const float C2 = in_range ? (1.0f - r) * 0.204081632653061224f : 1.0f;
+        const float c = C1 / (C1 + C2);
+        const float oc = 1.0f - c;
+        const float dm = m - mu;
+        put(S, k, mu + c * dm);
+        put(W, k, w0 / (c * u * q + oc + c * oc * (dm * dm) * w0));
+        const float b1 = b + 1.0f;
+        const float kk = (c * (a - b) - a * b1) / (c * c * (a + b + 2.0f) - (a + 2.0f * c) * b1);
+        put(A, k, (a + c) * kk);
+        put(B, k, (b1 - c) * kk);
       }
-      const float mu = get(S, k);
-      const float a = get(A, k), b = get(B, k);
-      const float t2 = tau * tau;
-      const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
-      if (p.compat) {
-        // the reference's expressions as written (update_bayesian.cu:140-180);
-        // sqrt(2 pi) is a double there, so the product and the reciprocal of
-        // gaussian() are double (geometry_helper.h:30-34)
-        const float s2 = 1.0f / w0;
-        const float ss2 = 1.0f / (1.0f / s2 + 1.0f / t2);
-        const float m = ss2 * (mu / s2 + x / t2);
-        const float sv = s2 + t2;
-        const double g = 1.0 / (2.5066282746310002 * (double)sqrtf(sv)) * (double)expf(-((x - mu) * (x - mu)) / sv);
-        float C1 = (float)((double)r * g);
-        float C2 = in_range ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : 1.0f;
-        const float sum = C1 + C2;
-        C1 /= sum;
-        C2 /= sum;
-        const float f = C1 * (a + 1) / (a + b + 1) + C2 * a / (a + b + 1);
-        const float e =
-            C1 * (a + 1) * (a + 2) / ((a + b + 1) * (a + b + 2)) + C2 * a * (a + 1) / ((a + b + 1) * (a + b + 2));
-        const float nsdf = C1 * m + C2 * mu;
-        const float var = C1 * (ss2 + m * m) + C2 * (s2 + mu * mu) - nsdf * nsdf;
-        put(S, k, nsdf);
-        put(W, k, 1.0f / var);
-        const float na = (e - f) / (f - e / f);
-        put(A, k, na);
-        put(B, k, na * (1.0f - f) / f);
-        continue;
-      }
-      // The same update with 4 divisions instead of 21.  With the stored
-      // weight w0 = 1/s^2 and u = w0 sigma^2, q = 1/(1 + u):
-      //   the product's variance s~^2 = sigma^2 q, its mean m = q (mu u + x),
-      //   1/(s^2 + sigma^2) = w0 q, so gaussian() = exp(-dx^2 w0 q) sqrt(w0 q) / sqrt(2 pi);
-      //   c = C1 / (C1 + C2) is the normalised inlier weight, 1 - c the outlier's;
-      //   sdf' = mu + c (m - mu);
-      //   the variance c s~^2 + (1 - c) s^2 + c (1 - c)(m - mu)^2 (the
-      //   reference's C1 (s~^2 + m^2) + C2 (s^2 + mu^2) - sdf'^2 without its
-      //   cancellation) gives w' = w0 / (c u q + (1 - c) + c (1 - c)(m - mu)^2 w0);
-      //   the Beta moments f, e of the reference give a' = f (e - f) / (f^2 - e)
-      //   = (a + c) k and b' = a' (1 - f) / f = (b + 1 - c) k with
-      //   k = (c (a - b) - a (b + 1)) / (c^2 (a + b + 2) - (a + 2c)(b + 1)),
-      //   which cancels far less than f^2 - e.
-      const float u = w0 * t2;
-      const float q = 1.0f / (1.0f + u);
-      const float m = q * (mu * u + x);
-      const float isv = w0 * q;
-      const float dx = x - mu;
-      const float g = mh_expf(-(dx * dx) * isv) * sqrtf(isv) * 0.398942280401432678f;
-      const float C1 = r * g;
-      const float C2 = in_range ? (1.0f - r) * 0.204081632653061224f : 1.0f;
-      const float c = C1 / (C1 + C2);
-      const float oc = 1.0f - c;
-      const float dm = m - mu;
-      put(S, k, mu + c * dm);
-      put(W, k, w0 / (c * u * q + oc + c * oc * (dm * dm) * w0));
-      const float b1 = b + 1.0f;
-      const float kk = (c * (a - b) - a * b1) / (c * c * (a + b + 2.0f) - (a + 2.0f * c) * b1);
-      put(A, k, (a + c) * kk);
-      put(B, k, (b1 - c) * kk);
+      *reinterpret_cast<float4 *>(d.sdf + base) = S;
+      *reinterpret_cast<float4 *>(d.w + base) = W;
+      *reinterpret_cast<float4 *>(d.a + base) = A;
+      *reinterpret_cast<float4 *>(d.b + base) = B;
+      note_wmax(d, cb.w, fmaxf(fmaxf(W.x, W.y), fmaxf(W.z, W.w)));
     }
-    *reinterpret_cast<float4 *>(d.sdf + base) = S;
-    *reinterpret_cast<float4 *>(d.w + base) = W;
-    *reinterpret_cast<float4 *>(d.a + base) = A;
-    *reinterpret_cast<float4 *>(d.b + base) = B;
-    note_wmax(d, cb.w, fmaxf(fmaxf(W.x, W.y), fmaxf(W.z, W.w)));
-    note_nnc(d, cb.w, sdf_nonneg(S.x) + sdf_nonneg(S.y) + sdf_nonneg(S.z) + sdf_nonneg(S.w) - pos_before);
+    __syncwarp();
+    note_neg(d, cb.w, S);
   }
 }
 __global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body(d); }

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/meshhash.h"
+#include "mh_div.h"
 
 #define MH_BLOCK_SIDE 8
 #define MH_BLOCK_VOXELS 512
@@ -84,7 +85,7 @@ struct DevParams {
   uint32_t linked_list_size;
   int value_capacity;
   int max_vertex_count, max_triangle_count, overflow_capacity;
-  float voxel_size, truncation_distance_scale, truncation_distance, sdf_upper_bound;
+  float voxel_size, inv_voxel, truncation_distance_scale, truncation_distance, sdf_upper_bound;
   float weight_sample;
   float fx, fy, cx, cy;
   uint32_t width, height;
@@ -94,6 +95,28 @@ struct DevParams {
   float min_raycast_depth, max_raycast_depth, raycast_step, sample_sdf_threshold, sdf_threshold;
   int enable_gradients, enable_bayesian;
   int compat;  // evaluate the reference's formulas as written
+};
+
+// The cells of a raycast's view: a bit per cell of U = 2 << shift voxels in
+// the view's bounding box.  A word holds 4 x 4 x 2 cells, so with U = 2 two
+// words hold a block (mh_raycast.cu).
+#define MH_GRID_BIAS 49152.0f        // 1.5 * 2^15: a float there has 8 bits of fraction
+#define MH_GRID_MAX_WORDS (1u << 25) // 128 MB
+struct RayGrid {
+  unsigned *bits;            // null: no grid, every sample is evaluated
+  int cx, cy, cz;            // first cell on each axis (a multiple of 4), in cells from the world's origin
+  unsigned nx, ny, nz;       // words on each axis
+  unsigned words;            // nx * ny * nz
+  int shift;                 // U = 2 << shift
+  float ox, oy, oz;          // world position of the first cell's lower corner
+  float inv_cell;            // 1 / (U voxel sizes)
+  // The blocks of the same box: entry (z bny + y) bnx + x holds tag | block
+  // index for a block that exists, anything with another top byte otherwise.
+  unsigned *blocks;          // null: blocks are looked up in the hash table
+  int bx, by, bz;            // first block on each axis
+  unsigned bnx, bny, bnz;
+  unsigned tag;              // this raycast's top byte, 1 .. 255
+  unsigned clear;            // the tags start over: entries to clear first (all that the buffer has), else 0
 };
 
 // Everything a kernel needs, passed by value (pointers + params).
@@ -109,8 +132,8 @@ struct Dev {
   int *life, *inner, *boundary, *nvtx;  // per block
   int *page_of;            // per block: mesh page or -1
   float *wmax;             // per block: upper bound of the largest voxel weight
-  int *nnc;                // per block: voxels whose sdf is non-negative (sdf_nonneg), 512 = all
-  uint8_t *cellok;         // per block, set before a raycast: it and its 7 upper neighbours count 512 (null: unused)
+  unsigned long long *neg; // per block: bit x/2 + 4 (y/2) + 16 (z/2) set if a voxel of that 2^3 may not be non-negative
+  RayGrid grid;            // the raycast's view
   uint8_t *touch;          // per block: set by the raycast when a ray looks it up (null: not recorded)
   int *vtx_slot;           // [pages * 512 * 3]
   int *tri_slot;           // [pages * 512 * 5]
@@ -184,15 +207,18 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31; }
 // A voxel counts as non-negative when its sdf lies in [0, 1e30) (NaN does
 // not).  A trilinear sample whose eight corners are all non-negative is then
 // non-negative itself and finite: its weights lie in [0, 1].  Every kernel
-// that writes sdf keeps the per-block count of such voxels (nnc) exact; the
-// raycast skips the gathers of samples whose corner blocks all count 512.
+// that writes sdf keeps the per-block masks (neg) of 2^3 voxel groups that may
+// hold another value: a bit may be set without need, never clear without.
+// The raycast's grid is made from them.
 __device__ __forceinline__ int sdf_nonneg(float s) { return s >= 0.0f && s < 1e30f ? 1 : 0; }
-// add the lanes' changes of one block's non-negative count (all active lanes
-// of the warp update the same block)
-__device__ __forceinline__ void note_nnc(const Dev &d, int blk, int delta) {
-  const unsigned act = __activemask();
-  const int sum = __reduce_add_sync(act, delta);
-  if ((int)lane_id() == __ffs(act) - 1 && sum) atomicAdd(d.nnc + blk, sum);
+// Bits of the 16 groups that a whole warp holds as a block's z layers 2w and
+// 2w + 1: lane = (x / 4) + 2 y + 16 (z & 1) with four voxels S along x.
+__device__ __forceinline__ unsigned neg_bits(const float4 &S) {
+  const bool lo = !(sdf_nonneg(S.x) & sdf_nonneg(S.y)), hi = !(sdf_nonneg(S.z) & sdf_nonneg(S.w));
+  unsigned a = __ballot_sync(0xffffffffu, lo), b = __ballot_sync(0xffffffffu, hi);
+  a |= a >> 16, b |= b >> 16;  // z
+  a |= a >> 2, b |= b >> 2;    // y: lane bits 0, 2, 3 are left, so a group row starts at bit 4 (y / 2)
+  return (a & 0x1111u) | (b & 0x1111u) << 1 | (a & 0x2222u) << 1 | (b & 0x2222u) << 2;
 }
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
@@ -304,10 +330,24 @@ struct BlockCache {
   }
 };
 
+// p / voxel_size on each axis, rounded as the division is
+__device__ __forceinline__ F3 in_voxels(const DevParams &p, F3 v) {
+  if (mh_div_ok(v.x, v.y, v.z))
+    return f3(mh_div(v.x, p.voxel_size, p.inv_voxel), mh_div(v.y, p.voxel_size, p.inv_voxel),
+              mh_div(v.z, p.voxel_size, p.inv_voxel));
+  return f3(v.x / p.voxel_size, v.y / p.voxel_size, v.z / p.voxel_size);
+}
+
 // Corner voxel indices of one axis for GetSpatialValue: exactly
-// WorldToVoxeli(p - v/2) and WorldToVoxeli(p - v/2 + v).
-__device__ __forceinline__ void corner_pair(float p, float off, float vs, float fl, float fr, int &c0, int &c1) {
-  if (fr > 0.01f && fr < 0.99f) {
+// WorldToVoxeli(p - v/2) and WorldToVoxeli(p - v/2 + v), for q = p / v with
+// integer part fl and fraction fr.  Both round a value that differs from
+// q - 1/2 or q + 1/2 by at most 5 roundings of 2^-24 (|q| + 1), so they are fl
+// and fl + 1 unless q lies that close to an integer; only there are the two
+// divisions evaluated.
+__device__ __forceinline__ void corner_pair(float p, float off, float vs, float q, float fl, float fr, int &c0,
+                                            int &c1) {
+  const float near = 1e-6f * (fabsf(q) + 1.0f);
+  if (fr > near && fr < 1.0f - near) {
     c0 = (int)fl;
     c1 = c0 + 1;
   } else {
@@ -327,16 +367,13 @@ __device__ __forceinline__ bool spatial_sample(const Dev &d, BlockCache &bc, F3 
                                                BlockCache *bc2 = nullptr) {
   const float off = d.p.voxel_size;
   const float vs = d.p.voxel_size;
-  const float qx = pos.x / vs, qy = pos.y / vs, qz = pos.z / vs;
-  const float fx = floorf(qx), fy = floorf(qy), fz = floorf(qz);
-  const float rx = qx - fx, ry = qy - fy, rz = qz - fz;
-  // The corner voxels are round-half-away((p - v/2)/v) and ((p + v/2)/v), which
-  // equal floor(p/v) and floor(p/v) + 1 unless p/v lies within rounding error
-  // of an integer; only there are the two extra divisions evaluated.
+  const F3 q = in_voxels(d.p, pos);
+  const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
+  const float rx = q.x - fx, ry = q.y - fy, rz = q.z - fz;
   int v0x, v0y, v0z, v1x, v1y, v1z;
-  corner_pair(pos.x, off, vs, fx, rx, v0x, v1x);
-  corner_pair(pos.y, off, vs, fy, ry, v0y, v1y);
-  corner_pair(pos.z, off, vs, fz, rz, v0z, v1z);
+  corner_pair(pos.x, off, vs, q.x, fx, rx, v0x, v1x);
+  corner_pair(pos.y, off, vs, q.y, fy, ry, v0y, v1y);
+  corner_pair(pos.z, off, vs, q.z, fz, rz, v0z, v1z);
   const int b0x = vox2blk(v0x), b0y = vox2blk(v0y), b0z = vox2blk(v0z);
   const int p0 = bc.get(d, b0x, b0y, b0z);
   if (p0 < 0) return false;

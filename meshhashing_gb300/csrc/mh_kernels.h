@@ -19,6 +19,15 @@ int launch_predict_inlier(const Dev &d, cudaStream_t s);
 
 int launch_mesh(const Dev &d, cudaStream_t s);
 
+// A volume's buffers for its view's grid: sizes for any view, and the grid of
+// the view from wTc in them (their next tag).
+struct RayGridBuf {
+  unsigned *bits = nullptr, *blocks = nullptr;
+  unsigned words = 0, entries = 0;
+  unsigned tag = 0;
+};
+void ray_grid_sizes(const mh_params &P, RayGridBuf &b);
+RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b);
 int launch_raycast(const Dev &d, float *depth, float *vert4, float *norm4, cudaStream_t s);
 int launch_count_flags(const uint8_t *flags, int n, int *out, cudaStream_t s);
 
@@ -42,6 +51,7 @@ int launch_batch_mesh(const Scene *t, int n, cudaStream_t s);
 int launch_batch_gc_low_surfel(const Scene *t, int n, cudaStream_t s);
 int launch_batch_gc_recycle(const Scene *t, int n, int which, cudaStream_t s);
 int launch_batch_gc_starve(const Scene *t, int n, cudaStream_t s);
+int launch_batch_ray_grid(const Scene *t, int n, cudaStream_t s);
 int launch_raycast_batch(const Scene *t, int n, int total_tiles, int shape, cudaStream_t s);
 int ray_tile_shapes();
 void ray_tile_shape(int i, int &tx, int &ty);

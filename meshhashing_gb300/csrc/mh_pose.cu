@@ -250,7 +250,7 @@ int mh_raycast_backward(mh_volume *v, const float cTw[16], const float *dL_ddept
   if ((r = ensure_acc(v)) != MH_OK) return r;
   if ((r = set_raycast_pose(v, cTw, s)) != MH_OK) return r;
   if (cudaMemsetAsync(v->acc, 0, sizeof(double) * 32, s) != cudaSuccess) return MH_ERR_CUDA;
-  if ((r = launch_raycast_grad(v->d, 0, dL_ddepth, dL_dnormal4, grad_sdf, nullptr, 0.0f, v->acc, s)) != MH_OK)
+  if ((r = launch_raycast_grad(with_ray_grid(v), 0, dL_ddepth, dL_dnormal4, grad_sdf, nullptr, 0.0f, v->acc, s)) != MH_OK)
     return r;
   double h[6];
   if (cudaMemcpyAsync(h, v->acc, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -273,7 +273,7 @@ int mh_raycast_normal_equations(mh_volume *v, const float cTw[16], const float *
   if ((r = ensure_acc(v)) != MH_OK) return r;
   if ((r = set_raycast_pose(v, cTw, s)) != MH_OK) return r;
   if (cudaMemsetAsync(v->acc, 0, sizeof(double) * 32, s) != cudaSuccess) return MH_ERR_CUDA;
-  if ((r = launch_raycast_grad(v->d, 1, nullptr, nullptr, nullptr, obs, max_residual, v->acc, s)) != MH_OK) return r;
+  if ((r = launch_raycast_grad(with_ray_grid(v), 1, nullptr, nullptr, nullptr, obs, max_residual, v->acc, s)) != MH_OK) return r;
   double h[29];
   if (cudaMemcpyAsync(h, v->acc, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

@@ -128,25 +128,40 @@ __global__ void k_scatter_fields(Dev d, const int *ptr, int n, const float *sdf,
   if (blk >= n) return;
   const int p = ptr[blk];
   if (p < 0) return;
-  __shared__ int npos;
-  if (threadIdx.x == 0) npos = 0;
+  __shared__ unsigned long long neg;
+  if (threadIdx.x == 0) neg = 0ull;
   __syncthreads();
-  int mine = 0;
   for (int v = threadIdx.x; v < MH_BLOCK_VOXELS; v += blockDim.x) {
     const size_t src = (size_t)blk * MH_BLOCK_VOXELS + v, dst = (size_t)p * MH_BLOCK_VOXELS + v;
     if (v == 0) d.wmax[p] = __int_as_float(0x7f800000);
     if (sdf) {
       d.sdf[dst] = sdf[src];
-      mine += sdf_nonneg(sdf[src]);
+      if (!sdf_nonneg(sdf[src])) atomicOr(&neg, 1ull << (((v >> 1) & 3) | ((v >> 2) & 12) | ((v >> 3) & 48)));
     }
     if (w) d.w[dst] = w[src];
     if (a) d.a[dst] = a[src];
     if (b) d.b[dst] = b[src];
   }
   if (sdf) {
-    atomicAdd(&npos, mine);
     __syncthreads();
-    if (threadIdx.x == 0) d.nnc[p] = npos;
+    if (threadIdx.x == 0) d.neg[p] = neg;
+  }
+}
+
+// out[i] = voxels of block ptr[i] whose sdf is non-negative (sdf_nonneg)
+__global__ void __launch_bounds__(128) k_count_nonneg(const float *sdf, const int *ptr, int n, int *out) {
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int p = ptr[i];
+    if (p < 0) continue;
+    __shared__ int count;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    int c = 0;
+    for (int v = threadIdx.x; v < MH_BLOCK_VOXELS; v += blockDim.x) c += sdf_nonneg(sdf[(size_t)p * MH_BLOCK_VOXELS + v]);
+    atomicAdd(&count, c);
+    __syncthreads();
+    if (threadIdx.x == 0) out[i] = count;
+    __syncthreads();
   }
 }
 
@@ -189,6 +204,13 @@ static Counters read_counters(mh_volume *v) {
     int _r = (expr);              \
     if (_r != MH_OK) return _r;   \
   } while (0)
+
+// The volume's device state with the grid of the raycast pose's view.
+Dev with_ray_grid(mh_volume *v) {
+  Dev d = v->d;
+  d.grid = ray_grid_for(v->hp, v->fc_host.rc_wTc, v->grid);
+  return d;
+}
 
 extern "C" {
 
@@ -252,7 +274,7 @@ int mh_volume_reset(mh_volume *v, void *stream) {
   MH_CUDA_TRY(cudaMemsetAsync(d.flags, 0, cap, s));
   k_fill_i32<<<grid_for(cap), 256, 0, s>>>(d.life, cap, MH_BLOCK_LIFE);
   // every voxel starts at sdf 0, which counts as non-negative
-  k_fill_i32<<<grid_for(cap), 256, 0, s>>>(d.nnc, cap, MH_BLOCK_VOXELS);
+  MH_CUDA_TRY(cudaMemsetAsync(d.neg, 0, sizeof(unsigned long long) * cap, s));
   k_fill_i32<<<grid_for(pv * 3), 256, 0, s>>>(d.vtx_slot, pv * 3, MH_FREE_PTR);
   k_fill_i32<<<grid_for(pv * 5), 256, 0, s>>>(d.tri_slot, pv * 5, MH_FREE_PTR);
   k_stack_init<<<grid_for(npg), 256, 0, s>>>(d.page_heap, (int)npg, (int)npg);
@@ -313,6 +335,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   q.max_triangle_count = (int)P.max_triangle_count;
   q.overflow_capacity = (int)P.overflow_capacity;
   q.voxel_size = P.voxel_size;
+  q.inv_voxel = 1.0f / P.voxel_size;
   q.truncation_distance_scale = P.truncation_distance_scale;
   q.truncation_distance = P.truncation_distance;
   q.sdf_upper_bound = P.sdf_upper_bound;
@@ -352,8 +375,10 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   const size_t pv = (size_t)d.page_capacity * MH_BLOCK_VOXELS;
   A(dalloc(v, &d.page_of, cap));
   A(dalloc(v, &d.wmax, cap));
-  A(dalloc(v, &d.nnc, cap));
-  A(dalloc(v, &d.cellok, cap));
+  A(dalloc(v, &d.neg, cap));
+  ray_grid_sizes(P, v->grid);
+  A(dalloc(v, &v->grid.bits, v->grid.words));
+  if (v->grid.entries) A(dalloc(v, &v->grid.blocks, v->grid.entries));
   A(dalloc(v, &d.mesh_list, cap));
   A(dalloc(v, &d.cube_list, cap));
   A(dalloc(v, &d.vtx_list, cap));
@@ -515,14 +540,14 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
   const size_t n = (size_t)v->hp.rc_width * v->hp.rc_height;
   if (on_device) {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
-    return launch_raycast(v->d, depth, vert4, norm4, s);
+    return launch_raycast(with_ray_grid(v), depth, vert4, norm4, s);
   }
   float *dd = depth ? v->rc_stage : nullptr;
   float *dv = vert4 ? v->rc_stage + n : nullptr;
   float *dn = norm4 ? v->rc_stage + 5 * n : nullptr;
   {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
-    TRY(launch_raycast(v->d, dd, dv, dn, s));
+    TRY(launch_raycast(with_ray_grid(v), dd, dv, dn, s));
   }
   if (depth) MH_CUDA_TRY(cudaMemcpyAsync(depth, dd, n * sizeof(float), cudaMemcpyDeviceToHost, s));
   if (vert4) MH_CUDA_TRY(cudaMemcpyAsync(vert4, dv, n * 4 * sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -563,7 +588,7 @@ int mh_raycast_footprint(mh_volume *v, const float cTw[16], int *blocks_touched,
     memcpy(fc.wTc, fc.rc_wTc, sizeof(float) * 16);
   }
   MH_CUDA_TRY(cudaMemcpyAsync(v->d.fc, &fc, sizeof(FrameConst), cudaMemcpyHostToDevice, s));
-  Dev d = v->d;
+  Dev d = v->d;  // without the view's grid: every sample is looked up
   d.touch = v->touch;
   TRY(launch_raycast(d, nullptr, nullptr, nullptr, s));
   TRY(launch_count_flags(v->touch, cap, dcount, s));
@@ -885,9 +910,15 @@ int mh_dump_nonneg_counts(mh_volume *v, int n, const int32_t *pos, int32_t *coun
   MH_CUDA_TRY(cudaDeviceSynchronize());
   std::vector<int> ptr;
   TRY(find_ptrs(v, n, pos, ptr, false));
-  std::vector<int> all((size_t)v->d.p.value_capacity);
-  MH_CUDA_TRY(cudaMemcpy(all.data(), v->d.nnc, sizeof(int) * all.size(), cudaMemcpyDeviceToHost));
-  for (int i = 0; i < n; ++i) count[i] = ptr[i] < 0 ? INT32_MIN : all[ptr[i]];
+  if (n == 0) return MH_OK;
+  // find_ptrs left the block indices in the scratch, after the positions, whose space takes the counts
+  int *dcount = v->scratch, *dptr = v->scratch + 3 * (size_t)n;
+  k_count_nonneg<<<grid_for((size_t)n, 1), 128>>>(v->d.sdf, dptr, n, dcount);
+  mh_count_launches(1);
+  MH_CUDA_TRY(cudaGetLastError());
+  MH_CUDA_TRY(cudaMemcpy(count, dcount, sizeof(int) * n, cudaMemcpyDeviceToHost));
+  for (int i = 0; i < n; ++i)
+    if (ptr[i] < 0) count[i] = INT32_MIN;
   return MH_OK;
 }
 

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "mh_internal.cuh"
+#include "mh_kernels.h"
 
 struct mh_pd_state;
 
@@ -15,6 +16,7 @@ struct mh_volume {
   Dev d;
   float *tv = nullptr;
   float *rc_stage = nullptr;  // device staging for host raycast outputs
+  RayGridBuf grid;            // cells and blocks of the raycast's view
   double *acc = nullptr;      // reduction target of the raycast gradients (allocated on first use)
   uint8_t *touch = nullptr;   // raycast footprint flags, one per block (allocated on first use)
   mh_pd_state *pd = nullptr;  // Huber-TV state (allocated on first use)
@@ -43,5 +45,7 @@ struct mh_volume {
 // 4x4 inverse by cofactors with the term order of float4x4::getInverse
 // (extern/cuda/matrix.h:964-1086)
 void inverse4(const float *m, float *out);
+// the device state with the grid of the raycast pose's view (fc_host.rc_wTc)
+Dev with_ray_grid(mh_volume *v);
 // releases the Huber-TV state of a volume (mh_huber.cu)
 void mh_pd_free(mh_volume *v);

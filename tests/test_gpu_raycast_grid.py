@@ -1,0 +1,73 @@
+"""The raycast's grid of cells and blocks against the FP32 oracle, bit for bit.
+
+The grid follows the view: cells of 2 voxels, or larger where the image is
+small (128 words a pixel), blocks from a dense array, or from the hash table
+where the view holds too many.  Images with ragged tiles, poses on and off the
+map, outside it and looking away, matrices that are not rigid, and more
+raycasts than the dense array has tags.
+"""
+import numpy as np
+import pytest
+
+from meshhashing_gb300 import Volume, config, scene
+from meshhashing_gb300.pose import left_update
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+POSES = {
+    "own": lambda T: T,
+    "moved": lambda T: left_update(T, [0.1, -0.07, 0.05, 0.1, 0.2, -0.15]),
+    "outside": lambda T: left_update(T, [3.0, -2.0, 0.4, 0.0, 0.0, 2.5]),
+    "away": lambda T: left_update(T, [40.0, 40.0, 0.0, 0.0, 0.0, 0.0]),
+    "scaled": lambda T: T @ np.diag([1.2, 0.8, 1.1, 1.0]),
+}
+
+
+def _map(w, h, voxel, frames=6, **over):
+    wl = scene.full_spline(frames, width=w, height=h)
+    p = config.params_for(wl, voxel_size=voxel, truncation=3 * voxel, value_capacity=1 << 16, bucket_count=1 << 16,
+                          max_vertex_count=1 << 16, max_triangle_count=1 << 16, **over)
+    v = Volume(p)
+    for i in range(frames):
+        v.integrate_frame(wl.frame(i), wl.pose(i))
+    o = Oracle(p, fp64=False)
+    pos, f = v.dump_blocks()
+    o.set_blocks(pos, f["sdf"], f["w"], f["a"], f["b"])
+    assert v.stats()["error"] == 0
+    return wl, v, o
+
+
+def _same(v, o, cTw):
+    gd, gv, gn = v.raycast(cTw)
+    od, ov, on = o.raycast(cTw)
+    for g, r in ((gd, od), (gv, ov), (gn, on)):
+        hit = np.isfinite(r)
+        assert np.array_equal(np.isfinite(g), hit)
+        np.testing.assert_array_equal(g[hit].view(np.uint32), r[hit].view(np.uint32))
+    return int(np.isfinite(od).sum())
+
+
+# cells of 8, 4, 2 and 8 voxels; at 1 mm 32, and the blocks come from the hash table
+@pytest.mark.parametrize("w,h,voxel", [(36, 28, 0.004), (124, 92, 0.004), (124, 92, 0.008), (52, 44, 0.0047),
+                                       (40, 28, 0.001)])
+def test_views(built, w, h, voxel):
+    wl, v, o = _map(w, h, voxel)
+    hits = {}
+    for name, move in POSES.items():
+        T = move(np.asarray(wl.pose(5), np.float64))
+        hits[name] = _same(v, o, np.linalg.inv(T).astype(np.float32))
+    assert hits["own"] > w * h // 4 and hits["away"] == 0
+    assert v.stats()["error"] == 0
+
+
+def test_more_raycasts_than_tags(built):
+    wl, v, o = _map(36, 28, 0.008)
+    poses = [np.linalg.inv(left_update(np.asarray(wl.pose(5), np.float64), [0.3 * s, 0.0, 0.0, 0.0, 0.0, 0.4 * s]))
+             .astype(np.float32) for s in (-1.0, 0.0, 1.0)]
+    first = [v.raycast(c) for c in poses]
+    for k in range(90):
+        for c, ref in zip(poses, first):
+            for a, b in zip(v.raycast(c), ref):
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), k
+    assert _same(v, o, poses[1]) > 0
