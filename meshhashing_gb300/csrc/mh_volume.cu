@@ -342,6 +342,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   q.weight_sample = (float)P.weight_sample;
   q.fx = P.fx, q.fy = P.fy, q.cx = P.cx, q.cy = P.cy;
   q.width = P.width, q.height = P.height;
+  q.pix_half = 0.5f - 4.8e-7f * (std::max((float)P.width + std::fabs(P.cx), (float)P.height + std::fabs(P.cy)) + 2.0f);
   q.min_depth_range = P.min_depth_range, q.max_depth_range = P.max_depth_range;
   q.rc_fx = P.rc_fx, q.rc_fy = P.rc_fy, q.rc_cx = P.rc_cx, q.rc_cy = P.rc_cy;
   q.rc_width = P.rc_width, q.rc_height = P.rc_height;
@@ -401,7 +402,8 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   A(dalloc(v, &d.fc, 1));
   A(dalloc(v, &d.ctr, 1));
   A(dalloc(v, &v->tv, npix * 9));
-  A(dalloc(v, &v->rc_stage, rpix * 9));
+  d.pixels = reinterpret_cast<float4 *>(v->tv);
+  A(dalloc(v, &v->rc_stage, rpix * 9 + 3));
   if (r == MH_OK) r = mh_volume_reset(v, nullptr);
   if (r != MH_OK) {
     mh_volume_destroy(v);
@@ -543,8 +545,9 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
     return launch_raycast(with_ray_grid(v), depth, vert4, norm4, s);
   }
   float *dd = depth ? v->rc_stage : nullptr;
-  float *dv = vert4 ? v->rc_stage + n : nullptr;
-  float *dn = norm4 ? v->rc_stage + 5 * n : nullptr;
+  // vertices and normals are written as float4: they start on such a boundary
+  float *dv = vert4 ? v->rc_stage + (n + 3) / 4 * 4 : nullptr;
+  float *dn = norm4 ? v->rc_stage + (n + 3) / 4 * 4 + 4 * n : nullptr;
   {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
     TRY(launch_raycast(with_ray_grid(v), dd, dv, dn, s));

@@ -71,3 +71,12 @@ def test_more_raycasts_than_tags(built):
             for a, b in zip(v.raycast(c), ref):
                 assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), k
     assert _same(v, o, poses[1]) > 0
+
+
+@pytest.mark.parametrize("w,h", [(37, 29), (33, 30), (31, 29)])
+def test_host_images_of_any_size(built, w, h):
+    """Pixel counts of 1, 2 and 3 modulo 4: the staged vertices and normals are vectors of four."""
+    assert (w * h) % 4 == {37: 1, 33: 2, 31: 3}[w]
+    wl, v, o = _map(w, h, 0.008)
+    T = np.asarray(wl.pose(5), np.float64)
+    assert _same(v, o, np.linalg.inv(T).astype(np.float32)) > 0
