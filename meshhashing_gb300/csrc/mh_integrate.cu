@@ -7,40 +7,44 @@
 // CTA covers one block per iteration with 4 consecutive voxels per thread, so
 // every voxel field moves as one aligned 128-bit load/store.  Voxel fields are
 // only loaded when at least one of the thread's voxels projects onto a valid
-// depth pixel inside the truncation band.
+// depth pixel inside the truncation band (sdf: of the warp's).
 #include "mh_internal.cuh"
 #include "mh_exp.h"
 #include "mh_kernels.h"
 #include "mh_batch.cuh"
 
+#include <algorithm>
+
 namespace {
 
-struct VoxProj {
-  float cam_z;
-  float depth;
-  float aux;
-  int pix;
-};
-
-// Per-voxel projection shared by the update kernels (update_simple.cu:26-46).
-// `aux` (the inlier ratio of the PSDF update, or null) is read at the same
-// pixel in the same round trip as the depth.
-__device__ __forceinline__ bool project_voxel(const DevParams &p, const float *cTw, const float *depth,
-                                              const float *aux, int vx, int vy, int vz, VoxProj &o) {
+// Pixel of a camera-frame point (update_simple.cu:26-46), or -1 outside the
+// image: the integer part of c.x fx / c.z + cx + 1/2, and of y.  Seven
+// roundings of 2^-24 (W + |cx|) at most lie between the value the divisions
+// give and the one an approximate reciprocal (1 unit in the last place) gives,
+// so the integer parts agree unless the latter comes that close to an integer
+// (1 - 2 pix_half; 0.2 % of voxels at 640x480); only there, and for points
+// that are not finite or far off, are the two divisions evaluated.
+__device__ __forceinline__ int pixel_of(const DevParams &p, F3 c) {
+  const float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(c.z));
+  const float ax = c.x * p.fx, ay = c.y * p.fy;
+  const float wx = fmaf(ax, r, p.cx + 0.5f), wy = fmaf(ay, r, p.cy + 0.5f);
+  const float mx = (wx - 0.5f) + kMagic, my = (wy - 0.5f) + kMagic;
+  int px = __float_as_int(mx) - 0x4b400000, py = __float_as_int(my) - 0x4b400000;
+  if (fabsf(wx - (mx - kMagic) - 0.5f) < p.pix_half && fabsf(wy - (my - kMagic) - 0.5f) < p.pix_half) {
+    if (px == -1) px = 0;  // (-1, 0) truncates to 0
+    if (py == -1) py = 0;
+  } else {
+    px = f2i(ax / c.z + p.cx + 0.5f);
+    py = f2i(ay / c.z + p.cy + 0.5f);
+  }
+  return (unsigned)px < p.width && (unsigned)py < p.height ? (int)((unsigned)py * p.width + (unsigned)px) : -1;
+}
+// camera-frame position of voxel (x, y, z) given as floats
+__device__ __forceinline__ F3 voxel_in_camera(const DevParams &p, const float *cTw, float x, float y, float z) {
   const float vs = p.voxel_size;
-  F3 c = mul_pt(cTw, f3((float)vx * vs, (float)vy * vs, (float)vz * vs));
-  const float u = c.x * p.fx / c.z + p.cx;
-  const float v = c.y * p.fy / c.z + p.cy;
-  const unsigned px = (unsigned)f2i(u + 0.5f), py = (unsigned)f2i(v + 0.5f);
-  if (px >= p.width || py >= p.height) return false;
-  const int pix = py * p.width + px;
-  const float d = __ldg(depth + pix);
-  o.aux = aux ? __ldg(aux + pix) : 0.0f;
-  if (depth_invalid(p, d)) return false;
-  o.cam_z = c.z;
-  o.depth = d;
-  o.pix = pix;
-  return true;
+  return mul_pt(cTw, f3(x * vs, y * vs, z * vs));
 }
 
 __device__ __forceinline__ float get(const float4 &v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
@@ -84,21 +88,25 @@ __device__ __forceinline__ void integrate_simple_body(const Dev &d) {
     if (c + (int)gridDim.x < n) next = d.cand[c + gridDim.x];
     if (cb.w < 0) continue;
     const int vx0 = cb.x * MH_BLOCK_SIDE + lx, vy = cb.y * MH_BLOCK_SIDE + ly, vz = cb.z * MH_BLOCK_SIDE + lz;
+    const float fx0 = (float)vx0, fy = (float)vy, fz = (float)vz;
     float sdf_new[4], w_new[4];
     bool act[4], any = false;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      VoxProj o;
       act[k] = false;
-      if (!project_voxel(p, cTw, d.depth, nullptr, vx0 + k, vy, vz, o)) continue;
-      float sdf = o.depth - o.cam_z;
+      const F3 cam = voxel_in_camera(p, cTw, fx0 + (float)k, fy, fz);
+      const int pix = pixel_of(p, cam);
+      if (pix < 0) continue;
+      const float depth = __ldg(d.depth + pix);
+      if (depth_invalid(p, depth)) continue;
+      float sdf = depth - cam.z;
       // 1 - normalized depth as (dmax - d) / (dmax - dmin): same value, no
       // cancellation near the far limit (update_simple.cu:49-55); the
       // compatibility mode keeps the reference's 1 - (d - dmin) / (dmax - dmin)
-      const float far = p.compat ? 1.0f - normalize_depth(p, o.depth)
-                                 : (p.max_depth_range - o.depth) / (p.max_depth_range - p.min_depth_range);
+      const float far = p.compat ? 1.0f - normalize_depth(p, depth)
+                                 : (p.max_depth_range - depth) / (p.max_depth_range - p.min_depth_range);
       const float w = fmaxf(10.0f * p.weight_sample * far, 1.0f);
-      const float tr = truncate_dist(p, o.depth);
+      const float tr = truncate_dist(p, depth);
       if (sdf <= -tr) continue;
       sdf = sdf >= 0.0f ? fminf(tr, sdf) : fmaxf(-tr, sdf);
       sdf_new[k] = sdf;
@@ -133,6 +141,26 @@ __global__ void __launch_bounds__(128) k_integrate_simple_b(const Scene *t, int 
   each_scene(t, n, [&](const Scene &c) { if (!c.d.p.enable_bayesian) integrate_simple_body(c.d); });
 }
 
+// What the PSDF update needs of a pixel, once per pixel instead of once per
+// voxel that projects onto it: depth (-inf if invalid), inlier ratio, the
+// measurement's variance and the outlier density (update_bayesian.cu:123-156).
+__device__ __forceinline__ void pixels_body(const Dev &d) {
+  const DevParams &p = d.p;
+  const int n = p.width * p.height;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float dd = d.depth[i], r = d.inlier[i];
+    const float tau = (dd - 0.4f) * 0.012f + 0.019f;
+    const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
+    const float out = p.compat ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : (1.0f - r) * 0.204081632653061224f;
+    d.pixels[i] = make_float4(depth_invalid(p, dd) ? -__int_as_float(0x7f800000) : dd, r, tau * tau,
+                              in_range ? out : 1.0f);
+  }
+}
+__global__ void __launch_bounds__(256) k_pixels(Dev d) { pixels_body(d); }
+__global__ void __launch_bounds__(256) k_pixels_b(const Scene *t, int n) {
+  each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) pixels_body(c.d); });
+}
+
 // UpdateBlocksBayesianKernel (mapping/update_bayesian.cu:103-185).  Per voxel
 // the update is division- and transcendental-bound, not load-bound, so the
 // default form restates it with 4 IEEE divisions (see below); compat mode
@@ -151,21 +179,21 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
     if (c + (int)gridDim.x < n) next = d.cand[c + gridDim.x];
     if (cb.w < 0) continue;
     const int vx0 = cb.x * MH_BLOCK_SIDE + lx, vy = cb.y * MH_BLOCK_SIDE + ly, vz = cb.z * MH_BLOCK_SIDE + lz;
-    float xs[4], rho[4], dep[4];
+    const float fx0 = (float)vx0, fy = (float)vy, fz = (float)vz;
+    float xs[4], rs[4], ts[4], cs[4];
     bool act[4], any = false;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      VoxProj o;
+      const F3 cam = voxel_in_camera(p, cTw, fx0 + (float)k, fy, fz);
+      const int pix = pixel_of(p, cam);
       act[k] = false;
-      if (!project_voxel(p, cTw, d.depth, d.inlier, vx0 + k, vy, vz, o)) continue;
-      float x = o.depth - o.cam_z;
-      const float r = o.aux;
-      const float tr = truncate_dist(p, o.depth);
-      if (x <= -tr) continue;
-      x = x >= 0.0f ? fminf(tr, x) : fmaxf(-tr, x);
-      xs[k] = x;
-      rho[k] = r;
-      dep[k] = o.depth;
+      if (pix < 0) continue;
+      const float4 px = __ldg(d.pixels + pix);
+      const float x = px.x - cam.z;
+      const float tr = truncate_dist(p, px.x);
+      if (px.x == -__int_as_float(0x7f800000) || x <= -tr) continue;
+      xs[k] = x >= 0.0f ? fminf(tr, x) : fmaxf(-tr, x);
+      rs[k] = px.y, ts[k] = px.z, cs[k] = px.w;
       act[k] = true;
       any = true;
     }
@@ -179,20 +207,17 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (!act[k]) continue;
-        const float x = xs[k], r = rho[k], dd = dep[k];
-        const float tau = (dd - 0.4f) * 0.012f + 0.019f;
+        const float x = xs[k], r = rs[k], t2 = ts[k];
         const float w0 = get(W, k);
         if (w0 == 0.0f) {
           put(S, k, x);
-          put(W, k, 1.0f / (tau * tau));
+          put(W, k, 1.0f / t2);
           put(A, k, r * 10.0f);
           put(B, k, (1.0f - r) * 10.0f);
           continue;
         }
         const float mu = get(S, k);
         const float a = get(A, k), b = get(B, k);
-        const float t2 = tau * tau;
-        const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
         if (p.compat) {
           // the reference's expressions as written (update_bayesian.cu:140-180);
           // sqrt(2 pi) is a double there, so the product and the reciprocal of
@@ -203,7 +228,7 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
           const float sv = s2 + t2;
           const double g = 1.0 / (2.5066282746310002 * (double)sqrtf(sv)) * (double)expf(-((x - mu) * (x - mu)) / sv);
           float C1 = (float)((double)r * g);
-          float C2 = in_range ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : 1.0f;
+          float C2 = cs[k];
           const float sum = C1 + C2;
           C1 /= sum;
           C2 /= sum;
@@ -237,10 +262,12 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
         const float m = q * (mu * u + x);
         const float isv = w0 * q;
         const float dx = x - mu;
-        const float g = mh_expf(-(dx * dx) * isv) * sqrtf(isv) * 0.398942280401432678f;
+        // mh_expf is 1 from -2^-25 up; in observed free space (x and mu at the
+        // truncation) whole warps stay there
+        const float ex = -(dx * dx) * isv;
+        const float g = (ex > -0x1p-25f ? 1.0f : mh_expf(ex)) * sqrtf(isv) * 0.398942280401432678f;
         const float C1 = r * g;
-        const float C2 = in_range ? (1.0f - r) * 0.204081632653061224f : 1.0f;
-        const float c = C1 / (C1 + C2);
+        const float c = C1 / (C1 + cs[k]);
         const float oc = 1.0f - c;
         const float dm = m - mu;
         put(S, k, mu + c * dm);
@@ -261,7 +288,7 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
   }
 }
 __global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body(d); }
-__global__ void __launch_bounds__(128) k_integrate_psdf_b(const Scene *t, int n) {
+__global__ void __launch_bounds__(128, 8) k_integrate_psdf_b(const Scene *t, int n) {
   each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) integrate_psdf_body(c.d); });
 }
 
@@ -294,11 +321,13 @@ __device__ __forceinline__ void predict_inlier_body(const Dev &d) {
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
       if (slots[3 * k] <= 0 && slots[3 * k + 1] <= 0 && slots[3 * k + 2] <= 0) continue;
-      VoxProj o;
-      if (!project_voxel(p, cTw, d.depth, nullptr, vx0 + k, vy, vz, o)) continue;
-      const int px = o.pix % p.width, py = o.pix / p.width;
+      const int pix = pixel_of(p, voxel_in_camera(p, cTw, (float)(vx0 + k), (float)vy, (float)vz));
+      if (pix < 0) continue;
+      const float depth = __ldg(d.depth + pix);
+      if (depth_invalid(p, depth)) continue;
+      const int px = pix % p.width, py = pix / p.width;
       const float rx = ((float)px - p.cx) / p.fx, ry = ((float)py - p.cy) / p.fy;
-      const F3 pc = f3(o.depth * rx, o.depth * ry, o.depth);
+      const F3 pc = f3(depth * rx, depth * ry, depth);
       const float vsdf = d.sdf[base + k], vw = d.w[base + k];
       const F3 npc = normalize3(f3(-pc.x, -pc.y, -pc.z));
 #pragma unroll 1
@@ -322,7 +351,7 @@ __device__ __forceinline__ void predict_inlier_body(const Dev &d) {
         w_ang = fmaxf(w_ang, 0.1f);
         float ir = w_disk * w_dist * w_ang;
         ir = fmaxf(ir, 0.01f);
-        atomicMax(reinterpret_cast<int *>(d.inlier + o.pix), __float_as_int(ir));
+        atomicMax(reinterpret_cast<int *>(d.inlier + pix), __float_as_int(ir));
       }
     }
   }
@@ -382,8 +411,9 @@ int launch_integrate_simple(const Dev &d, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 int launch_integrate_psdf(const Dev &d, cudaStream_t s) {
+  k_pixels<<<std::min((int)(d.p.width * d.p.height + 255) / 256, mh_sm_count() * 8), 256, 0, s>>>(d);
   k_integrate_psdf<<<mh_resident_grid((const void *)k_integrate_psdf, 128, 16), 128, 0, s>>>(d);
-  mh_count_launches(1);
+  mh_count_launches(2);
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 int launch_predict_inlier(const Dev &d, cudaStream_t s) {
@@ -418,8 +448,9 @@ int launch_batch_integrate(const Scene *t, int n, int has_simple, int has_psdf, 
     mh_count_launches(1);
   }
   if (has_psdf) {
+    k_pixels_b<<<mh_sm_count() * 4, 256, 0, s>>>(t, n);
     k_integrate_psdf_b<<<mh_resident_grid((const void *)k_integrate_psdf_b, 128, cta_per_sm), 128, 0, s>>>(t, n);
-    mh_count_launches(1);
+    mh_count_launches(2);
   }
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }

@@ -88,6 +88,7 @@ struct DevParams {
   float voxel_size, inv_voxel, truncation_distance_scale, truncation_distance, sdf_upper_bound;
   float weight_sample;
   float fx, fy, cx, cy;
+  float pix_half;           // 1/2 less the rounding of a projection (pixel_of)
   uint32_t width, height;
   float min_depth_range, max_depth_range;
   float rc_fx, rc_fy, rc_cx, rc_cy;
@@ -154,6 +155,7 @@ struct Dev {
   int4 *vwork;             // mesh pass: (owner block, voxel, slot, -) to compute
   int vwork_capacity;
   float *depth, *inlier;   // current frame (W x H)
+  float4 *pixels;          // the PSDF update's pixel records (in the TV scratch)
   FrameConst *fc;
   Counters *ctr;
 };
