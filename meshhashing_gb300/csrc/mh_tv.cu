@@ -16,11 +16,12 @@
 //    iterate, so the dual and primal steps fuse into a single pass with no
 //    grid-wide barrier;
 //  * k_tv_tile (a volume's frames) and its batch twin k_tv_tile_b: ten
-//    iterations per launch on a 64 x 32 tile held in shared memory with a
-//    10-pixel halo, so 20 iterations take 2 launches instead of 22.
+//    iterations per launch on a tile of pixels and a 10-pixel halo, held in
+//    registers, so 20 iterations take 2 launches instead of 22.
 #include "mh_internal.cuh"
 #include "mh_kernels.h"
 #include "mh_batch.cuh"
+#include "mh_round.cuh"
 
 #include <algorithm>
 
@@ -107,23 +108,26 @@ __global__ void k_tv_out_b(const Scene *t, int n, int launches) {
 }
 
 // ------------------------------------------------------------------ tiled
-// Up to TV_K iterations per launch for one TV_TW x TV_TH tile of pixels: the
-// tile and a TV_K-pixel halo sit in shared memory, every iteration runs the
-// dual step over the whole region, then the primal step, and values go stale
-// by one pixel per iteration from the region's edge inwards, so the tile's
-// own pixels stay exact through TV_K iterations.  Each value is computed by
-// the same expressions as tv_iter_body (the dual of a neighbour is the
-// neighbour's own new dual), so the result is bit-identical to running
-// k_tv_iter once per iteration.  The first launch initialises from the depth
-// frame (as k_tv_init), the last writes the frame back (as k_tv_out); between
-// launches the iterate goes through the ping-pong planes.
-#define TV_TW 64
-#define TV_TH 32
+// Up to TV_K iterations per launch for one tile of pixels: the tile and a
+// TV_K-pixel halo form a region whose values go stale by one pixel per
+// iteration from its edge inwards, so the tile's own pixels stay exact through
+// TV_K iterations.  Each value is computed by the same expressions as
+// tv_iter_body (the dual of a neighbour is the neighbour's own new dual), so
+// the result is bit-identical to running k_tv_iter once per iteration.  The
+// first launch initialises from the depth frame (as k_tv_init), the last
+// writes the frame back (as k_tv_out); between launches the iterate goes
+// through the ping-pong planes.
+//
+// A thread owns a strip of R rows of one column and keeps its state in
+// registers.  Shared memory carries what a strip reads of its neighbours: the
+// extrapolated iterate to the right and below, the duals to the left and
+// above.  Bound by instruction issue, so validity is kept as bits and norm and
+// quotients are the rounded ones of mh_round.cuh, without branches: they are
+// those of the operators for depths within 2^-10 .. 2^30 mm (`plain`, for the
+// whole region; a dual value below 2^-60, which they may round otherwise,
+// cannot change the iterate then).  640x480, 20 iterations: 125 -> 48 us
+// (96 us with the operators' division and square root).
 #define TV_K 10
-#define TV_RW (TV_TW + 2 * TV_K)
-#define TV_RH (TV_TH + 2 * TV_K)
-#define TV_RN (TV_RW * TV_RH)
-constexpr size_t kTvTileSmem = sizeof(float) * 5 * TV_RN;
 
 struct TvTile {
   const float *depth_in;  // first launch: the depth frame (metres); else null
@@ -135,83 +139,146 @@ struct TvTile {
   float lambda;
 };
 
-__device__ __forceinline__ void tv_tile_body(const TvTile &b, int tile_x, int tile_y) {
-  extern __shared__ float sm[];
-  float *sf = sm, *su = sm + TV_RN, *sub = sm + 2 * TV_RN, *spx = sm + 3 * TV_RN, *spy = sm + 4 * TV_RN;
+// Region of RW = TW + 2 TV_K columns and RH = R G rows (the tile: RH - 2 TV_K),
+// one thread for each column of each of the G strips.
+template <int TW, int R, int G> struct TvShape {
+  static constexpr int RW = TW + 2 * TV_K, RH = R * G, TH = RH - 2 * TV_K, THREADS = (RW * G + 31) / 32 * 32;
+};
+
+template <int TW, int R, int G> __device__ __forceinline__ void tv_tile_body(const TvTile &b, int tile_x, int tile_y) {
+  typedef TvShape<TW, R, G> T;
+  __shared__ float s_ub[T::RH][T::RW], s_px[T::RH][T::RW], s_py[G][T::RW];
   const float tau = 0.35355339059327373f, sigma = 0.35355339059327373f;
-  const int x0 = tile_x * TV_TW - TV_K, y0 = tile_y * TV_TH - TV_K;
   const float NI = -__int_as_float(0x7f800000);
-  for (int r = threadIdx.x; r < TV_RN; r += blockDim.x) {
-    const int gx = x0 + r % TV_RW, gy = y0 + r / TV_RW;
-    float f = 0.0f, u = 0.0f, ub = 0.0f, px = 0.0f, py = 0.0f;
-    if (gx >= 0 && gx < b.W && gy >= 0 && gy < b.H) {
-      const int i = gy * b.W + gx;
-      if (b.depth_in) {
-        const float z = b.depth_in[i];
-        const bool ok = z > 0.0f && z < 1e30f;
-        f = u = ub = ok ? z * 1000.0f : NI;
-      } else {
-        f = b.f[i], u = b.u[i], ub = b.ub[i], px = b.px[i], py = b.py[i];
+  const int lx = threadIdx.x % T::RW, g = threadIdx.x / T::RW, ly0 = g * R;
+  const int x0 = tile_x * TW - TV_K, y0 = tile_y * T::TH - TV_K, gx = x0 + lx, gy0 = y0 + ly0;
+  const bool live = g < G;  // the last warp's surplus threads only keep the barriers
+  const float den = 1.0f + tau * b.lambda, rden = 1.0f / den;
+  // tf: tau lambda f, the data term
+  float tf[R], u[R], ub[R], px[R], py[R];
+  unsigned valid = 0, right = 0, below = 0;
+  bool plain = den < 0x1p20f;
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int gy = gy0 + j;
+      float f = NI;  // outside the image: like a hole
+      u[j] = ub[j] = NI, px[j] = py[j] = 0.0f;
+      if (gx >= 0 && gx < b.W && gy >= 0 && gy < b.H) {
+        const int i = gy * b.W + gx;
+        if (b.depth_in) {
+          const float z = b.depth_in[i];
+          const bool ok = z > 0.0f && z < 1e30f;
+          f = u[j] = ub[j] = ok ? z * 1000.0f : NI;
+          if (lx >= TV_K && lx < TV_K + TW && ly0 + j >= TV_K && ly0 + j < TV_K + T::TH) b.f[i] = f;
+        } else {
+          f = b.f[i], u[j] = b.u[i], ub[j] = b.ub[i], px[j] = b.px[i], py[j] = b.py[i];
+        }
       }
+      if (f > -1e30f) valid |= 1u << j, plain = plain && f > 0x1p-10f && f < 0x1p30f;
+      tf[j] = tau * b.lambda * f;
+      s_px[ly0 + j][lx] = f;
     }
-    sf[r] = f, su[r] = u, sub[r] = ub, spx[r] = px, spy[r] = py;
+  }
+  plain = __syncthreads_and(plain);
+  // pairs of valid pixels: to the right and below
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const bool vi = valid >> j & 1u;
+      if (vi && gx + 1 < b.W && lx + 1 < T::RW && s_px[ly0 + j][lx + 1] > -1e30f) right |= 1u << j;
+      if (vi && gy0 + j + 1 < b.H && ly0 + j + 1 < T::RH && s_px[ly0 + j + 1][lx] > -1e30f) below |= 1u << j;
+      s_ub[ly0 + j][lx] = ub[j];
+    }
   }
   __syncthreads();
+  const bool has_left = gx > 0 && lx > 0, has_above = gy0 > 0 && ly0 > 0;
   for (int it = 0; it < b.iters; ++it) {
-    // dual step (dual_at): forward differences of ub over valid pairs
-    for (int r = threadIdx.x; r < TV_RN; r += blockDim.x) {
-      const int lx = r % TV_RW, ly = r / TV_RW, gx = x0 + lx, gy = y0 + ly;
-      const bool vi = sf[r] > -1e30f;
-      float gxd = 0.0f, gyd = 0.0f;
-      if (vi && gx + 1 < b.W && lx + 1 < TV_RW && sf[r + 1] > -1e30f) gxd = sub[r + 1] - sub[r];
-      if (vi && gy + 1 < b.H && ly + 1 < TV_RH && sf[r + TV_RW] > -1e30f) gyd = sub[r + TV_RW] - sub[r];
-      const float qx = spx[r] + sigma * gxd;
-      const float qy = spy[r] + sigma * gyd;
-      const float nrm = fmaxf(1.0f, sqrtf(qx * qx + qy * qy));
-      spx[r] = qx / nrm;
-      spy[r] = qy / nrm;
+    // dual step (dual_at): forward differences of ub over valid pairs; the
+    // norm max(1, sqrt(n2)) is sqrt(max(1, n2))
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        float gxd = 0.0f, gyd = 0.0f;
+        if (right >> j & 1u) gxd = s_ub[ly0 + j][lx + 1] - ub[j];
+        if (below >> j & 1u) gyd = (j + 1 < R ? ub[(j + 1) % R] : s_ub[ly0 + R][lx]) - ub[j];
+        const float qx = px[j] + sigma * gxd;
+        const float qy = py[j] + sigma * gyd;
+        const float n2 = qx * qx + qy * qy;
+        if (plain) {
+          const float nrm = sqrt_round(fmaxf(1.0f, n2)), rn = rcp_round(nrm);
+          px[j] = mh_div(qx, nrm, rn), py[j] = mh_div(qy, nrm, rn);
+        } else {
+          const float nrm = fmaxf(1.0f, sqrtf(n2));
+          px[j] = qx / nrm, py[j] = qy / nrm;
+        }
+        s_px[ly0 + j][lx] = px[j];
+      }
+      s_py[g][lx] = py[R - 1];
     }
     __syncthreads();
-    // primal step and extrapolation (tv_iter_body)
-    for (int r = threadIdx.x; r < TV_RN; r += blockDim.x) {
-      if (!(sf[r] > -1e30f)) {
-        su[r] = sf[r];
-        sub[r] = sf[r];
-        continue;
+    // primal step and extrapolation (tv_iter_body); invalid pixels keep -inf
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const float pxl = has_left ? s_px[ly0 + j][lx - 1] : 0.0f;
+        const float pyu = j > 0 ? py[(j + R - 1) % R] : has_above ? s_py[g - 1][lx] : 0.0f;
+        const float div = (px[j] - pxl) + (py[j] - pyu);
+        const float u0 = u[j];
+        const float num = u0 + tau * div + tf[j];
+        const float un = plain ? mh_div(num, den, rden) : num / den;
+        if (valid >> j & 1u) {
+          u[j] = un;
+          ub[j] = 2.0f * un - u0;
+          s_ub[ly0 + j][lx] = ub[j];
+        }
       }
-      const int lx = r % TV_RW, ly = r / TV_RW, gx = x0 + lx, gy = y0 + ly;
-      const float pxl = (gx > 0 && lx > 0) ? spx[r - 1] : 0.0f;
-      const float pyu = (gy > 0 && ly > 0) ? spy[r - TV_RW] : 0.0f;
-      const float div = (spx[r] - pxl) + (spy[r] - pyu);
-      const float u0 = su[r];
-      const float un = (u0 + tau * div + tau * b.lambda * sf[r]) / (1.0f + tau * b.lambda);
-      su[r] = un;
-      sub[r] = 2.0f * un - u0;
     }
     __syncthreads();
   }
-  for (int k = threadIdx.x; k < TV_TW * TV_TH; k += blockDim.x) {
-    const int lx = TV_K + k % TV_TW, ly = TV_K + k / TV_TW, gx = x0 + lx, gy = y0 + ly;
-    if (gx >= b.W || gy >= b.H) continue;
-    const int r = ly * TV_RW + lx, i = gy * b.W + gx;
-    if (b.depth_in) b.f[i] = sf[r];
+  if (!live || lx < TV_K || lx >= TV_K + TW || gx >= b.W) return;
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int gy = gy0 + j;
+    if (ly0 + j < TV_K || ly0 + j >= TV_K + T::TH || gy >= b.H) continue;
+    const int i = gy * b.W + gx;
     if (b.depth_out) {
-      b.depth_out[i] = sf[r] > -1e30f ? su[r] * 0.001f : NI;
+      b.depth_out[i] = valid >> j & 1u ? u[j] * 0.001f : NI;
     } else {
-      b.u2[i] = su[r], b.ub2[i] = sub[r], b.px2[i] = spx[r], b.py2[i] = spy[r];
+      b.u2[i] = u[j], b.ub2[i] = ub[j], b.px2[i] = px[j], b.py2[i] = py[j];
     }
   }
 }
-__global__ void __launch_bounds__(1024) k_tv_tile(TvTile b) { tv_tile_body(b, blockIdx.x, blockIdx.y); }
 
-int tv_tile_count(int W, int H) { return ((W + TV_TW - 1) / TV_TW) * ((H + TV_TH - 1) / TV_TH); }
+// Tile shapes, largest first.  A launch takes the smallest whose tiles fit the
+// SMs in one wave: the time of a launch is that of one region, so a small image
+// spreads over more SMs although its halos cost more (322x238, 20 iterations:
+// 128 -> 32 us; 640x480 with the largest: 48 us).  The batch, whose scenes fill
+// the GPU together, takes the largest.
+#define TV_SHAPE0 64, 5, 11
+#define TV_SHAPE1 32, 4, 10
+#define TV_SHAPE2 16, 2, 16
+template <int TW, int R, int G>
+__global__ void __launch_bounds__(TvShape<TW, R, G>::THREADS) k_tv_tile(TvTile b) {
+  tv_tile_body<TW, R, G>(b, blockIdx.x, blockIdx.y);
+}
+template <int TW, int R, int G> static bool launch_tv_tile(const TvTile &b, bool any, cudaStream_t s) {
+  typedef TvShape<TW, R, G> T;
+  const dim3 grid((b.W + TW - 1) / TW, (b.H + T::TH - 1) / T::TH);
+  if (!any && (long long)grid.x * grid.y > mh_sm_count()) return false;
+  k_tv_tile<TW, R, G><<<grid, T::THREADS, 0, s>>>(b);
+  return true;
+}
+
+typedef TvShape<TV_SHAPE0> TvBatch;
+int tv_tile_count(int W, int H) { return ((W + 63) / 64) * ((H + TvBatch::TH - 1) / TvBatch::TH); }
 
 // Launch `launch` (of ceil(iterations / TV_K)) of the tiled TV for every
 // active scene: the scenes' tiles are concatenated (Scene::tv_tile0); planes
 // 1-4 of a scene's TV scratch hold the iterate after an even number of
 // launches, planes 5-8 after an odd number.  Bit-identical to the single
 // scene's launches, and so to one launch per iteration.
-__global__ void __launch_bounds__(1024) k_tv_tile_b(const Scene *t, int n, int total, int launch, int iters, int last,
+__global__ void __launch_bounds__(TvBatch::THREADS) k_tv_tile_b(const Scene *t, int n, int total, int launch, int iters, int last,
                                                     float lambda) {
   each_tile(t, n, total, &Scene::tv_tile0, [&](const Scene &c, int lt) {
     const int W = c.d.p.width, H = c.d.p.height;
@@ -224,8 +291,9 @@ __global__ void __launch_bounds__(1024) k_tv_tile_b(const Scene *t, int n, int t
     b.u = A, b.ub = A + np, b.px = A + 2 * np, b.py = A + 3 * np;
     b.u2 = B, b.ub2 = B + np, b.px2 = B + 2 * np, b.py2 = B + 3 * np;
     b.W = W, b.H = H, b.iters = iters, b.lambda = lambda;
-    const int tw = (W + TV_TW - 1) / TV_TW;
-    tv_tile_body(b, lt % tw, lt / tw);
+    const int tw = (W + 63) / 64;
+    tv_tile_body<TV_SHAPE0>(b, lt % tw, lt / tw);
+    __syncthreads();  // the next tile reuses the shared arrays
   });
 }
 
@@ -235,14 +303,8 @@ int launch_denoise_tv_iterated(const Dev &d, float *tv, float lambda, int iterat
 int launch_denoise_tv(const Dev &d, float *tv, float lambda, int iterations, cudaStream_t s) {
   const int W = d.p.width, H = d.p.height, n = W * H;
   if (iterations <= 0) return launch_denoise_tv_iterated(d, tv, lambda, iterations, s);
-  // 87 KB of dynamic shared memory needs the opt-in; the attribute belongs to
-  // the current device, so it is set on every call (it is idempotent)
-  if (cudaFuncSetAttribute(k_tv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTvTileSmem) !=
-      cudaSuccess)
-    return MH_ERR_CUDA;
   float *A[4] = {tv + (size_t)n, tv + 2 * (size_t)n, tv + 3 * (size_t)n, tv + 4 * (size_t)n};
   float *B[4] = {tv + 5 * (size_t)n, tv + 6 * (size_t)n, tv + 7 * (size_t)n, tv + 8 * (size_t)n};
-  const dim3 grid((W + TV_TW - 1) / TV_TW, (H + TV_TH - 1) / TV_TH);
   int launches = 0;
   for (int done = 0; done < iterations; done += TV_K) {
     TvTile b;
@@ -255,7 +317,8 @@ int launch_denoise_tv(const Dev &d, float *tv, float lambda, int iterations, cud
     b.u = A[0], b.ub = A[1], b.px = A[2], b.py = A[3];
     b.u2 = B[0], b.ub2 = B[1], b.px2 = B[2], b.py2 = B[3];
     b.W = W, b.H = H, b.lambda = lambda;
-    k_tv_tile<<<grid, 1024, kTvTileSmem, s>>>(b);
+    if (!launch_tv_tile<TV_SHAPE2>(b, false, s) && !launch_tv_tile<TV_SHAPE1>(b, false, s))
+      launch_tv_tile<TV_SHAPE0>(b, true, s);
     ++launches;
     for (int k = 0; k < 4; ++k) std::swap(A[k], B[k]);
   }
@@ -367,14 +430,11 @@ extern "C" int mh_denoise_tv_static(const float *depth_in, float *depth_out, int
 // per launch (20 iterations: 2 launches instead of 22).
 int launch_batch_tv(const Scene *t, int n, int tv_tiles, float lambda, int iterations, cudaStream_t s) {
   if (iterations <= 0 || tv_tiles <= 0) return MH_OK;
-  if (cudaFuncSetAttribute(k_tv_tile_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTvTileSmem) !=
-      cudaSuccess)
-    return MH_ERR_CUDA;
   const int launches = (iterations + TV_K - 1) / TV_K;
-  const int g = std::max(1, std::min(tv_tiles, mh_sm_count() * 2));
+  const int g = std::max(1, std::min(tv_tiles, mh_sm_count()));
   for (int k = 0; k < launches; ++k) {
     const int iters = std::min(TV_K, iterations - k * TV_K);
-    k_tv_tile_b<<<g, 1024, kTvTileSmem, s>>>(t, n, tv_tiles, k, iters, k == launches - 1 ? 1 : 0, lambda);
+    k_tv_tile_b<<<g, TvBatch::THREADS, 0, s>>>(t, n, tv_tiles, k, iters, k == launches - 1 ? 1 : 0, lambda);
   }
   int count = launches;
   if (launches == 1) {

@@ -64,3 +64,34 @@ def test_tv_matches_fp64_oracle(built):
     moved = np.abs(got[ok] - before[ok]).max()
     print(f"TV vs FP64: max |ddepth| = {err:.3e} m; the denoiser moved depths by up to {moved:.3e} m")
     assert moved > 1e-3 and err <= 1e-5, (err, moved)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (16, 12), (17, 13), (63, 33), (200, 113), (385, 241), (641, 37)])
+def test_tile_shapes_bit_identical_to_per_iteration(built, w, h):
+    """Images of one pixel, one tile and its edges, and each tile shape (the
+    smallest whose tiles fit one wave); depths of every size, below the range
+    in which the quotients need no operator included."""
+    import torch
+    p = config.make_params(w, h, 300.0, 300.0, w / 2, h / 2, voxel_size=0.008, truncation=0.024, bayesian=True,
+                           bucket_count=1 << 10, value_capacity=1 << 10, max_vertex_count=1 << 10,
+                           max_triangle_count=1 << 10)
+    p.min_depth_range = 0.0
+    v = Volume(p)
+    L = _lib.load()
+    rng = np.random.default_rng(w * 1000 + h)
+    for tiny in (False, True):
+        d = rng.uniform(0.5, 4.0, (h, w)).astype(np.float32)
+        d[rng.random((h, w)) < 0.05] = np.inf
+        if tiny:
+            d[rng.random((h, w)) < 0.2] *= np.float32(1e-25)
+        for iters in (1, 10, 13):
+            v.set_frame(d, np.eye(4, dtype=np.float32))
+            prep = v.depth()
+            v.denoise_tv(0.1, iters)
+            got = v.depth()
+            src = torch.from_numpy(prep).cuda()
+            out = torch.empty((h, w), dtype=torch.float32, device="cuda")
+            assert L.mh_denoise_tv_static(C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()), w, h, C.c_float(0.1),
+                                          iters, None) == 0
+            torch.cuda.synchronize()
+            np.testing.assert_array_equal(got.view(np.uint32), out.cpu().numpy().view(np.uint32))
