@@ -14,14 +14,16 @@
 //          where w > 2; sdf_bar = 2 sdf - sdf_prev.
 // Differences use face neighbours that exist, are observed and carry the
 // mask; otherwise the gradient (or divergence) is 0, as in the reference.
-// The per-voxel state (7 words, plus one for the per-call work list) lives in
-// arrays laid out like the voxel storage, allocated on first use; the mask is an epoch stamp, so voxels not
-// initialised by the latest init read as unmasked.  Every pass runs one
-// thread per candidate voxel over a face-neighbour table that is built once
-// per call, so no pass waits on a hash probe.
+// The per-voxel state (7 words) lives in arrays laid out like the voxel
+// storage, allocated on first use; the mask is an epoch stamp, so voxels not
+// initialised by the latest init read as unmasked.  Init runs one thread per
+// candidate voxel, the iterations one CTA per candidate block over a
+// face-neighbour table and per-voxel flags that are built once per call, so no
+// pass waits on a hash probe or tests its neighbours' weights again.
 #include <cstring>
 
 #include "mh_kernels.h"
+#include "mh_round.cuh"
 #include "mh_volume.h"
 
 namespace {
@@ -117,42 +119,81 @@ __global__ void __launch_bounds__(256) k_pd_init(Dev d, PD pd, const int *nbt) {
   }
 }
 
-// Work list of a call: (candidate << 9 | local voxel) of every observed,
-// masked candidate voxel, one CTA per candidate block, one atomic per block.
-// Each voxel's update reads only the previous pass's state, so the order of
-// the list does not change the result.
-__global__ void __launch_bounds__(256) k_pd_list(Dev d, PD pd, unsigned *list, int *count) {
-  __shared__ int wsum[8], base;
-  const int n = cand_count(d);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// The iterations run one 128-thread CTA per candidate block: thread t holds
+// the four voxels x = 4 (t & 1) .. + 3 of row y = t / 2 & 7 of layer z = t / 16,
+// so a field moves as one float4 per thread.
+__device__ __forceinline__ int first_voxel(int t) { return t * 4; }
+
+// Flags of a call, 16 bits a thread: bits 0-3 the voxel is usable, 4-7 its
+// three upper face neighbours are usable too, 8-11 its three lower ones.
+// Neither pass changes the weights or the mask, so they hold for all
+// iterations of the call.
+__global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, uint16_t *flags) {
+  // usable voxels of the block with a layer around it, 10 x 10 x 10
+  __shared__ uint8_t us[1000];
+  const int n = cand_count(d), t = threadIdx.x;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int blk = d.cand[c].w;
-    bool f[2];
+    if (blk < 0) {
+      flags[(size_t)c * 128 + t] = 0;
+      continue;
+    }
+    const int i0 = first_voxel(t);
+    uint8_t *own = us + (i0 & 7) + 1 + 10 * (((i0 >> 3) & 7) + 1) + 100 * ((i0 >> 6) + 1);
+    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + i0;
+    const float4 w = *reinterpret_cast<const float4 *>(d.w + base);
+    const uint4 m = *reinterpret_cast<const uint4 *>(pd.mask + base);
+    own[0] = w.x >= kEps && m.x == pd.epoch, own[1] = w.y >= kEps && m.y == pd.epoch;
+    own[2] = w.z >= kEps && m.z == pd.epoch, own[3] = w.w >= kEps && m.w == pd.epoch;
+    for (int i = t; i < 384; i += 128) {
+      const int face = i >> 6, a = i & 7, b = (i >> 3) & 7, k = face >> 1, up = !(face & 1);
+      const int q = __ldg(nbt + 6 * c + face);  // 2 k: upper, 2 k + 1: lower
+      const int in = up ? 0 : 7, out = up ? 9 : 0;
+      const int li = k == 0 ? in + 8 * a + 64 * b : k == 1 ? a + 8 * in + 64 * b : a + 8 * b + 64 * in;
+      const int o = k == 0 ? out + 10 * (a + 1) + 100 * (b + 1) : k == 1 ? a + 1 + 10 * out + 100 * (b + 1)
+                                                                        : a + 1 + 10 * (b + 1) + 100 * out;
+      us[o] = q >= 0 && usable(d, pd, (long long)q * MH_BLOCK_VOXELS + li);
+    }
+    __syncthreads();
+    unsigned f = 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long g = (long long)blk * MH_BLOCK_VOXELS + threadIdx.x + 256 * h;
-      f[h] = blk >= 0 && d.w[g] >= kEps && pd.mask[g] == pd.epoch;
+    for (int k = 0; k < 4; ++k) {
+      const uint8_t *u = own + k;
+      if (!u[0]) continue;
+      f |= 1u << k;
+      if (u[1] && u[10] && u[100]) f |= 16u << k;
+      if (u[-1] && u[-10] && u[-100]) f |= 256u << k;
     }
-    const unsigned b0 = __ballot_sync(0xffffffffu, f[0]), b1 = __ballot_sync(0xffffffffu, f[1]);
-    if (lane == 0) wsum[wid] = __popc(b0) + __popc(b1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int w = 0; w < 8; ++w) {
-        const int x = wsum[w];
-        wsum[w] = tot;
-        tot += x;
-      }
-      base = tot ? atomicAdd(count, tot) : 0;
-    }
-    __syncthreads();
-    const unsigned lt = (1u << lane) - 1u;
-    int o = base + wsum[wid];
-    if (f[0]) list[o + __popc(b0 & lt)] = ((unsigned)c << 9) | threadIdx.x;
-    o += __popc(b0);
-    if (f[1]) list[o + __popc(b1 & lt)] = ((unsigned)c << 9) | (threadIdx.x + 256);
+    flags[(size_t)c * 128 + t] = (uint16_t)f;
     __syncthreads();
   }
+}
+
+__device__ __forceinline__ float lane4(const float4 &v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+__device__ __forceinline__ float4 load4(const float *f, size_t base) { return *reinterpret_cast<const float4 *>(f + base); }
+__device__ __forceinline__ void store4(float *f, size_t base, const float *v) {
+  *reinterpret_cast<float4 *>(f + base) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// A block's field with the layers above it on each axis, 9 x 9 x 9 (edges and
+// corners unused), and with those below it.
+struct Tile9 {
+  float v[729];
+};
+// own voxels of the tile; off = 1 leaves room for the layers below
+__device__ __forceinline__ void tile_own(Tile9 &s, int t, int off, const float4 &v) {
+  const int i = first_voxel(t);
+  float *o = s.v + (i & 7) + off + 9 * (((i >> 3) & 7) + off) + 81 * ((i >> 6) + off);
+  o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
+}
+// 64 voxels of a neighbour's face of axis k: its first layer (up) or its last
+__device__ __forceinline__ void tile_face(Tile9 &s, int i, int k, bool up, int q, const float *field) {
+  if (q < 0) return;  // no voxel here has the neighbour: the flags say so
+  const int a = i & 7, b = i >> 3, in = up ? 0 : 7, out = up ? 8 : 0, off = up ? 0 : 1;
+  const int li = k == 0 ? in + 8 * a + 64 * b : k == 1 ? a + 8 * in + 64 * b : a + 8 * b + 64 * in;
+  const int o = k == 0 ? out + 9 * (a + off) + 81 * (b + off) : k == 1 ? a + off + 9 * out + 81 * (b + off)
+                                                                      : a + off + 9 * (b + off) + 81 * out;
+  s.v[o] = __ldg(field + (size_t)q * MH_BLOCK_VOXELS + li);
 }
 
 template <int NV> __device__ __forceinline__ void cta_sum(float (&v)[NV], double *acc) {
@@ -171,64 +212,130 @@ template <int NV> __device__ __forceinline__ void cta_sum(float (&v)[NV], double
   }
 }
 
-// dual step and energies (PrimalDualIteratePass1Kernel)
-__global__ void __launch_bounds__(256) k_pd_dual(Dev d, PD pd, const int *nbt, const unsigned *list,
-                                                 const int *count, float sigma, double *err) {
-  const int n = *count;
-  float e[2] = {0.0f, 0.0f};
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const unsigned code = list[t];
-    const int c = (int)(code >> 9), li = (int)(code & 511);
-    const int blk = d.cand[c].w;
-    const long long g = (long long)blk * MH_BLOCK_VOXELS + li;
-    long long q[3];
-    faces<1>(nbt, c, blk, li, q);
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) ok &= usable(d, pd, q[k]);
-    const float s = d.sdf[g], b = pd.bar[g];
-    float gs[3] = {0.0f, 0.0f, 0.0f}, gb[3] = {0.0f, 0.0f, 0.0f};
-    if (ok) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) gs[k] = d.sdf[q[k]] - s, gb[k] = pd.bar[q[k]] - b;
-    }
-    const float dd = fabsf(s - pd.sdf0[g]);
-    e[0] += dd * dd;
-    e[1] += huber(sqrtf(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]), kAlpha);
-    float px = pd.px[g] + sigma * gb[0], py = pd.py[g] + sigma * gb[1], pz = pd.pz[g] + sigma * gb[2];
-    const float h = 1.0f + sigma * kAlpha;
-    px /= h, py /= h, pz /= h;
-    const float nrm = fmaxf(1.0f, sqrtf(px * px + py * py + pz * pz));
-    pd.px[g] = px / nrm, pd.py[g] = py / nrm, pd.pz[g] = pz / nrm;
-  }
-  cta_sum<2>(e, err);
+// a / b for y = RN(1 / b), b of moderate size: without the operator's tests,
+// which send the many zeros down its long way (the sign of a zero is not kept:
+// nothing depends on it)
+__device__ __forceinline__ float pd_div(float a, float b, float y) {
+  const float m = fabsf(a);
+  return (m > 0x1p-60f && m < 0x1p60f) || m == 0.0f ? mh_div(a, b, y) : a / b;
 }
 
-// primal step and extrapolation (PrimalDualIteratePass2Kernel)
-__global__ void __launch_bounds__(256) k_pd_primal(Dev d, PD pd, const int *nbt, const unsigned *list,
-                                                   const int *count, float lambda, float tau) {
-  const int n = *count;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const unsigned code = list[t];
-    const int c = (int)(code >> 9), li = (int)(code & 511);
+// Dual step (PrimalDualIteratePass1Kernel), with the energies where they are
+// asked for.  Bound by the traffic: 28 B a voxel (the extrapolated sdf and the
+// dual read, the dual written; 8 more for the energies) and the faces: 390 us
+// for 120 k blocks.  One thread per entry of
+// a list of usable voxels took 660 us and read 12 B more a voxel; with the
+// operators' divisions this form takes 700 us.
+template <bool kEnergy>
+__global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, const uint16_t *flags, float sigma,
+                                                 double *err) {
+  __shared__ Tile9 bar, sdf;
+  const int n = cand_count(d), t = threadIdx.x;
+  const float h = 1.0f + sigma * kAlpha, rh = 1.0f / h;
+  const bool h_ok = h > 0x1p-20f && h < 0x1p20f;
+  float e[2] = {0.0f, 0.0f};
+  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+    const unsigned f = flags[(size_t)c * 128 + t];
+    if (!__syncthreads_or(f)) continue;
     const int blk = d.cand[c].w;
-    const long long g = (long long)blk * MH_BLOCK_VOXELS + li;
-    long long q[3];
-    faces<-1>(nbt, c, blk, li, q);
-    bool ok = true;
+    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
+    const float4 B = load4(pd.bar, base), X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
+    float4 S, S0;
+    if (kEnergy) S = load4(d.sdf, base), S0 = load4(pd.sdf0, base);
+    tile_own(bar, t, 0, B);
+    if (kEnergy) tile_own(sdf, t, 0, S);
+    for (int i = t; i < 192; i += 128) {
+      const int k = i >> 6, q = __ldg(nbt + 6 * c + 2 * k);
+      tile_face(bar, i & 63, k, true, q, pd.bar);
+      if (kEnergy) tile_face(sdf, i & 63, k, true, q, d.sdf);
+    }
+    __syncthreads();
+    const int i0 = first_voxel(t), o0 = (i0 & 7) + 9 * ((i0 >> 3) & 7) + 81 * (i0 >> 6);
+    float px[4], py[4], pz[4];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) ok &= usable(d, pd, q[k]);
-    float div = 0.0f;
-    if (ok) div = (pd.px[q[0]] - pd.px[g]) + (pd.py[q[1]] - pd.py[g]) + (pd.pz[q[2]] - pd.pz[g]);
-    const float prev = d.sdf[g], s0 = pd.sdf0[g], w = pd.w[g];
-    const float lam = lambda * w;
-    float s = prev - tau * div;
-    s = (s + lam * tau * s0) / (1.0f + lam * tau);
-    if (w > 2.0f) s = s0;
-    d.sdf[g] = s;
-    if (!sdf_nonneg(s) && sdf_nonneg(prev))
-      atomicOr(d.neg + blk, 1ull << (((li >> 1) & 3) | ((li >> 2) & 12) | ((li >> 3) & 48)));
-    pd.bar[g] = 2.0f * s - prev;
+    for (int k = 0; k < 4; ++k) {
+      px[k] = lane4(X, k), py[k] = lane4(Y, k), pz[k] = lane4(Z, k);
+      if (!(f >> k & 1u)) continue;
+      const float b = lane4(B, k);
+      const float *o = bar.v + o0 + k;
+      float gb[3] = {0.0f, 0.0f, 0.0f};
+      if (f >> (4 + k) & 1u) gb[0] = o[1] - b, gb[1] = o[9] - b, gb[2] = o[81] - b;
+      if (kEnergy) {
+        const float s = lane4(S, k);
+        const float *os = sdf.v + o0 + k;
+        float gs[3] = {0.0f, 0.0f, 0.0f};
+        if (f >> (4 + k) & 1u) gs[0] = os[1] - s, gs[1] = os[9] - s, gs[2] = os[81] - s;
+        const float dd = fabsf(s - lane4(S0, k));
+        e[0] += dd * dd;
+        e[1] += huber(sqrtf(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]), kAlpha);
+      }
+      float x = px[k] + sigma * gb[0], y = py[k] + sigma * gb[1], z = pz[k] + sigma * gb[2];
+      if (h_ok) x = pd_div(x, h, rh), y = pd_div(y, h, rh), z = pd_div(z, h, rh);
+      else x /= h, y /= h, z /= h;
+      // max(1, sqrt(n2)) is sqrt(max(1, n2))
+      const float n2 = x * x + y * y + z * z;
+      if (n2 < 0x1p60f) {
+        const float nrm = sqrt_round(fmaxf(1.0f, n2)), rn = rcp_round(nrm);
+        px[k] = pd_div(x, nrm, rn), py[k] = pd_div(y, nrm, rn), pz[k] = pd_div(z, nrm, rn);
+      } else {
+        const float nrm = fmaxf(1.0f, sqrtf(n2));
+        px[k] = x / nrm, py[k] = y / nrm, pz[k] = z / nrm;
+      }
+    }
+    if (f) store4(pd.px, base, px), store4(pd.py, base, py), store4(pd.pz, base, pz);
+    __syncthreads();
+  }
+  if (kEnergy) cta_sum<2>(e, err);
+}
+
+// Primal step and extrapolation (PrimalDualIteratePass2Kernel).  Bound by the
+// traffic: 32 B a voxel (the dual, sdf, sdf0 and the weight read, sdf and its
+// extrapolation written) and the faces: 382 us for 120 k blocks, 5.1 TB/s
+// without the faces.
+__global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt, const uint16_t *flags, float lambda,
+                                                   float tau) {
+  __shared__ Tile9 tx, ty, tz;
+  const int n = cand_count(d), t = threadIdx.x;
+  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+    const unsigned f = flags[(size_t)c * 128 + t];
+    if (!__syncthreads_or(f)) continue;
+    const int blk = d.cand[c].w;
+    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
+    const float4 X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
+    const float4 S = load4(d.sdf, base), S0 = load4(pd.sdf0, base), Wt = load4(pd.w, base);
+    tile_own(tx, t, 1, X), tile_own(ty, t, 1, Y), tile_own(tz, t, 1, Z);
+    for (int i = t; i < 192; i += 128) {
+      const int k = i >> 6, q = __ldg(nbt + 6 * c + 2 * k + 1);
+      if (k == 0) tile_face(tx, i & 63, 0, false, q, pd.px);
+      else if (k == 1) tile_face(ty, i & 63, 1, false, q, pd.py);
+      else tile_face(tz, i & 63, 2, false, q, pd.pz);
+    }
+    __syncthreads();
+    const int i0 = first_voxel(t), o0 = (i0 & 7) + 1 + 9 * (((i0 >> 3) & 7) + 1) + 81 * ((i0 >> 6) + 1);
+    float so[4] = {S.x, S.y, S.z, S.w}, bo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      bo[k] = 0.0f;
+      if (!(f >> k & 1u)) continue;
+      float div = 0.0f;
+      if (f >> (8 + k) & 1u) {
+        const int o = o0 + k;
+        div = (tx.v[o - 1] - lane4(X, k)) + (ty.v[o - 9] - lane4(Y, k)) + (tz.v[o - 81] - lane4(Z, k));
+      }
+      const float prev = so[k], s0 = lane4(S0, k), w = lane4(Wt, k);
+      const float lam = lambda * w;
+      float s = prev - tau * div;
+      s = (s + lam * tau * s0) / (1.0f + lam * tau);
+      if (w > 2.0f) s = s0;
+      so[k] = s;
+      bo[k] = 2.0f * s - prev;
+    }
+    // voxels that are not usable keep their sdf; their extrapolation is not read
+    if (f) store4(d.sdf, base, so), store4(pd.bar, base, bo);
+    // a warp holds two layers of the block, as in the fusion kernels
+    const unsigned neg = neg_bits(make_float4(so[0], so[1], so[2], so[3]));
+    if ((t & 31) == 0) reinterpret_cast<uint16_t *>(d.neg + blk)[t >> 5] = (uint16_t)neg;
+    __syncthreads();
   }
 }
 
@@ -239,15 +346,15 @@ struct mh_pd_state {
   size_t voxels = 0;
   double *err = nullptr;
   int *nbt = nullptr;   // face-neighbour table of the candidate list (6 per candidate)
-  unsigned *list = nullptr;  // work list of the call (one entry per observed, masked voxel)
-  int *count = nullptr;      // its length
+  uint16_t *flags = nullptr;  // per-voxel flags of the call (128 words per candidate)
+  bool fresh = false;         // no iteration since the last init: bar and p are 0
 };
 
-static int grid_of(const void *fn) { return mh_resident_grid(fn, 256, 8); }
+static int grid_of(const void *fn, int block = 256) { return mh_resident_grid(fn, block, 2048 / block); }
 
 static int pd_ensure(mh_volume *v) {
   if (v->pd) return MH_OK;
-  if (v->hp.value_capacity > (1u << 23)) return MH_ERR_INVALID;  // work-list entries hold candidate << 9
+  if (v->hp.value_capacity > (1u << 23)) return MH_ERR_INVALID;
   mh_pd_state *st = new mh_pd_state();
   const size_t nv = (size_t)v->hp.value_capacity * MH_BLOCK_VOXELS;
   float **f[6] = {&st->pd.sdf0, &st->pd.bar, &st->pd.w, &st->pd.px, &st->pd.py, &st->pd.pz};
@@ -256,8 +363,7 @@ static int pd_ensure(mh_volume *v) {
   ok = ok && cudaMalloc((void **)&st->pd.mask, sizeof(unsigned) * nv) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->err, sizeof(double) * 2) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->nbt, sizeof(int) * 6 * (size_t)v->hp.value_capacity) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&st->list, sizeof(unsigned) * nv) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&st->count, sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->flags, sizeof(uint16_t) * 128 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMemset(st->pd.mask, 0, sizeof(unsigned) * nv) == cudaSuccess;
   st->pd.epoch = 0;
   st->voxels = nv;
@@ -275,7 +381,7 @@ void mh_pd_free(mh_volume *v) {
   if (!st) return;
   for (void *p : {(void *)st->pd.sdf0, (void *)st->pd.bar, (void *)st->pd.w, (void *)st->pd.px, (void *)st->pd.py,
                   (void *)st->pd.pz, (void *)st->pd.mask, (void *)st->err, (void *)st->nbt,
-                  (void *)st->list, (void *)st->count})
+                  (void *)st->flags})
     if (p) cudaFree(p);
   delete st;
   v->pd = nullptr;
@@ -293,6 +399,7 @@ int mh_huber_tv_init(mh_volume *v, void *stream) {
   k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
   k_pd_init<<<grid_of((const void *)k_pd_init), 256, 0, s>>>(v->d, st->pd, st->nbt);
   mh_count_launches(2);
+  st->fresh = true;
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 
@@ -305,18 +412,23 @@ int mh_huber_tv_iterate(mh_volume *v, float lambda, float sigma, float tau, int 
   double last[2] = {0.0, 0.0};
   if (iterations > 0) {
     // the candidate list may have changed since init: rebuild the face table
-    // and the work list of this call (neither pass changes w or the mask)
+    // and the flags of this call (neither pass changes w or the mask)
     k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-    MH_CUDA_TRY(cudaMemsetAsync(st->count, 0, sizeof(int), s));
-    k_pd_list<<<grid_of((const void *)k_pd_list), 256, 0, s>>>(v->d, st->pd, st->list, st->count);
+    k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags);
+    MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2, s));
     mh_count_launches(2);
   }
-  const int gd = grid_of((const void *)k_pd_dual), gp = grid_of((const void *)k_pd_primal);
+  const int gd = grid_of((const void *)k_pd_dual<false>, 128), ge = grid_of((const void *)k_pd_dual<true>, 128),
+            gp = grid_of((const void *)k_pd_primal, 128);
   for (int it = 0; it < iterations; ++it) {
-    MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2, s));
-    k_pd_dual<<<gd, 256, 0, s>>>(v->d, st->pd, st->nbt, st->list, st->count, sigma, st->err);
-    k_pd_primal<<<gp, 256, 0, s>>>(v->d, st->pd, st->nbt, st->list, st->count, lambda, tau);
-    mh_count_launches(2);
+    // only the last pass's energies are returned; the first dual step after
+    // init leaves p = 0 (bar is 0)
+    const bool last = it + 1 == iterations;
+    if (last) k_pd_dual<true><<<ge, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, sigma, st->err);
+    else if (!st->fresh) k_pd_dual<false><<<gd, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, sigma, nullptr);
+    k_pd_primal<<<gp, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, lambda, tau);
+    mh_count_launches(last || !st->fresh ? 2 : 1);
+    st->fresh = false;
   }
   MH_CUDA_TRY(cudaGetLastError());
   if (energy && iterations > 0) {

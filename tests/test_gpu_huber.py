@@ -118,3 +118,36 @@ def test_huber_tv_iterate_before_init_is_refused(built):
         v.huber_tv_iterate(1.0, 8.0, 0.01, 1)
     with pytest.raises(MeshHashError):
         v.huber_tv_init() or v.huber_tv_iterate(1.0, 8.0, 0.01, -1)
+
+
+@pytest.mark.parametrize("cells,scale", [([(0, 0, 0)], 1.0), ([(0, 0, 0), (1, 0, 0)], 1.0),
+                                         ([(0, 0, 0), (0, 1, 0), (0, 0, 1), (-1, -1, -1)], 1.0),
+                                         ([(x, y, z) for x in range(3) for y in range(3) for z in range(3)], 1.0),
+                                         ([(0, 0, 0), (1, 0, 0), (0, 0, 1)], 1e-22)])
+def test_huber_tv_block_edges(built, cells, scale):
+    """Blocks alone, side by side and diagonal, with unobserved voxels at
+    their faces, a neighbour that is masked but no longer a candidate, and
+    values too small for quotients without the operator's tests."""
+    wl = scene.small_circle(4)
+    p = config.params_for(wl, value_capacity=1 << 10, bucket_count=1 << 10, max_vertex_count=1 << 10,
+                          max_triangle_count=1 << 10)
+    rng = np.random.default_rng(len(cells))
+    pos = np.array(cells, np.int32)
+    sdf = (rng.uniform(-0.02, 0.02, (len(cells), 512)) * scale).astype(np.float32)
+    w = np.where(rng.random((len(cells), 512)) < 0.2, 0.0, 5.0).astype(np.float32)
+    v, o = Volume(p), Oracle(p, fp64=False)
+    v.load_blocks(pos, sdf, w)
+    o.set_blocks(pos, sdf, w, np.zeros_like(w), np.zeros_like(w))
+    for x in (v, o):
+        x.set_candidates(pos)
+        x.huber_tv_init()
+    for keep in (pos, pos[:max(1, len(pos) - 1)]):
+        v.set_candidates(keep)
+        o.set_candidates(keep)
+        for iters in (1, 2, 3):
+            e, eo = v.huber_tv_iterate(2.0, 8.0, 0.01, iters), o.huber_tv_iterate(2.0, 8.0, 0.01, iters)
+            np.testing.assert_allclose(e, eo, rtol=1e-4, atol=1e-30)
+        _, got, _ = _sorted(v)
+        _, want = _oracle_sdf(o)
+        # the data weight is exp() of two libraries, a few units apart
+        np.testing.assert_allclose(got, want, rtol=0, atol=2e-6 * np.abs(sdf).max())
