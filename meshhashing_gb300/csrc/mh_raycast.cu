@@ -25,9 +25,10 @@
 //    the hash table through a register cache;
 //  * all state in registers: one sampler serves the march, the previous sample
 //    and the regula falsi (a phase variable picks the next position);
-//  * a warp covers 8x4 pixels, so its rays cross the same cells.
+//  * a warp covers 8x4 pixels, so its rays cross the same cells; in small
+//    images, which leave the chip's lanes idle, 4 or 8 lanes share a ray.
 // A 640x480 view of the 4 mm map (461 k blocks, grid included): 1.99 -> 0.39
-// ms against hash lookups and block-wide skips; 161x119 at 8 mm: 0.46 -> 0.15
+// ms against hash lookups and block-wide skips; 161x119 at 8 mm: 0.46 -> 0.09
 // ms.  What is left is latency: a ray's evaluations follow one another, two
 // dependent loads and about 200 instructions each, and the rays with many of
 // them (along surfaces, behind walls) end last.
@@ -43,11 +44,18 @@
 #define RC_TY 8
 #define GR_TX 16
 #define GR_TY 8
+// threads of a CTA where lanes share rays
+#define RC_GROUP_THREADS 256
 // Lanes with a sample to evaluate before a warp leaves the search for it.  All
 // 32 is the fewest evaluations, but every lane waits for the longest search;
 // 640x480 / 161x119 views, us: 32: 549 / 252, 16: 475 / 204, 8: 463 / 191,
 // 4: 437 / 180, 2: 476 / 185, 1: 527 / 225.
 #define RC_WAIT 4
+// The same where lanes share a ray: lanes of half a warp's rays.
+#define RC_GROUP_WAIT 16
+// Largest images of which 8 lanes and 4 lanes share a ray, see launch_raycast.
+#define RC_PIXELS8 65536
+#define RC_PIXELS4 131072
 
 // ------------------------------------------------------------------ forward
 // The forward march keeps its whole state in registers: one sampler is
@@ -68,6 +76,7 @@ namespace {
 enum { SM_OK = 0, SM_MISS0 = 1, SM_MISS0_NEW = 2, SM_MISS = 3 };
 
 struct Nbhd {
+  static constexpr int LANES = 1;
   int bx, by, bz;    // block of the first corner of the last sample
   unsigned looked;   // bit n: block n = (bx, by, bz) + (n & 1, n >> 1 & 1, n >> 2 & 1) looked up
   unsigned miss;     // bit n: block n is missing
@@ -83,8 +92,25 @@ struct Nbhd {
 // The blocks of a sample from the view's dense array; only the first corner's
 // block is remembered.
 struct DenseNbhd {
+  static constexpr int LANES = 1;
   int bx, by, bz;
   __device__ __forceinline__ void init() { bx = by = bz = 0x7fffffff; }
+};
+
+// The same for G lanes that share a ray, lanes base .. base + G - 1 of the
+// warp: lane j holds corners 8 / G j and up.
+template <int G> struct GroupNbhd {
+  static constexpr int LANES = G;
+  int j;
+  unsigned base;
+  unsigned lanes;  // the warp's lanes that sample together, whole groups
+  __device__ __forceinline__ void init() {
+    j = threadIdx.x & (G - 1);
+    base = threadIdx.x & 31 & ~(G - 1);
+    lanes = 0xffffffffu;
+  }
+  // the group's bits of a warp ballot
+  __device__ __forceinline__ unsigned of(unsigned ballot) const { return (ballot >> base) & ((1u << G) - 1u); }
 };
 
 // Corner voxels of GetSpatialValue at pos (both of each axis) and the
@@ -209,6 +235,34 @@ __device__ __forceinline__ int nb_sample(const Dev &d, N &c, F3 pos, bool want, 
   return SM_OK;
 }
 
+// 8 / G corners a lane; every lane of the group gets the result.
+template <int G>
+__device__ __forceinline__ int nb_sample(const Dev &d, GroupNbhd<G> &c, F3 pos, bool, float &s) {
+  const Corners k = corners_at(d.p, pos);
+  const RayGrid &g = d.grid;
+  float v[8 / G];
+  bool there = true;
+#pragma unroll
+  for (int q = 0; q < 8 / G; ++q) {
+    const int i = c.j * (8 / G) + q;
+    const bool mx = i & 4, my = i & 2, mz = i & 1;
+    const int vx = mx ? k.v1x : k.v0x, vy = my ? k.v1y : k.v0y, vz = mz ? k.v1z : k.v0z;
+    const unsigned bx = min((unsigned)((vx >> 3) - g.bx), g.bnx - 1u), by = min((unsigned)((vy >> 3) - g.by), g.bny - 1u),
+                   bz = min((unsigned)((vz >> 3) - g.bz), g.bnz - 1u);
+    const unsigned b = __ldg(g.blocks + (bz * g.bny + by) * g.bnx + bx) ^ g.tag;
+    float x = 0.0f;
+    if (b < 0x1000000u) x = __ldg(d.sdf + (size_t)b * MH_BLOCK_VOXELS + (vx & 7) + (vy & 7) * 8 + (vz & 7) * 64);
+    else there = false;
+    v[q] = (mx ? k.rx : 1.0f - k.rx) * (my ? k.ry : 1.0f - k.ry) * (mz ? k.rz : 1.0f - k.rz) * x;
+  }
+  const bool ok = c.of(__ballot_sync(c.lanes, there)) == (1u << G) - 1u;
+  float acc = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc += __shfl_sync(c.lanes, v[i % (8 / G)], c.base + i / (8 / G));
+  s = acc;
+  return ok ? SM_OK : SM_MISS;
+}
+
 // One axis of a slab test with the direction's reciprocal: narrows [lo, hi]
 // to the t for which the ray's coordinate lies inside (a, b).  The bounds
 // carry a few ulp of rounding; the box margins below absorb them.
@@ -316,6 +370,36 @@ __device__ __forceinline__ bool search_step(const RayGrid &g, const GridRay &r, 
   return false;
 }
 
+// 4 G samples of it at once, four a lane, for the group's ray (active:
+// t is to move).  All 32 lanes call it.
+//
+// The march's t is t + step rounded, again and again.  While t keeps its
+// exponent every step adds the same multiple d of its last place, unless step
+// lies halfway between two multiples and they alternate; two equal steps rule
+// that out.  Then t after n steps is t + n d, exactly, and a lane gets its
+// samples with one multiply-add; else it takes the steps.
+template <int G>
+__device__ __forceinline__ bool search_step(const RayGrid &g, const GridRay &r, unsigned base, const GroupNbhd<G> &p,
+                                            float step, bool active, float &t, float &tl) {
+  float s0 = t, before = tl;  // this lane's first sample and the one before it
+  const float t1 = t + step, d = t1 - t, end = fmaf((float)(4 * G), d, t);
+  if (t1 + step - t1 == d && (__float_as_uint(t) ^ __float_as_uint(end)) < 0x800000u) {
+    s0 = fmaf((float)(4 * p.j), d, t);
+    if (p.j) before = fmaf((float)(4 * p.j - 1), d, t);
+  } else {
+    for (int i = 0; i < 4 * p.j; ++i) before = s0, s0 += step;
+  }
+  // where the ray goes on and the sample before, as far as this lane knows
+  float next = s0, last = before;
+  const bool mine = search_step(g, r, base, step, next, last);
+  const unsigned hits = p.of(__ballot_sync(0xffffffffu, mine));
+  const int from = p.base + (hits ? __ffs(hits) - 1 : G - 1);
+  next = __shfl_sync(0xffffffffu, next, from);
+  last = __shfl_sync(0xffffffffu, last, from);
+  if (active) t = next, tl = last;
+  return hits != 0u;
+}
+
 // The sample n steps before t of a march through `first`, or `first` if there
 // are fewer between them.
 __device__ __forceinline__ float step_back(float first, float t, float step, int n) {
@@ -362,6 +446,30 @@ __device__ __forceinline__ float skip_missing(const Dev &d, const Nbhd &c, F3 ca
   return x;
 }
 
+// A sample a lane at a time; c.lanes scan together.
+template <int G>
+__device__ __forceinline__ float skip_missing(const Dev &d, const GroupNbhd<G> &c, F3 cam, F3 wd, float step, float x,
+                                              float end) {
+  const RayGrid &g = d.grid;
+  while (true) {
+    float q = x, next = x;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      if (i == c.j) q = next;
+      next += step;
+    }
+    const Corners k = corners_at(d.p, f3(cam.x + q * wd.x, cam.y + q * wd.y, cam.z + q * wd.z));
+    const unsigned bx = min((unsigned)((k.v0x >> 3) - g.bx), g.bnx - 1u),
+                   by = min((unsigned)((k.v0y >> 3) - g.by), g.bny - 1u),
+                   bz = min((unsigned)((k.v0z >> 3) - g.bz), g.bnz - 1u);
+    const bool stop = !(q < end) || (__ldg(g.blocks + (bz * g.bny + by) * g.bnx + bx) ^ g.tag) < 0x1000000u;
+    const unsigned hits = c.of(__ballot_sync(c.lanes, stop));
+    const float at = __shfl_sync(c.lanes, q, c.base + (hits ? __ffs(hits) - 1 : 0));
+    if (__all_sync(c.lanes, hits != 0u)) return at;
+    x = hits ? at : next;  // the groups go on together
+  }
+}
+
 }  // namespace
 
 // What one ray's march found: whether a hit was accepted, the two march
@@ -379,10 +487,10 @@ struct March {
 // ray cam + t * wd, t from t_min while t < t_max, with the exact skips
 // described above; spacing > 0 also evaluates GetSpatialSDFGradient at the hit
 // with central differences `spacing` voxels either side (spatial_query.h:68-97
-// uses 0.5).  All 32 lanes of a warp call it (active: the lane has a ray): it
-// keeps them together, searching in one loop and evaluating, whatever their
-// phases, in one inlined sampler, so that neither waits for lanes of the other
-// kind that left the loop at another place.
+// uses 0.5).  All 32 lanes of a warp call it, with their group's ray where lanes
+// share one (active: there is a ray): it keeps them together, searching in one
+// loop and evaluating, whatever their phases, in one inlined sampler, so that
+// neither waits for lanes of the other kind that left the loop at another place.
 template <class N>
 __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3 wd, float t_min, float t_max,
                                            float spacing) {
@@ -412,21 +520,28 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
     unsigned searching;
 #pragma unroll 1
     while ((searching = __ballot_sync(0xffffffffu, phase == PH_SEARCH)) != 0u &&
-           __popc(__ballot_sync(0xffffffffu, phase > PH_SEARCH)) < RC_WAIT) {
+           __popc(__ballot_sync(0xffffffffu, phase > PH_SEARCH)) < (N::LANES > 1 ? RC_GROUP_WAIT : RC_WAIT)) {
+      bool found = false;
+      if constexpr (N::LANES > 1) {  // the warp's groups step together
+        const bool mine = phase == PH_SEARCH && t < t_max;
+        found = search_step(d.grid, gr, gbase, c, step, mine, t, tl) && mine;
+      }
       if (phase == PH_SEARCH) {
-        const bool found = t < t_max && (!use_grid || search_step(d.grid, gr, gbase, step, t, tl));
+        if constexpr (N::LANES == 1) found = t < t_max && (!use_grid || search_step(d.grid, gr, gbase, step, t, tl));
         if (!(t < t_max)) phase = PH_DONE;
         else if (found) phase = PH_MARCH;
       }
       __syncwarp();
     }
     if (!searching && !__any_sync(0xffffffffu, phase != PH_DONE)) break;
+    if constexpr (N::LANES > 1) c.lanes = __ballot_sync(0xffffffffu, phase > PH_SEARCH);
     if (phase > PH_SEARCH) {
       float tp = phase == PH_MARCH ? t : x;
       if (phase == PH_REFINE) tp = m = l + (ls / (ls - rs)) * (r - l);
       const F3 pos = f3(cam.x + tp * wd.x, cam.y + tp * wd.y, cam.z + tp * wd.z);
       float s = 0.0f;
       const int res = nb_sample(d, c, pos, phase != PH_SCAN, s);
+      if constexpr (N::LANES > 1) c.lanes = __ballot_sync(c.lanes, phase == PH_SCAN);
       bool refine = false, resume = false;  // start the regula falsi / go on after the negative sample at t
       if (phase == PH_MARCH) {
         if (res == SM_OK && s < 0.0f && tl != NI && prev_t != tl) {
@@ -503,6 +618,7 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
     __syncwarp();
   }
   // the gradient's samples, axis by axis, minus side first
+  if constexpr (N::LANES > 1) c.lanes = __ballot_sync(0xffffffffu, out.hit && spacing > 0.0f);
   if (out.hit && spacing > 0.0f) {
     const F3 iso = f3(cam.x + out.m * wd.x, cam.y + out.m * wd.y, cam.z + out.m * wd.z);
     const float h = spacing * vs;
@@ -529,16 +645,17 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
 template <class N, int TX, int TY>
 __device__ __forceinline__ void raycast_body(const Dev &d, int tile_x, int tile_y, float *out_depth, float4 *out_vert, float4 *out_norm) {
   __shared__ float sm[32];
-  const int tid = threadIdx.x + threadIdx.y * TX;
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
   if (tid < 16) sm[tid] = d.fc->rc_wTc[tid];
   else if (tid < 32) sm[tid] = d.fc->rc_cTw[tid - 16];
   __syncthreads();
   const float *wTc = sm, *cTw = sm + 16;
   const DevParams &p = d.p;
-  // a warp covers 8x4 pixels
-  const int warp = tid >> 5, wx = TX / 8;
-  const unsigned x = tile_x * TX + (warp % wx) * 8 + (tid & 7);
-  const unsigned y = tile_y * TY + (warp / wx) * 4 + ((tid >> 3) & 3);
+  // a warp covers 8x4 pixels; 2x2 or 4x2 where 8 or 4 lanes share one
+  constexpr int WX = N::LANES == 8 ? 2 : N::LANES == 4 ? 4 : 8, WY = 32 / N::LANES / WX;
+  const int warp = tid >> 5, ray = (tid & 31) / N::LANES, wx = TX / WX;
+  const unsigned x = tile_x * TX + (warp % wx) * WX + ray % WX;
+  const unsigned y = tile_y * TY + (warp / wx) * WY + ray / WX;
   const bool inside = x < p.rc_width && y < p.rc_height;
   const size_t pix = (size_t)y * p.rc_width + x;
   const float NI = -__int_as_float(0x7f800000);
@@ -568,13 +685,20 @@ __device__ __forceinline__ void raycast_body(const Dev &d, int tile_x, int tile_
       o_norm = make_float4(nc.x, nc.y, nc.z, 1.0f);
     }
   }
-  if (out_depth) out_depth[pix] = o_depth;
-  if (out_vert) out_vert[pix] = o_vert;
-  if (out_norm) out_norm[pix] = o_norm;
+  // a group's lanes write an image each
+  const int lane = tid & (N::LANES - 1);
+  if (out_depth && (N::LANES == 1 || lane == 0)) out_depth[pix] = o_depth;
+  if (out_vert && (N::LANES == 1 || lane == 1)) out_vert[pix] = o_vert;
+  if (out_norm && (N::LANES == 1 || lane == 2)) out_norm[pix] = o_norm;
 }
 template <class N>
 __global__ void __launch_bounds__(RC_TX *RC_TY, 12) k_raycast(Dev d, float *out_depth, float4 *out_vert, float4 *out_norm) {
   raycast_body<N, RC_TX, RC_TY>(d, blockIdx.x, blockIdx.y, out_depth, out_vert, out_norm);
+}
+template <int G>
+__global__ void __launch_bounds__(RC_GROUP_THREADS, 4) k_raycast_group(Dev d, float *out_depth, float4 *out_vert,
+                                                                       float4 *out_norm) {
+  raycast_body<GroupNbhd<G>, 32 / G, RC_GROUP_THREADS / 32>(d, blockIdx.x, blockIdx.y, out_depth, out_vert, out_norm);
 }
 // batched raycast over the scenes' concatenated TX x TY tiles; the tile shape
 // is an autotuned choice (the scene table's ray_tile0 follows it)
@@ -807,13 +931,26 @@ int launch_count_flags(const uint8_t *flags, int n, int *out, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 
+// A ray is a chain of dependent steps of about 1000 cycles each.  Lanes that
+// share one search 4 G samples at once and evaluate with 8 / G corners each,
+// which shortens the chain but takes more instructions in all (the position's
+// and the state's on every lane), so it is for images that cannot fill the
+// chip: 152 SMs x 768 lanes are 117 k.  Views of a 24-frame map, us, with
+// 1 / 4 / 8 lanes a ray: 100x75, 8 mm: 190 / 146 / 110; 160x120, 4 mm: 356 /
+// 230 / 188; 240x180, 6 mm: 202 / 156 / 129; 320x240, 4 mm: 475 / 350 / 332;
+// 320x240, 8 mm: 161 / 135 / 146; 400x300, 6 mm: 205 / 200 / 226; 450x340, 5
+// mm: 243 / 242 / 276; 640x480, 6 mm: 263 / 346 / 442.  Needs the dense array.
 int launch_raycast(const Dev &d, float *depth, float *vert4, float *norm4, cudaStream_t s) {
   const int r = fill_ray_grid(d, s);
   if (r != MH_OK) return r;
-  dim3 blk(RC_TX, RC_TY);
-  dim3 grid((d.p.rc_width + RC_TX - 1) / RC_TX, (d.p.rc_height + RC_TY - 1) / RC_TY);
+  const size_t pixels = (size_t)d.p.rc_width * d.p.rc_height;
+  const int lanes = !d.grid.bits || !d.grid.blocks || pixels > RC_PIXELS4 ? 1 : pixels > RC_PIXELS8 ? 4 : 8;
+  const unsigned tx = lanes > 1 ? 32 / lanes : RC_TX, ty = lanes > 1 ? RC_GROUP_THREADS / 32 : RC_TY;
+  const dim3 blk(RC_TX, RC_TY), grid((d.p.rc_width + tx - 1) / tx, (d.p.rc_height + ty - 1) / ty);
   float4 *v4 = reinterpret_cast<float4 *>(vert4), *n4 = reinterpret_cast<float4 *>(norm4);
-  if (d.grid.blocks) k_raycast<DenseNbhd><<<grid, blk, 0, s>>>(d, depth, v4, n4);
+  if (lanes == 8) k_raycast_group<8><<<grid, RC_GROUP_THREADS, 0, s>>>(d, depth, v4, n4);
+  else if (lanes == 4) k_raycast_group<4><<<grid, RC_GROUP_THREADS, 0, s>>>(d, depth, v4, n4);
+  else if (d.grid.blocks) k_raycast<DenseNbhd><<<grid, blk, 0, s>>>(d, depth, v4, n4);
   else k_raycast<Nbhd><<<grid, blk, 0, s>>>(d, depth, v4, n4);
   mh_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;

@@ -80,3 +80,21 @@ def test_host_images_of_any_size(built, w, h):
     wl, v, o = _map(w, h, 0.008)
     T = np.asarray(wl.pose(5), np.float64)
     assert _same(v, o, np.linalg.inv(T).astype(np.float32)) > 0
+
+
+# The last and first images of 8, 4 and 1 lanes a ray, whole and ragged tiles.
+@pytest.mark.parametrize("w,h", [(1, 1), (5, 3), (256, 256), (257, 256), (512, 256), (513, 256)])
+def test_lanes_of_a_ray(built, w, h):
+    wl, v, o = _map(w, h, 0.016)
+    T = np.asarray(wl.pose(5), np.float64)
+    hits = [_same(v, o, np.linalg.inv(m(T)).astype(np.float32)) for m in (POSES["own"], POSES["moved"])]
+    assert hits[0] > w * h // 4 or w * h < 100
+
+
+# Steps that lie halfway between two floats: t + step rounds down and up in turn
+# from 0.25 m, 0.5 m or 1 m on, so its samples have no closed form there.
+@pytest.mark.parametrize("half", [2.0 ** -26, 2.0 ** -25, 2.0 ** -24])
+def test_steps_that_round_both_ways(built, half):
+    wl, v, o = _map(60, 44, 0.008, raycast_step=2.0 ** -7 + half)
+    T = np.asarray(wl.pose(5), np.float64)
+    assert _same(v, o, np.linalg.inv(T).astype(np.float32)) > 60 * 44 // 4
