@@ -359,6 +359,23 @@ __device__ __forceinline__ void corner_pair(float p, float off, float vs, float 
   }
 }
 
+// Corner voxels of GetSpatialValue at pos (both of each axis) and the
+// position's fractions.
+struct SampleAt {
+  int v0x, v0y, v0z, v1x, v1y, v1z;
+  float rx, ry, rz;
+};
+__device__ __forceinline__ SampleAt sample_at(const DevParams &p, F3 pos) {
+  SampleAt k;
+  const F3 q = in_voxels(p, pos);
+  const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
+  k.rx = q.x - fx, k.ry = q.y - fy, k.rz = q.z - fz;
+  corner_pair(pos.x, p.voxel_size, p.voxel_size, q.x, fx, k.rx, k.v0x, k.v1x);
+  corner_pair(pos.y, p.voxel_size, p.voxel_size, q.y, fy, k.ry, k.v0y, k.v1y);
+  corner_pair(pos.z, p.voxel_size, p.voxel_size, q.z, fz, k.rz, k.v0z, k.v1z);
+  return k;
+}
+
 // GetSpatialValue (geometry/spatial_query.h:23-66): trilinear sdf (and the
 // interpolated sqrt(1/inv_sigma2) when want_radius); false if any corner
 // block is missing.  The block of corner 0 is looked up first, so a sample
