@@ -52,7 +52,7 @@ struct mh_batch {
   int step = 0;
   std::vector<float *> out_depth, out_vert, out_norm;
   std::vector<void *> allocs;
-  mh_batch_tuning tune{0, 16};
+  mh_batch_tuning tune{0, 2};  // the second is an index into kCtaCaps
   // graph per pinned block, with the configuration it was captured for
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   int g_tv_it[2] = {-1, -1}, g_host[2] = {-1, -1};

@@ -108,3 +108,10 @@ def test_batch_device_inputs_and_graph_replay(built):
         np.testing.assert_array_equal(fs["sdf"].view(np.uint32), fb["sdf"].view(np.uint32))
         assert ts == tb
     batch.close()
+
+
+def test_tuning_of_a_new_batch(built):
+    wl, p, _ = _scenes()[2]
+    batch = Batch([Volume(p)], raycast=True)
+    assert batch.tuning() == {"ray_tile": (16, 8), "integrate_cta_per_sm": 16}
+    batch.close()
