@@ -123,13 +123,13 @@ __global__ void __launch_bounds__(ALLOC_TILE * ALLOC_TILE) k_alloc_b(const Scene
 // (core/collect_block_array.cu:25-91), over the block pool's live indices
 // [0, high_water) instead of all hash entries; warp-ballot compaction with one
 // atomic per warp.
-__device__ __forceinline__ void collect_body(const Dev &d, int frustum) {
+__device__ __forceinline__ void collect_body(const Dev &d, Share sh, int frustum) {
   __shared__ float cTw[16];
   if (threadIdx.x < 16) cTw[threadIdx.x] = d.fc->cTw[threadIdx.x];
   __syncthreads();
   const int hw = *reinterpret_cast<volatile int *>(&d.ctr->high_water);
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < hw; base += stride) {
+  const int stride = sh.stride * blockDim.x;
+  for (int base = sh.first * blockDim.x; base < hw; base += stride) {
     const int i = base + threadIdx.x;
     bool keep = false;
     int4 bp = make_int4(0, 0, 0, 0);
@@ -144,9 +144,10 @@ __device__ __forceinline__ void collect_body(const Dev &d, int frustum) {
     if (keep) d.cand[slot + __popc(m & lanemask_lt())] = make_int4(bp.x, bp.y, bp.z, i);
   }
 }
-__global__ void __launch_bounds__(256) k_collect(Dev d, int frustum) { collect_body(d, frustum); }
+__global__ void __launch_bounds__(256) k_collect(Dev d, int frustum) { collect_body(d, whole_grid(), frustum); }
 __global__ void __launch_bounds__(256) k_collect_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { collect_body(c.d, 1); });
+  each_scene(t, n, 256, [&](const Scene &c) { return count_of(c.d, &Counters::high_water); },
+             [&](const Scene &c, Share sh) { collect_body(c.d, sh, 1); });
 }
 
 // Insert host-given blocks (state loading) and report their indices.

@@ -17,9 +17,9 @@
 
 
 // CollectLowSurfelBlocksKernel, first half (recycle.cu:91-99)
-__device__ __forceinline__ void gc_life_body(const Dev &d) {
+__device__ __forceinline__ void gc_life_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+  for (int c = sh.first * blockDim.x + threadIdx.x; c < n; c += sh.stride * blockDim.x) {
     d.flags[c] = 0;
     const int ptr = d.cand[c].w;
     if (ptr < 0) continue;
@@ -27,19 +27,20 @@ __device__ __forceinline__ void gc_life_body(const Dev &d) {
     else d.life[ptr] = MH_BLOCK_LIFE;
   }
 }
-__global__ void k_gc_life(Dev d) { gc_life_body(d); }
+__global__ void k_gc_life(Dev d) { gc_life_body(d, whole_grid()); }
 __global__ void k_gc_life_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { gc_life_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return count_of(c.d, &Counters::cand_count); },
+             [&](const Scene &c, Share sh) { gc_life_body(c.d, sh); });
 }
 
 // CollectLowSurfelBlocksKernel, second half (recycle.cu:102-113).  Eight lanes a
 // candidate, six with a neighbour each: one after the other the six dependent
 // lookups took 22 us against 9 us for a 320x240 PSDF frame at 6 mm (cold).
-__device__ __forceinline__ void gc_flag_body(const Dev &d) {
+__device__ __forceinline__ void gc_flag_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
   const int j = threadIdx.x & 7, per_cta = blockDim.x / 8;
   const int step = j & 1 ? -1 : 1;
-  for (int base = blockIdx.x * per_cta; base < n; base += gridDim.x * per_cta) {
+  for (int base = sh.first * per_cta; base < n; base += sh.stride * per_cta) {
     const int c = base + threadIdx.x / 8;
     const int4 cb = c < n ? d.cand[c] : make_int4(0, 0, 0, -1);
     const bool low = cb.w >= 0 && d.life[cb.w] <= 0;
@@ -53,15 +54,16 @@ __device__ __forceinline__ void gc_flag_body(const Dev &d) {
     if (low && j == 0 && !around) d.flags[c] = 1;
   }
 }
-__global__ void k_gc_flag(Dev d) { gc_flag_body(d); }
+__global__ void k_gc_flag(Dev d) { gc_flag_body(d, whole_grid()); }
 __global__ void k_gc_flag_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { gc_flag_body(c.d); });
+  each_scene(t, n, 32, [&](const Scene &c) { return count_of(c.d, &Counters::cand_count); },
+             [&](const Scene &c, Share sh) { gc_flag_body(c.d, sh); });
 }
 
 // StarveOccupiedBlocksKernel (recycle.cu:15-25)
-__device__ __forceinline__ void gc_starve_body(const Dev &d) {
+__device__ __forceinline__ void gc_starve_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int ptr = d.cand[c].w;
     if (ptr < 0) continue;
     float4 *w4 = reinterpret_cast<float4 *>(d.w + (size_t)ptr * MH_BLOCK_VOXELS) + threadIdx.x;
@@ -71,17 +73,18 @@ __device__ __forceinline__ void gc_starve_body(const Dev &d) {
     *w4 = w;
   }
 }
-__global__ void __launch_bounds__(128) k_gc_starve(Dev d) { gc_starve_body(d); }
+__global__ void __launch_bounds__(128) k_gc_starve(Dev d) { gc_starve_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_gc_starve_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.starve) gc_starve_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return c.starve ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { gc_starve_body(c.d, sh); });
 }
 
 // CollectGarbageBlockArrayKernel (recycle.cu:28-75)
-__device__ __forceinline__ void gc_garbage_body(const Dev &d) {
+__device__ __forceinline__ void gc_garbage_body(const Dev &d, Share sh) {
   __shared__ float smin[4], smax[4];
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
   const float inf = __int_as_float(0x7f800000);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int ptr = d.cand[c].w;
     if (ptr < 0) {
       if (threadIdx.x == 0) d.flags[c] = 0;
@@ -113,15 +116,16 @@ __device__ __forceinline__ void gc_garbage_body(const Dev &d) {
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(128) k_gc_garbage(Dev d) { gc_garbage_body(d); }
+__global__ void __launch_bounds__(128) k_gc_garbage(Dev d) { gc_garbage_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_gc_garbage_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.starve) gc_garbage_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return c.starve ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { gc_garbage_body(c.d, sh); });
 }
 
 // RecycleGarbageTrianglesKernel (recycle.cu:117-142)
-__device__ __forceinline__ void gc_recycle_tri_body(const Dev &d) {
+__device__ __forceinline__ void gc_recycle_tri_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int ptr = d.cand[c].w;
     if (ptr < 0 || !d.flags[c]) continue;
     const int pg = d.page_of[ptr];
@@ -140,16 +144,17 @@ __device__ __forceinline__ void gc_recycle_tri_body(const Dev &d) {
     }
   }
 }
-__global__ void __launch_bounds__(128) k_gc_recycle_tri(Dev d) { gc_recycle_tri_body(d); }
+__global__ void __launch_bounds__(128) k_gc_recycle_tri(Dev d) { gc_recycle_tri_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_gc_recycle_tri_b(const Scene *t, int n, int which) {
-  each_scene(t, n, [&](const Scene &c) { if (which ? c.starve : c.recycle) gc_recycle_tri_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return (which ? c.starve : c.recycle) ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { gc_recycle_tri_body(c.d, sh); });
 }
 
 // RecycleGarbageVerticesKernel (recycle.cu:144-181) + FreeEntry + Block::Clear
-__device__ __forceinline__ void gc_recycle_vtx_body(const Dev &d) {
+__device__ __forceinline__ void gc_recycle_vtx_body(const Dev &d, Share sh) {
   __shared__ int live;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = d.cand[c];
     if (cb.w < 0 || !d.flags[c]) continue;
     const int ptr = cb.w;
@@ -201,9 +206,10 @@ __device__ __forceinline__ void gc_recycle_vtx_body(const Dev &d) {
     if (threadIdx.x == 0) stack_push(&d.ctr->heap_top, d.heap, ptr);
   }
 }
-__global__ void __launch_bounds__(128) k_gc_recycle_vtx(Dev d) { gc_recycle_vtx_body(d); }
+__global__ void __launch_bounds__(128) k_gc_recycle_vtx(Dev d) { gc_recycle_vtx_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_gc_recycle_vtx_b(const Scene *t, int n, int which) {
-  each_scene(t, n, [&](const Scene &c) { if (which ? c.starve : c.recycle) gc_recycle_vtx_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return (which ? c.starve : c.recycle) ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { gc_recycle_vtx_body(c.d, sh); });
 }
 
 int launch_gc_low_surfel(const Dev &d, cudaStream_t s) {

@@ -73,7 +73,7 @@ __device__ __forceinline__ void note_neg(const Dev &d, int blk, const float4 &S)
 }  // namespace
 
 // UpdateBlocksSimpleKernel + Voxel::Update (core/voxel.h:107-115)
-__device__ __forceinline__ void integrate_simple_body(const Dev &d) {
+__device__ __forceinline__ void integrate_simple_body(const Dev &d, Share sh) {
   __shared__ float cTw[16];
   if (threadIdx.x < 16) cTw[threadIdx.x] = d.fc->cTw[threadIdx.x];
   __syncthreads();
@@ -82,10 +82,10 @@ __device__ __forceinline__ void integrate_simple_body(const Dev &d) {
   const int t = threadIdx.x;
   const int lx = (t & 1) * 4, ly = (t >> 1) & 7, lz = t >> 4;
   // the next candidate is fetched one iteration ahead
-  int4 next = (int)blockIdx.x < n ? d.cand[blockIdx.x] : make_int4(0, 0, 0, -1);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  int4 next = sh.first < n ? d.cand[sh.first] : make_int4(0, 0, 0, -1);
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = next;
-    if (c + (int)gridDim.x < n) next = d.cand[c + gridDim.x];
+    if (c + sh.stride < n) next = d.cand[c + sh.stride];
     if (cb.w < 0) continue;
     const int vx0 = cb.x * MH_BLOCK_SIDE + lx, vy = cb.y * MH_BLOCK_SIDE + ly, vz = cb.z * MH_BLOCK_SIDE + lz;
     const float fx0 = (float)vx0, fy = (float)vy, fz = (float)vz;
@@ -136,18 +136,19 @@ __device__ __forceinline__ void integrate_simple_body(const Dev &d) {
     note_neg(d, cb.w, S);
   }
 }
-__global__ void __launch_bounds__(128) k_integrate_simple(Dev d) { integrate_simple_body(d); }
+__global__ void __launch_bounds__(128) k_integrate_simple(Dev d) { integrate_simple_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_integrate_simple_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (!c.d.p.enable_bayesian) integrate_simple_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return c.d.p.enable_bayesian ? 0 : count_of(c.d, &Counters::cand_count); },
+             [&](const Scene &c, Share sh) { integrate_simple_body(c.d, sh); });
 }
 
 // What the PSDF update needs of a pixel, once per pixel instead of once per
 // voxel that projects onto it: depth (-inf if invalid), inlier ratio, the
 // measurement's variance and the outlier density (update_bayesian.cu:123-156).
-__device__ __forceinline__ void pixels_body(const Dev &d) {
+__device__ __forceinline__ void pixels_body(const Dev &d, Share sh) {
   const DevParams &p = d.p;
   const int n = p.width * p.height;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = sh.first * blockDim.x + threadIdx.x; i < n; i += sh.stride * blockDim.x) {
     const float dd = d.depth[i], r = d.inlier[i];
     const float tau = (dd - 0.4f) * 0.012f + 0.019f;
     const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
@@ -156,16 +157,17 @@ __device__ __forceinline__ void pixels_body(const Dev &d) {
                               in_range ? out : 1.0f);
   }
 }
-__global__ void __launch_bounds__(256) k_pixels(Dev d) { pixels_body(d); }
+__global__ void __launch_bounds__(256) k_pixels(Dev d) { pixels_body(d, whole_grid()); }
 __global__ void __launch_bounds__(256) k_pixels_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) pixels_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return c.d.p.enable_bayesian ? (int)(c.d.p.width * c.d.p.height) : 0; },
+             [&](const Scene &c, Share sh) { pixels_body(c.d, sh); });
 }
 
 // UpdateBlocksBayesianKernel (mapping/update_bayesian.cu:103-185).  Per voxel
 // the update is division- and transcendental-bound, not load-bound, so the
 // default form restates it with 4 IEEE divisions (see below); compat mode
 // evaluates the reference's expressions as written.
-__device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
+__device__ __forceinline__ void integrate_psdf_body(const Dev &d, Share sh) {
   __shared__ float cTw[16];
   if (threadIdx.x < 16) cTw[threadIdx.x] = d.fc->cTw[threadIdx.x];
   __syncthreads();
@@ -173,10 +175,10 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
   const int t = threadIdx.x;
   const int lx = (t & 1) * 4, ly = (t >> 1) & 7, lz = t >> 4;
-  int4 next = (int)blockIdx.x < n ? d.cand[blockIdx.x] : make_int4(0, 0, 0, -1);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  int4 next = sh.first < n ? d.cand[sh.first] : make_int4(0, 0, 0, -1);
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = next;
-    if (c + (int)gridDim.x < n) next = d.cand[c + gridDim.x];
+    if (c + sh.stride < n) next = d.cand[c + sh.stride];
     if (cb.w < 0) continue;
     const int vx0 = cb.x * MH_BLOCK_SIDE + lx, vy = cb.y * MH_BLOCK_SIDE + ly, vz = cb.z * MH_BLOCK_SIDE + lz;
     const float fx0 = (float)vx0, fy = (float)vy, fz = (float)vz;
@@ -287,9 +289,10 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d) {
     note_neg(d, cb.w, S);
   }
 }
-__global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body(d); }
+__global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128, 8) k_integrate_psdf_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) integrate_psdf_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return c.d.p.enable_bayesian ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { integrate_psdf_body(c.d, sh); });
 }
 
 // PredictOutlierRatioKernel (mapping/update_bayesian.cu:36-101).  The
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(128, 8) k_integrate_psdf_b(const Scene *t, int
 // the positive ratios involved (all >= 0.01).  Blocks that own no vertex are
 // skipped.  The vertex normal is transformed by cTw as a point (with the
 // translation), as the reference does (update_bayesian.cu:83-86).
-__device__ __forceinline__ void predict_inlier_body(const Dev &d) {
+__device__ __forceinline__ void predict_inlier_body(const Dev &d, Share sh) {
   __shared__ float cTw[16];
   if (threadIdx.x < 16) cTw[threadIdx.x] = d.fc->cTw[threadIdx.x];
   __syncthreads();
@@ -305,7 +308,7 @@ __device__ __forceinline__ void predict_inlier_body(const Dev &d) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->vtx_list_count);
   const int t = threadIdx.x;
   const int lx = (t & 1) * 4, ly = (t >> 1) & 7, lz = t >> 4;
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = d.cand[d.vtx_list[c]];
     const int pg = __ldg(d.page_of + cb.w);
     const size_t base = (size_t)cb.w * MH_BLOCK_VOXELS + t * 4;
@@ -356,17 +359,18 @@ __device__ __forceinline__ void predict_inlier_body(const Dev &d) {
     }
   }
 }
-__global__ void __launch_bounds__(128) k_predict_inlier(Dev d) { predict_inlier_body(d); }
+__global__ void __launch_bounds__(128) k_predict_inlier(Dev d) { predict_inlier_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_predict_inlier_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) predict_inlier_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return c.d.p.enable_bayesian ? count_of(c.d, &Counters::vtx_list_count) : 0; },
+             [&](const Scene &c, Share sh) { predict_inlier_body(c.d, sh); });
 }
 
 // Candidates owning at least one vertex (and so a mesh page), for the
 // inlier prediction; one thread per candidate, warp-ballot compaction.
-__device__ __forceinline__ void vtx_select_body(const Dev &d) {
+__device__ __forceinline__ void vtx_select_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+  const int stride = sh.stride * blockDim.x;
+  for (int base = sh.first * blockDim.x; base < n; base += stride) {
     const int i = base + threadIdx.x;
     bool keep = false;
     if (i < n) {
@@ -380,27 +384,29 @@ __device__ __forceinline__ void vtx_select_body(const Dev &d) {
     if (keep) d.vtx_list[slot + __popc(m & lanemask_lt())] = i;
   }
 }
-__global__ void __launch_bounds__(256) k_vtx_select(Dev d) { vtx_select_body(d); }
+__global__ void __launch_bounds__(256) k_vtx_select(Dev d) { vtx_select_body(d, whole_grid()); }
 __global__ void __launch_bounds__(256) k_vtx_select_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { if (c.d.p.enable_bayesian) vtx_select_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return c.d.p.enable_bayesian ? count_of(c.d, &Counters::cand_count) : 0; },
+             [&](const Scene &c, Share sh) { vtx_select_body(c.d, sh); });
 }
 
 // Sensor::Process tail: depth validity (ConvertDepthFormatKernel,
 // sensor/preprocess.cu:25-42) and inlier-ratio reset to 0.1 (:10-23).  Raw
 // 16-bit depth is read as the reference reads it, through a signed short, so
 // raw values of 32768 and above are negative depths and invalid.
-__device__ __forceinline__ void preprocess_body(const Dev &d, const float *src, const uint16_t *src16, float range_factor) {
+__device__ __forceinline__ void preprocess_body(const Dev &d, Share sh, const float *src, const uint16_t *src16, float range_factor) {
   const int n = d.p.width * d.p.height;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = sh.first * blockDim.x + threadIdx.x; i < n; i += sh.stride * blockDim.x) {
     float z = src16 ? range_factor * (float)(int16_t)src16[i] : src[i];
     const bool ok = z >= d.p.min_depth_range && z <= d.p.max_depth_range;
     d.depth[i] = ok ? z : -__int_as_float(0x7f800000);
     d.inlier[i] = 0.1f;
   }
 }
-__global__ void k_preprocess(Dev d, const float *src, const uint16_t *src16, float range_factor) { preprocess_body(d, src, src16, range_factor); }
+__global__ void k_preprocess(Dev d, const float *src, const uint16_t *src16, float range_factor) { preprocess_body(d, whole_grid(), src, src16, range_factor); }
 __global__ void k_preprocess_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { preprocess_body(c.d, c.src, nullptr, 0.0f); });
+  each_scene(t, n, 256, [&](const Scene &c) { return (int)(c.d.p.width * c.d.p.height); },
+             [&](const Scene &c, Share sh) { preprocess_body(c.d, sh, c.src, nullptr, 0.0f); });
 }
 
 static int grid_persistent(int per_sm) { return mh_sm_count() * per_sm; }

@@ -204,6 +204,12 @@ __device__ __forceinline__ int hash_find(const Dev &d, int x, int y, int z) {
   return -1;
 }
 
+// A CTA's place in a grid-stride loop.
+struct Share {
+  int first, stride;
+};
+__device__ __forceinline__ Share whole_grid() { return Share{(int)blockIdx.x, (int)gridDim.x}; }
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31; }
 
 // A voxel counts as non-negative when its sdf lies in [0, 1e30) (NaN does

@@ -74,12 +74,12 @@ __device__ __forceinline__ unsigned claim_slots(const Dev &d, uint32_t *cw, unsi
 // Candidates the cube pass must tile: a block holding a mesh page, or one
 // whose weight bound reaches the MC gate (otherwise no cube in it is valid).
 // One thread per candidate, warp-ballot compaction.
-__device__ __forceinline__ void mc_select_body(const Dev &d) {
+__device__ __forceinline__ void mc_select_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
   const float lim = 1.0f / d.p.voxel_size;
   const float lim2 = lim * lim;
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+  const int stride = sh.stride * blockDim.x;
+  for (int base = sh.first * blockDim.x; base < n; base += stride) {
     const int i = base + threadIdx.x;
     int4 cb = make_int4(0, 0, 0, -1);
     bool keep = false;
@@ -94,9 +94,10 @@ __device__ __forceinline__ void mc_select_body(const Dev &d) {
     if (keep) d.cube_list[slot + __popc(m & lanemask_lt())] = cb;
   }
 }
-__global__ void __launch_bounds__(256) k_mc_select(Dev d) { mc_select_body(d); }
+__global__ void __launch_bounds__(256) k_mc_select(Dev d) { mc_select_body(d, whole_grid()); }
 __global__ void __launch_bounds__(256) k_mc_select_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_select_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return count_of(c.d, &Counters::cand_count); },
+             [&](const Scene &c, Share sh) { mc_select_body(c.d, sh); });
 }
 // Counts of the finished pass, and the next pass's start.  Run by one thread of
 // the last kernel, which reads only mesh_list_count (k_mc_cubes clears that).
@@ -119,7 +120,7 @@ __device__ __forceinline__ void mc_end_body(const Dev &d) {
 // atomicCAS a cube and edge and an atomicAdd a vertex, one after the other, took
 // 41 us against 18 us for a 320x240 PSDF frame at 6 mm (cold).  What is left is
 // the latency of a block's chain: candidate, hash, tile, pages, claims.
-__device__ __forceinline__ void mc_cubes_body(const Dev &d) {
+__device__ __forceinline__ void mc_cubes_body(const Dev &d, Share sh) {
   __shared__ uint8_t tile[729];
   __shared__ unsigned own[729];
   __shared__ int nb[8], page[8];
@@ -130,11 +131,11 @@ __device__ __forceinline__ void mc_cubes_body(const Dev &d) {
   const float lim = 1.0f / d.p.voxel_size;
   const float lim2 = lim * lim;
   const int x = tid & 7, y = (tid >> 3) & 7, z = tid >> 6;
-  if (blockIdx.x == 0 && tid == 0) {
+  if (sh.first == 0 && tid == 0) {
     d.ctr->mesh_list_count = 0;
     d.ctr->cube_blocks_sum += (unsigned long long)n;
   }
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = d.cube_list[c];
     if (tid < 8) {
       const int dx = tid & 1, dy = (tid >> 1) & 1, dz = tid >> 2;
@@ -230,16 +231,17 @@ __device__ __forceinline__ void mc_cubes_body(const Dev &d) {
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(512, 3) k_mc_cubes(Dev d) { mc_cubes_body(d); }
+__global__ void __launch_bounds__(512, 3) k_mc_cubes(Dev d) { mc_cubes_body(d, whole_grid()); }
 __global__ void __launch_bounds__(512, 2) k_mc_cubes_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_cubes_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return max(1, count_of(c.d, &Counters::cube_list_count)); },
+             [&](const Scene &c, Share sh) { mc_cubes_body(c.d, sh); });
 }
 
 // candidates holding a page after pass 1; the others get zero surfel counts
-__device__ __forceinline__ void mc_list_body(const Dev &d) {
+__device__ __forceinline__ void mc_list_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
-  const int stride = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+  const int stride = sh.stride * blockDim.x;
+  for (int base = sh.first * blockDim.x; base < n; base += stride) {
     const int i = base + threadIdx.x;
     int ptr = -1;
     bool keep = false;
@@ -257,9 +259,10 @@ __device__ __forceinline__ void mc_list_body(const Dev &d) {
     if (keep) d.mesh_list[slot + __popc(m & lanemask_lt())] = ptr;
   }
 }
-__global__ void __launch_bounds__(256) k_mc_list(Dev d) { mc_list_body(d); }
+__global__ void __launch_bounds__(256) k_mc_list(Dev d) { mc_list_body(d, whole_grid()); }
 __global__ void __launch_bounds__(256) k_mc_list_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_list_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return count_of(c.d, &Counters::cand_count); },
+             [&](const Scene &c, Share sh) { mc_list_body(c.d, sh); });
 }
 
 // ------------------------------------------------------------------ vertices
@@ -301,14 +304,14 @@ __device__ __forceinline__ size_t voxel_index(int block, int x, int y, int z) {
 // latency of dependent loads: a thread a vertex, with seven samples one after
 // the other and a hash lookup for every corner in another block, took 52 us
 // against 17 us for a 320x240 PSDF frame at 6 mm (cold).
-__device__ __forceinline__ void mc_vertices_body(const Dev &d) {
+__device__ __forceinline__ void mc_vertices_body(const Dev &d, Share sh) {
   const int n = min(*reinterpret_cast<volatile int *>(&d.ctr->vwork_count), d.vwork_capacity);
-  const int per_cta = blockDim.x / 8, stride = gridDim.x * per_cta;
+  const int per_cta = blockDim.x / 8, stride = sh.stride * per_cta;
   const int j = threadIdx.x & 7;
   const unsigned base8 = threadIdx.x & 24;
   const float vs = d.p.voxel_size;
 #pragma unroll 1
-  for (int base = blockIdx.x * per_cta; base < n; base += stride) {
+  for (int base = sh.first * per_cta; base < n; base += stride) {
     const int i = base + threadIdx.x / 8;
     bool live = i < n;
     int4 wk = make_int4(0, 0, 0, 0);
@@ -416,20 +419,21 @@ __device__ __forceinline__ void mc_vertices_body(const Dev &d) {
     __syncwarp();
   }
 }
-__global__ void __launch_bounds__(128) k_mc_vertices(Dev d) { mc_vertices_body(d); }
+__global__ void __launch_bounds__(128) k_mc_vertices(Dev d) { mc_vertices_body(d, whole_grid()); }
 __global__ void __launch_bounds__(128) k_mc_vertices_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_vertices_body(c.d); });
+  each_scene(t, n, 16, [&](const Scene &c) { return count_of(c.d, &Counters::vwork_count); },
+             [&](const Scene &c, Share sh) { mc_vertices_body(c.d, sh); });
 }
 
 // ------------------------------------------------------------------ pass 2
-__device__ __forceinline__ void mc_triangles_body(const Dev &d) {
+__device__ __forceinline__ void mc_triangles_body(const Dev &d, Share sh) {
   __shared__ int nbp[8];
   __shared__ int cnt[2];
   const int tid = threadIdx.x;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->mesh_list_count);
   const int x = tid & 7, y = (tid >> 3) & 7, z = tid >> 6;
   const bool inner = x >= 1 && y >= 1 && z >= 1 && x < 7 && y < 7 && z < 7;
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int blk = d.mesh_list[c];
     const int4 bp = d.block_pos[blk];
     if (tid < 8) {
@@ -501,9 +505,10 @@ __device__ __forceinline__ void mc_triangles_body(const Dev &d) {
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(512) k_mc_triangles(Dev d) { mc_triangles_body(d); }
+__global__ void __launch_bounds__(512) k_mc_triangles(Dev d) { mc_triangles_body(d, whole_grid()); }
 __global__ void __launch_bounds__(512) k_mc_triangles_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_triangles_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return count_of(c.d, &Counters::mesh_list_count); },
+             [&](const Scene &c, Share sh) { mc_triangles_body(c.d, sh); });
 }
 
 // ------------------------------------------------------------------ recycle
@@ -511,10 +516,10 @@ __global__ void __launch_bounds__(512) k_mc_triangles_b(const Scene *t, int n) {
 // looked at: what bounds them is the latency of one load after the other.  A
 // slot at a time, and the triangle slots again for each page's end, took 15 and
 // 17 us against 11 and 7 us for a 320x240 PSDF frame at 6 mm (cold).
-__device__ __forceinline__ void mc_recycle_tri_body(const Dev &d) {
+__device__ __forceinline__ void mc_recycle_tri_body(const Dev &d, Share sh) {
   constexpr int N = MH_BLOCK_VOXELS * 5 / 4 / MC_RECYCLE_THREADS;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->mesh_list_count);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int pg = d.page_of[d.mesh_list[c]];
     int *ts = d.tri_slot + (size_t)pg * MH_BLOCK_VOXELS * 5;
     int4 held[N];
@@ -542,16 +547,17 @@ __device__ __forceinline__ void mc_recycle_tri_body(const Dev &d) {
     }
   }
 }
-__global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_tri(Dev d) { mc_recycle_tri_body(d); }
+__global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_tri(Dev d) { mc_recycle_tri_body(d, whole_grid()); }
 __global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_tri_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_recycle_tri_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return count_of(c.d, &Counters::mesh_list_count); },
+             [&](const Scene &c, Share sh) { mc_recycle_tri_body(c.d, sh); });
 }
 
-__device__ __forceinline__ void mc_recycle_vtx_body(const Dev &d) {
+__device__ __forceinline__ void mc_recycle_vtx_body(const Dev &d, Share sh) {
   constexpr int N = MH_BLOCK_VOXELS * 3 / 4 / MC_RECYCLE_THREADS;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->mesh_list_count);
-  if (blockIdx.x == 0 && threadIdx.x == 0) mc_end_body(d);
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  if (sh.first == 0 && threadIdx.x == 0) mc_end_body(d);
+  for (int c = sh.first; c < n; c += sh.stride) {
     const int blk = d.mesh_list[c];
     const int pg = d.page_of[blk];
     int *vs = d.vtx_slot + (size_t)pg * MH_BLOCK_VOXELS * 3;
@@ -593,9 +599,10 @@ __device__ __forceinline__ void mc_recycle_vtx_body(const Dev &d) {
     __syncthreads();
   }
 }
-__global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_vtx(Dev d) { mc_recycle_vtx_body(d); }
+__global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_vtx(Dev d) { mc_recycle_vtx_body(d, whole_grid()); }
 __global__ void __launch_bounds__(MC_RECYCLE_THREADS) k_mc_recycle_vtx_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { mc_recycle_vtx_body(c.d); });
+  each_scene(t, n, 1, [&](const Scene &c) { return max(1, count_of(c.d, &Counters::mesh_list_count)); },
+             [&](const Scene &c, Share sh) { mc_recycle_vtx_body(c.d, sh); });
 }
 
 int launch_mesh(const Dev &d, cudaStream_t s) {

@@ -741,12 +741,12 @@ int launch_raycast_batch(const Scene *t, int n, int total, int shape, cudaStream
 // of them marked: 41 us (cold), of 390 us for the raycast with it.  Cells of 4
 // voxels cost less here (14 us) and more in the march, which then evaluates 6.4
 // samples a ray instead of 3.4 (507 us in all).
-__device__ __forceinline__ void ray_grid_body(const Dev &d) {
+__device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
   const RayGrid &g = d.grid;
   if (!g.bits) return;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->high_water);
   const int nx = (int)g.nx, ny = (int)g.ny, nz = (int)g.nz;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = sh.first * blockDim.x + threadIdx.x; i < n; i += sh.stride * blockDim.x) {
     const int4 b = d.block_pos[i];
     if (!b.w) continue;
     if (g.blocks) {
@@ -785,16 +785,17 @@ __device__ __forceinline__ void ray_grid_body(const Dev &d) {
     }
   }
 }
-__global__ void __launch_bounds__(256) k_ray_grid(Dev d) { ray_grid_body(d); }
+__global__ void __launch_bounds__(256) k_ray_grid(Dev d) { ray_grid_body(d, whole_grid()); }
 __global__ void __launch_bounds__(256) k_ray_grid_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) { ray_grid_body(c.d); });
+  each_scene(t, n, 256, [&](const Scene &c) { return c.d.grid.bits ? count_of(c.d, &Counters::high_water) : 0; },
+             [&](const Scene &c, Share sh) { ray_grid_body(c.d, sh); });
 }
 __global__ void __launch_bounds__(256) k_ray_grid_clear_b(const Scene *t, int n) {
-  each_scene(t, n, [&](const Scene &c) {
-    if (!c.d.grid.bits) return;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < c.d.grid.words; i += gridDim.x * blockDim.x)
+  each_scene(t, n, 256, [&](const Scene &c) { return c.d.grid.bits ? (int)max(c.d.grid.words, c.d.grid.clear) : 0; },
+             [&](const Scene &c, Share sh) {
+    for (unsigned i = sh.first * blockDim.x + threadIdx.x; i < c.d.grid.words; i += sh.stride * blockDim.x)
       c.d.grid.bits[i] = 0u;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < c.d.grid.clear; i += gridDim.x * blockDim.x)
+    for (unsigned i = sh.first * blockDim.x + threadIdx.x; i < c.d.grid.clear; i += sh.stride * blockDim.x)
       c.d.grid.blocks[i] = 0u;
   });
 }

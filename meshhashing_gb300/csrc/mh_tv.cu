@@ -93,17 +93,18 @@ __device__ __forceinline__ void tv_iter_body(const TvBuf &b) {
 }
 __global__ void __launch_bounds__(256) k_tv_iter(TvBuf b) { tv_iter_body(b); }
 
-__device__ __forceinline__ void tv_out_body(const float *f, const float *u, float *depth, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+__device__ __forceinline__ void tv_out_body(const float *f, const float *u, float *depth, int n, Share sh) {
+  for (int i = sh.first * blockDim.x + threadIdx.x; i < n; i += sh.stride * blockDim.x)
     depth[i] = valid_at(f, i) ? u[i] * 0.001f : -__int_as_float(0x7f800000);
 }
-__global__ void k_tv_out(const float *f, const float *u, float *depth, int n) { tv_out_body(f, u, depth, n); }
+__global__ void k_tv_out(const float *f, const float *u, float *depth, int n) { tv_out_body(f, u, depth, n, whole_grid()); }
 // a batch's TV result after `launches` tiled launches: planes 1-4 hold the
 // iterate after an even number of launches, planes 5-8 after an odd number
 __global__ void k_tv_out_b(const Scene *t, int n, int launches) {
-  each_scene(t, n, [&](const Scene &c) {
+  each_scene(t, n, 256, [&](const Scene &c) { return (int)(c.d.p.width * c.d.p.height); },
+             [&](const Scene &c, Share sh) {
     const size_t np = (size_t)c.d.p.width * c.d.p.height;
-    tv_out_body(c.tv, c.tv + np * ((launches & 1) ? 5 : 1), c.d.depth, (int)np);
+    tv_out_body(c.tv, c.tv + np * ((launches & 1) ? 5 : 1), c.d.depth, (int)np, sh);
   });
 }
 

@@ -115,3 +115,41 @@ def test_tuning_of_a_new_batch(built):
     batch = Batch([Volume(p)], raycast=True)
     assert batch.tuning() == {"ray_tile": (16, 8), "integrate_cta_per_sm": 16}
     batch.close()
+
+
+# One round of the scene table is 32 scenes; some never take a frame, so they
+# have no blocks, and the simple and the Bayesian update alternate.
+@pytest.mark.parametrize("n", [1, 33, 40])
+def test_many_scenes(built, n):
+    specs = []
+    for i in range(n):
+        w, h = ((32, 24), (64, 48), (40, 28))[i % 3]
+        wl = scene.full_spline(8, width=w, height=h, seed=i)
+        specs.append((wl, config.params_for(wl, voxel_size=0.02, truncation=0.06, value_capacity=1 << 13,
+                                            bucket_count=1 << 12, max_vertex_count=1 << 14, max_triangle_count=1 << 14,
+                                            bayesian=i % 2 == 1)))
+    singles = [Volume(p) for _, p in specs]
+    batched = [Volume(p) for _, p in specs]
+    batch = Batch(batched, raycast=True)
+    for k in range(4):
+        active = [1 if n == 1 or (i % 5 != 4 and (i + k) % 3 != 2) else 0 for i in range(n)]
+        for i, (wl, _) in enumerate(specs):
+            if active[i]:
+                singles[i].integrate_frame(wl.frame(k), wl.pose(k))
+        batch.step([wl.frame(k) if a else None for (wl, _), a in zip(specs, active)],
+                   [wl.pose(k) if a else None for (wl, _), a in zip(specs, active)], active=active, use_graph=k >= 2)
+    total = 0
+    for i in range(n):
+        ps, fs, (vs, ts) = _state(singles[i])
+        pb, fb, (vb, tb) = _state(batched[i])
+        np.testing.assert_array_equal(ps, pb)
+        for key in ("sdf", "w", "a", "b"):
+            np.testing.assert_array_equal(fs[key].view(np.uint32), fb[key].view(np.uint32))
+        assert ts == tb
+        for m, r in zip(batched[i].block_meta(pb), singles[i].block_meta(pb)):
+            np.testing.assert_array_equal(m, r)
+        assert {q: x for q, x in batched[i].stats().items() if q.endswith("_sum") or q == "error"} == \
+               {q: x for q, x in singles[i].stats().items() if q.endswith("_sum") or q == "error"}
+        total += len(pb)
+    assert total > 0
+    batch.close()
