@@ -63,6 +63,7 @@ struct Counters {
   int mesh_list_count; // candidates holding a mesh page this pass
   int cube_list_count; // candidates the cube pass must tile this pass
   int vtx_list_count;  // candidates owning vertices (inlier prediction)
+  int upd_count;       // candidates that the PSDF update may change
   int ray_next;        // next ray handed out by the raycast
   unsigned long long cand_sum;   // sum of candidate counts over mesh calls
   unsigned long long vwork_sum;  // sum of computed vertices over mesh calls
@@ -144,6 +145,8 @@ struct Dev {
   int *page_owner;         // per page: block index or -1
   int *mesh_list;          // candidates holding a page (this mesh pass)
   int4 *cube_list;         // candidates the cube pass tiles (x, y, z, block)
+  int4 *upd_list;          // candidates the PSDF update may change; cube_list's memory, which no
+                           // pass holds from one stage to the next
   int *vtx_list;           // candidate indices owning vertices
   int page_capacity;
   Vertex *vtx;
@@ -156,6 +159,7 @@ struct Dev {
   int vwork_capacity;
   float *depth, *inlier;   // current frame (W x H)
   float4 *pixels;          // the PSDF update's pixel records (in the TV scratch)
+  unsigned *tile_far;      // ... and the depth up to which each 4x4 tile of them updates voxels
   FrameConst *fc;
   Counters *ctr;
 };
@@ -300,6 +304,10 @@ __device__ __forceinline__ float truncate_dist(const DevParams &p, float z) {
 __device__ __forceinline__ float normalize_depth(const DevParams &p, float z) {
   return (z - p.min_depth_range) / (p.max_depth_range - p.min_depth_range);
 }
+// pixels of a tile of tile_far, each way
+#define FAR_TILE 4
+__host__ __device__ __forceinline__ int far_tiles_x(const DevParams &p) { return (int)(p.width + FAR_TILE - 1) / FAR_TILE; }
+__host__ __device__ __forceinline__ int far_tiles_y(const DevParams &p) { return (int)(p.height + FAR_TILE - 1) / FAR_TILE; }
 __device__ __forceinline__ bool depth_invalid(const DevParams &p, float d) {
   return d == -__int_as_float(0x7f800000) || d == 0.0f || d >= p.sdf_upper_bound;
 }

@@ -382,6 +382,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   if (v->grid.entries) A(dalloc(v, &v->grid.blocks, v->grid.entries));
   A(dalloc(v, &d.mesh_list, cap));
   A(dalloc(v, &d.cube_list, cap));
+  d.upd_list = d.cube_list;
   A(dalloc(v, &d.vtx_list, cap));
   A(dalloc(v, &d.page_heap, (size_t)d.page_capacity));
   A(dalloc(v, &d.page_owner, (size_t)d.page_capacity));
@@ -403,6 +404,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   A(dalloc(v, &d.ctr, 1));
   A(dalloc(v, &v->tv, npix * 9));
   d.pixels = reinterpret_cast<float4 *>(v->tv);
+  d.tile_far = reinterpret_cast<unsigned *>(v->tv + 4 * (size_t)P.width * P.height);
   A(dalloc(v, &v->rc_stage, rpix * 9 + 3));
   if (r == MH_OK) r = mh_volume_reset(v, nullptr);
   if (r != MH_OK) {
