@@ -119,6 +119,7 @@ struct RayGrid {
   unsigned bnx, bny, bnz;
   unsigned tag;              // this raycast's top byte, 1 .. 255
   unsigned clear;            // the tags start over: entries to clear first (all that the buffer has), else 0
+  bool filled;               // the buffers hold this grid already
 };
 
 // Everything a kernel needs, passed by value (pointers + params).

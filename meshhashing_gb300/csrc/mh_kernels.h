@@ -27,7 +27,8 @@ struct RayGridBuf {
   unsigned tag = 0;
 };
 void ray_grid_sizes(const mh_params &P, RayGridBuf &b);
-RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b);
+RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b, double margin = 0.0);
+bool ray_grid_covers(const mh_params &P, const float wTc[16], const RayGrid &g);
 int launch_raycast(const Dev &d, float *depth, float *vert4, float *norm4, cudaStream_t s);
 int launch_count_flags(const uint8_t *flags, int n, int *out, cudaStream_t s);
 

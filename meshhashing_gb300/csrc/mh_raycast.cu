@@ -827,17 +827,12 @@ void ray_grid_sizes(const mh_params &P, RayGridBuf &b) {
   b.entries = entries <= 67108864.0 && P.value_capacity <= (1u << 24) ? (unsigned)entries : 0u;
 }
 
-// The smallest cells (U = 2, 4, ... voxels) for which the box around the view
-// fits the words and the coordinates' rounding (4 units in the last place)
-// stays below 1/128 cell.  The samples of a pixel lie at wTc (z r), z in the
-// raycast range and r the pixel's ray, so the box is the hull of the view's
-// eight corners when wTc is rigid; any other matrix gets the ball that holds
-// every ray (their directions are normalised).  No grid (null bits) for a pose
-// that is not finite or far out.
-RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b) {
-  RayGrid g{};
-  if (!b.bits) return g;
-  double lo[3], hi[3];
+// The box around a view, false for a pose that is not finite or far out.  The
+// samples of a pixel lie at wTc (z r), z in the raycast range and r the pixel's
+// ray, so the box is the hull of the view's eight corners when wTc is rigid;
+// any other matrix gets the ball that holds every ray (their directions are
+// normalised).
+static bool view_box(const mh_params &P, const float wTc[16], double lo[3], double hi[3]) {
   const ViewCone v(P);
   bool rigid = true;
   for (int i = 0; i < 3; ++i)
@@ -861,8 +856,15 @@ RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b) {
     // the directions' deviation from unit length, and the march's rounding
     const double pad = 2e-3 * v.len * zs[1];
     lo[a] -= pad, hi[a] += pad;
-    if (!(lo[a] > -1e6 && hi[a] < 1e6)) return g;
+    if (!(lo[a] > -1e6 && hi[a] < 1e6)) return false;
   }
+  return true;
+}
+
+// The smallest cells (U = 2, 4, ... voxels) for which a box fits the words and
+// the coordinates' rounding (4 units in the last place) stays below 1/128 cell.
+static RayGrid grid_of(const mh_params &P, const double lo[3], const double hi[3], const RayGridBuf &b) {
+  RayGrid g{};
   double far = 0.0;
   for (int a = 0; a < 3; ++a) far = std::max(far, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
   for (int shift = 0; shift < 12; ++shift) {
@@ -896,6 +898,22 @@ RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b) {
     g.blocks = b.blocks;
     g.bx = c[0], g.by = c[1], g.bz = c[2];
     g.bnx = (unsigned)n[0], g.bny = (unsigned)n[1], g.bnz = (unsigned)n[2];
+  }
+  return g;
+}
+
+// No grid (null bits) for a pose that is not finite or far out.  `margin`
+// widens the box on each side where that does not make the cells larger.
+RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b, double margin) {
+  double lo[3], hi[3];
+  if (!b.bits || !view_box(P, wTc, lo, hi)) return RayGrid{};
+  RayGrid g = grid_of(P, lo, hi, b);
+  if (margin > 0.0 && g.bits) {
+    for (int a = 0; a < 3; ++a) lo[a] -= margin, hi[a] += margin;
+    const RayGrid wide = grid_of(P, lo, hi, b);
+    if (wide.bits && wide.shift == g.shift && !wide.blocks == !g.blocks) g = wide;
+  }
+  if (g.blocks) {
     b.tag = b.tag % 255u + 1u;
     g.tag = b.tag << 24;
     g.clear = b.tag == 1u ? b.entries : 0u;
@@ -903,8 +921,23 @@ RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b) {
   return g;
 }
 
+// Whether g, made for another pose, holds this pose's view.
+bool ray_grid_covers(const mh_params &P, const float wTc[16], const RayGrid &g) {
+  double lo[3], hi[3];
+  if (!g.bits || !view_box(P, wTc, lo, hi)) return false;
+  const double cell = (double)(2 << g.shift) * (double)P.voxel_size, side = 8.0 * (double)P.voxel_size;
+  const int c[3] = {g.cx, g.cy, g.cz}, bl[3] = {g.bx, g.by, g.bz};
+  const unsigned n[3] = {4 * g.nx, 4 * g.ny, 2 * g.nz}, bn[3] = {g.bnx, g.bny, g.bnz};
+  for (int a = 0; a < 3; ++a) {
+    if (!(lo[a] / cell - 2.0 >= c[a] && std::floor(hi[a] / cell) + 3.0 <= c[a] + (double)n[a])) return false;
+    if (g.blocks && !(std::floor(lo[a] / side) - 1.0 >= bl[a] && std::floor(hi[a] / side) + 2.0 <= bl[a] + (double)bn[a]))
+      return false;
+  }
+  return true;
+}
+
 static int fill_ray_grid(const Dev &d, cudaStream_t s) {
-  if (!d.grid.bits) return MH_OK;
+  if (!d.grid.bits || d.grid.filled) return MH_OK;
   MH_CUDA_TRY(cudaMemsetAsync(d.grid.bits, 0, sizeof(unsigned) * (size_t)d.grid.words, s));
   if (d.grid.clear)
     MH_CUDA_TRY(cudaMemsetAsync(d.grid.blocks, 0, sizeof(unsigned) * (size_t)d.grid.clear, s));

@@ -98,3 +98,23 @@ def test_steps_that_round_both_ways(built, half):
     wl, v, o = _map(60, 44, 0.008, raycast_step=2.0 ** -7 + half)
     T = np.asarray(wl.pose(5), np.float64)
     assert _same(v, o, np.linalg.inv(T).astype(np.float32)) > 60 * 44 // 4
+
+
+# One grid serves a refinement's poses where it covers them: the last pass's sums
+# against those of a grid made for that pose alone.  Its inverse may differ by
+# units in the last place, 1e-6 m of depth, which moves a pixel in a thousand
+# across the gate at most.
+@pytest.mark.parametrize("w,h,voxel", [(64, 48, 0.008), (124, 92, 0.004), (40, 28, 0.001)])
+@pytest.mark.parametrize("off", [0.0, 0.01, 0.3])
+def test_refinement_on_one_grid(built, w, h, voxel, off):
+    wl, v, o = _map(w, h, voxel)
+    T = np.asarray(wl.pose(5), np.float64)
+    v.set_frame(wl.frame(5), T)
+    start = left_update(T, [off, -off, 0.5 * off, -off, 0.7 * off, off])
+    for n in (0, 1, 6):
+        T1, cost, count = v.refine_pose(start, iterations=n, max_residual=0.05)
+        _, _, cost2, count2 = v.normal_equations(np.linalg.inv(T1.astype(np.float64)).astype(np.float32),
+                                                 max_residual=0.05)
+        assert abs(count - count2) <= 2 + 1e-3 * w * h
+        assert abs(cost - cost2) <= 1e-3 * cost2 + 3 * 0.05 ** 2
+        assert off > 0.1 or count > 0
