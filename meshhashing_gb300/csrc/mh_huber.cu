@@ -16,10 +16,10 @@
 // mask; otherwise the gradient (or divergence) is 0, as in the reference.
 // The per-voxel state (7 words) lives in arrays laid out like the voxel
 // storage, allocated on first use; the mask is an epoch stamp, so voxels not
-// initialised by the latest init read as unmasked.  Init runs one thread per
-// candidate voxel, the iterations one CTA per candidate block over a
-// face-neighbour table and per-voxel flags that are built once per call, so no
-// pass waits on a hash probe or tests its neighbours' weights again.
+// initialised by the latest init read as unmasked.  All passes run one CTA per
+// candidate block over a face-neighbour table; the iterations' per-voxel flags
+// are built once per call, so no pass waits on a hash probe or tests its
+// neighbours' weights again.
 #include <cstring>
 
 #include "mh_kernels.h"
@@ -36,8 +36,6 @@ struct PD {
   unsigned *mask;
   unsigned epoch;
 };
-
-__device__ __forceinline__ float huber(float x, float a) { return fabsf(x) < a ? 0.5f * (x * x) / a : fabsf(x) - 0.5f * a; }
 
 __device__ __forceinline__ int cand_count(const Dev &d) { return *reinterpret_cast<volatile int *>(&d.ctr->cand_count); }
 
@@ -59,113 +57,75 @@ __global__ void __launch_bounds__(256) k_pd_faces(Dev d, int *nbt) {
   }
 }
 
-// Global voxel index of the face neighbour (axis k, direction s) of local
-// voxel li (= x + 8 y + 64 z) of candidate c in pool block blk; -1 when the
-// neighbour's block does not exist.
-template <int K, int S>
-__device__ __forceinline__ long long face(const int *nbt, int c, int blk, int li) {
-  constexpr int sh = 3 * K;
-  const int cn = ((li >> sh) & 7) + S;
-  if ((unsigned)cn > 7u) {
-    const int q = __ldg(nbt + 6 * c + 2 * K + (S < 0));
-    return q < 0 ? -1 : (long long)q * MH_BLOCK_VOXELS + ((li & ~(7 << sh)) | ((cn & 7) << sh));
-  }
-  return (long long)blk * MH_BLOCK_VOXELS + li + S * (1 << sh);
-}
-
-template <int S>
-__device__ __forceinline__ void faces(const int *nbt, int c, int blk, int li, long long (&q)[3]) {
-  q[0] = face<0, S>(nbt, c, blk, li);
-  q[1] = face<1, S>(nbt, c, blk, li);
-  q[2] = face<2, S>(nbt, c, blk, li);
-}
-
 // neighbour usable by the masked queries: block exists, voxel observed, mask set
 __device__ __forceinline__ bool usable(const Dev &d, const PD &pd, long long g) {
   return g >= 0 && d.w[g] >= kEps && pd.mask[g] == pd.epoch;
 }
 
-// The init loop runs one thread per voxel of the candidate list, grid-stride
-// over candidates x 512; a warp covers 32 voxels of one block.
-#define PD_FOR_EACH_VOXEL(d, n)                                                                   \
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < (long long)(n) * 512; \
-       t += (long long)gridDim.x * blockDim.x)
-
-__global__ void __launch_bounds__(256) k_pd_init(Dev d, PD pd, const int *nbt) {
-  const int n = cand_count(d);
-  PD_FOR_EACH_VOXEL(d, n) {
-    const int c = (int)(t >> 9), li = (int)(t & 511);
-    const int blk = d.cand[c].w;
-    if (blk < 0) continue;
-    const long long g = (long long)blk * MH_BLOCK_VOXELS + li;
-    if (d.w[g] < kEps) continue;
-    long long q[3];
-    faces<1>(nbt, c, blk, li, q);
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) ok &= q[k] >= 0 && d.w[q[k]] >= kEps;
-    const float s = d.sdf[g];
-    float gr[3] = {0.0f, 0.0f, 0.0f};
-    if (ok) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) gr[k] = d.sdf[q[k]] - s;
-    }
-    const float len = sqrtf(gr[0] * gr[0] + gr[1] * gr[1] + gr[2] * gr[2]);
-    pd.w[g] = expf(len / d.p.voxel_size);
-    pd.sdf0[g] = s;
-    pd.bar[g] = 0.0f;
-    pd.px[g] = pd.py[g] = pd.pz[g] = 0.0f;
-    pd.mask[g] = pd.epoch;
-  }
-}
-
-// The iterations run one 128-thread CTA per candidate block: thread t holds
+// All passes run one 128-thread CTA per candidate block: thread t holds
 // the four voxels x = 4 (t & 1) .. + 3 of row y = t / 2 & 7 of layer z = t / 16,
 // so a field moves as one float4 per thread.
 __device__ __forceinline__ int first_voxel(int t) { return t * 4; }
 
-// Flags of a call, 16 bits a thread: bits 0-3 the voxel is usable, 4-7 its
-// three upper face neighbours are usable too, 8-11 its three lower ones.
-// Neither pass changes the weights or the mask, so they hold for all
-// iterations of the call.
-__global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, uint16_t *flags) {
-  // usable voxels of the block with a layer around it, 10 x 10 x 10
-  __shared__ uint8_t us[1000];
+// The voxels of a block that the masked queries may use, a byte for each row of
+// 8 voxels along x; `stamp` tells that the block's bytes are of this call.
+__global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, unsigned *stamp, unsigned call) {
   const int n = cand_count(d), t = threadIdx.x;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int blk = d.cand[c].w;
-    if (blk < 0) {
-      flags[(size_t)c * 128 + t] = 0;
-      continue;
-    }
-    const int i0 = first_voxel(t);
-    uint8_t *own = us + (i0 & 7) + 1 + 10 * (((i0 >> 3) & 7) + 1) + 100 * ((i0 >> 6) + 1);
-    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + i0;
+    if (blk < 0) continue;
+    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
     const float4 w = *reinterpret_cast<const float4 *>(d.w + base);
     const uint4 m = *reinterpret_cast<const uint4 *>(pd.mask + base);
-    own[0] = w.x >= kEps && m.x == pd.epoch, own[1] = w.y >= kEps && m.y == pd.epoch;
-    own[2] = w.z >= kEps && m.z == pd.epoch, own[3] = w.w >= kEps && m.w == pd.epoch;
-    for (int i = t; i < 384; i += 128) {
-      const int face = i >> 6, a = i & 7, b = (i >> 3) & 7, k = face >> 1, up = !(face & 1);
-      const int q = __ldg(nbt + 6 * c + face);  // 2 k: upper, 2 k + 1: lower
-      const int in = up ? 0 : 7, out = up ? 9 : 0;
-      const int li = k == 0 ? in + 8 * a + 64 * b : k == 1 ? a + 8 * in + 64 * b : a + 8 * b + 64 * in;
-      const int o = k == 0 ? out + 10 * (a + 1) + 100 * (b + 1) : k == 1 ? a + 1 + 10 * out + 100 * (b + 1)
-                                                                        : a + 1 + 10 * (b + 1) + 100 * out;
-      us[o] = q >= 0 && usable(d, pd, (long long)q * MH_BLOCK_VOXELS + li);
-    }
-    __syncthreads();
     unsigned f = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint8_t *u = own + k;
-      if (!u[0]) continue;
-      f |= 1u << k;
-      if (u[1] && u[10] && u[100]) f |= 16u << k;
-      if (u[-1] && u[-10] && u[-100]) f |= 256u << k;
+    if (w.x >= kEps && m.x == pd.epoch) f |= 1u;
+    if (w.y >= kEps && m.y == pd.epoch) f |= 2u;
+    if (w.z >= kEps && m.z == pd.epoch) f |= 4u;
+    if (w.w >= kEps && m.w == pd.epoch) f |= 8u;
+    const unsigned hi = __shfl_down_sync(0xffffffffu, f, 1);
+    if (!(t & 1)) use[(size_t)blk * 64 + t / 2] = (uint8_t)(f | hi << 4);
+    if (t == 0) stamp[blk] = call;
+  }
+}
+
+// Flags of a call, 16 bits a thread: bits 0-3 the voxel is usable, 4-7 its
+// three upper face neighbours are usable too, 8-11 its three lower ones.
+// Neither pass changes the weights or the mask, so they hold for all
+// iterations of the call.  A thread takes a row from the bytes of k_pd_usable:
+// reading weights and masks of the faces' voxels, a 32-byte sector each along
+// x, took 250 us for 120 k blocks against 134 us for both passes.
+__global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, const uint8_t *use,
+                                                  const unsigned *stamp, unsigned call, uint16_t *flags) {
+  const int n = cand_count(d), row = threadIdx.x & 63, y = row & 7, z = row >> 3;
+  for (int c = blockIdx.x * 2 + (threadIdx.x >> 6); c < n; c += gridDim.x * 2) {
+    const int blk = d.cand[c].w;
+    unsigned *out = reinterpret_cast<unsigned *>(flags) + (size_t)c * 64 + row;
+    if (blk < 0) {
+      *out = 0u;
+      continue;
     }
-    flags[(size_t)c * 128 + t] = (uint16_t)f;
-    __syncthreads();
+    // row r of the neighbour `face`, the voxels `want` of it
+    auto beyond = [&](int face, int r, unsigned want) -> unsigned {
+      const int q = __ldg(nbt + 6 * c + face);
+      if (q < 0) return 0u;
+      if (stamp[q] == call) return use[(size_t)q * 64 + r];
+      unsigned f = 0;
+      for (int x = 0; x < 8; ++x)
+        if ((want >> x & 1u) && usable(d, pd, (long long)q * MH_BLOCK_VOXELS + r * 8 + x)) f |= 1u << x;
+      return f;
+    };
+    const uint8_t *own = use + (size_t)blk * 64;
+    const unsigned u = own[row];
+    unsigned f = 0u;
+    if (u) {
+      const unsigned xu = u >> 1 | (u & 128u ? (beyond(0, row, 1u) & 1u) << 7 : 0u);
+      const unsigned xl = (u << 1 & 255u) | (u & 1u ? beyond(1, row, 128u) >> 7 : 0u);
+      const unsigned yu = y < 7 ? own[row + 1] : beyond(2, row - 7, u), yl = y > 0 ? own[row - 1] : beyond(3, row + 7, u);
+      const unsigned zu = z < 7 ? own[row + 8] : beyond(4, row - 56, u), zl = z > 0 ? own[row - 8] : beyond(5, row + 56, u);
+      const unsigned up = u & xu & yu & zu, lo = u & xl & yl & zl;
+      f = (u & 15u) | (up & 15u) << 4 | (lo & 15u) << 8 | (u >> 4) << 16 | (up >> 4) << 20 | (lo >> 4) << 24;
+    }
+    *out = f;
   }
 }
 
@@ -220,6 +180,59 @@ __device__ __forceinline__ float pd_div(float a, float b, float y) {
   return (m > 0x1p-60f && m < 0x1p60f) || m == 0.0f ? mh_div(a, b, y) : a / b;
 }
 
+// The Huber norm of a vector of squared length n2
+__device__ __forceinline__ float pd_huber(float n2) {
+  const float x = n2 == 0.0f ? 0.0f : n2 > 0x1p-60f && n2 < 0x1p60f ? sqrt_round(n2) : sqrtf(n2);
+  return x < kAlpha ? pd_div(0.5f * (x * x), kAlpha, 1.0f / kAlpha) : x - 0.5f * kAlpha;
+}
+
+// PrimalDualInit: weights from the gradient, the iterate's start.  Bound by the
+// traffic, 36 B a voxel and the faces: 480 us for 120 k blocks.  A thread a voxel
+// took 508 us; without the operators' long ways this form takes 479.
+__global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt) {
+  __shared__ Tile9 sdf, weight;
+  const int n = cand_count(d), t = threadIdx.x;
+  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+    const int blk = d.cand[c].w;
+    if (blk < 0) continue;
+    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
+    const float4 W = load4(d.w, base), S = load4(d.sdf, base);
+    const bool any = W.x >= kEps || W.y >= kEps || W.z >= kEps || W.w >= kEps;
+    if (!__syncthreads_or(any)) continue;
+    tile_own(sdf, t, 0, S), tile_own(weight, t, 0, W);
+    for (int i = t; i < 192; i += 128) {
+      const int k = i >> 6, q = __ldg(nbt + 6 * c + 2 * k), a = i & 7, b = i >> 3 & 7;
+      const int o = k == 0 ? 8 + 9 * a + 81 * b : k == 1 ? a + 72 + 81 * b : a + 9 * b + 648;
+      weight.v[o] = 0.0f;
+      tile_face(sdf, i & 63, k, true, q, d.sdf);
+      tile_face(weight, i & 63, k, true, q, d.w);
+    }
+    __syncthreads();
+    if (any) {
+      const int i0 = first_voxel(t), o0 = (i0 & 7) + 9 * ((i0 >> 3) & 7) + 81 * (i0 >> 6);
+      float w[4], s0[4];
+      unsigned m[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // what a voxel that is not observed gets is not read: its mask differs
+        w[k] = 0.0f, s0[k] = lane4(S, k), m[k] = 0u;
+        if (!(lane4(W, k) >= kEps)) continue;
+        const float *o = sdf.v + o0 + k, *q = weight.v + o0 + k;
+        float gr[3] = {0.0f, 0.0f, 0.0f};
+        if (q[1] >= kEps && q[9] >= kEps && q[81] >= kEps) gr[0] = o[1] - s0[k], gr[1] = o[9] - s0[k], gr[2] = o[81] - s0[k];
+        const float len = sqrtf(gr[0] * gr[0] + gr[1] * gr[1] + gr[2] * gr[2]);
+        w[k] = expf(len / d.p.voxel_size);
+        m[k] = pd.epoch;
+      }
+      const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      store4(pd.w, base, w), store4(pd.sdf0, base, s0), store4(pd.bar, base, zero);
+      store4(pd.px, base, zero), store4(pd.py, base, zero), store4(pd.pz, base, zero);
+      *reinterpret_cast<uint4 *>(pd.mask + base) = make_uint4(m[0], m[1], m[2], m[3]);
+    }
+    __syncthreads();
+  }
+}
+
 // Dual step (PrimalDualIteratePass1Kernel), with the energies where they are
 // asked for.  Bound by the traffic: 28 B a voxel (the extrapolated sdf and the
 // dual read, the dual written; 8 more for the energies) and the faces: 390 us
@@ -267,7 +280,7 @@ __global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, c
         if (f >> (4 + k) & 1u) gs[0] = os[1] - s, gs[1] = os[9] - s, gs[2] = os[81] - s;
         const float dd = fabsf(s - lane4(S0, k));
         e[0] += dd * dd;
-        e[1] += huber(sqrtf(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]), kAlpha);
+        e[1] += pd_huber(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]);
       }
       float x = px[k] + sigma * gb[0], y = py[k] + sigma * gb[1], z = pz[k] + sigma * gb[2];
       if (h_ok) x = pd_div(x, h, rh), y = pd_div(y, h, rh), z = pd_div(z, h, rh);
@@ -347,6 +360,9 @@ struct mh_pd_state {
   double *err = nullptr;
   int *nbt = nullptr;   // face-neighbour table of the candidate list (6 per candidate)
   uint16_t *flags = nullptr;  // per-voxel flags of the call (128 words per candidate)
+  uint8_t *use = nullptr;     // usable voxels, 64 bytes per pool block
+  unsigned *stamp = nullptr;  // call that wrote a block's bytes
+  unsigned call = 0;
   bool fresh = false;         // no iteration since the last init: bar and p are 0
 };
 
@@ -364,6 +380,9 @@ static int pd_ensure(mh_volume *v) {
   ok = ok && cudaMalloc((void **)&st->err, sizeof(double) * 2) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->nbt, sizeof(int) * 6 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->flags, sizeof(uint16_t) * 128 * (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->use, 64 * (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->stamp, sizeof(unsigned) * (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMemset(st->stamp, 0, sizeof(unsigned) * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMemset(st->pd.mask, 0, sizeof(unsigned) * nv) == cudaSuccess;
   st->pd.epoch = 0;
   st->voxels = nv;
@@ -381,7 +400,7 @@ void mh_pd_free(mh_volume *v) {
   if (!st) return;
   for (void *p : {(void *)st->pd.sdf0, (void *)st->pd.bar, (void *)st->pd.w, (void *)st->pd.px, (void *)st->pd.py,
                   (void *)st->pd.pz, (void *)st->pd.mask, (void *)st->err, (void *)st->nbt,
-                  (void *)st->flags})
+                  (void *)st->flags, (void *)st->use, (void *)st->stamp})
     if (p) cudaFree(p);
   delete st;
   v->pd = nullptr;
@@ -397,7 +416,7 @@ int mh_huber_tv_init(mh_volume *v, void *stream) {
   st->pd.epoch += 1;
   cudaStream_t s = (cudaStream_t)stream;
   k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-  k_pd_init<<<grid_of((const void *)k_pd_init), 256, 0, s>>>(v->d, st->pd, st->nbt);
+  k_pd_init<<<grid_of((const void *)k_pd_init, 128), 128, 0, s>>>(v->d, st->pd, st->nbt);
   mh_count_launches(2);
   st->fresh = true;
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
@@ -414,9 +433,12 @@ int mh_huber_tv_iterate(mh_volume *v, float lambda, float sigma, float tau, int 
     // the candidate list may have changed since init: rebuild the face table
     // and the flags of this call (neither pass changes w or the mask)
     k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-    k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags);
+    st->call += 1;
+    k_pd_usable<<<grid_of((const void *)k_pd_usable, 128), 128, 0, s>>>(v->d, st->pd, st->use, st->stamp, st->call);
+    k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->use, st->stamp,
+                                                                     st->call, st->flags);
     MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2, s));
-    mh_count_launches(2);
+    mh_count_launches(3);
   }
   const int gd = grid_of((const void *)k_pd_dual<false>, 128), ge = grid_of((const void *)k_pd_dual<true>, 128),
             gp = grid_of((const void *)k_pd_primal, 128);
