@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) k_pixels_b(const Scene *t, int n) {
 // or behind everything in it.  Of the 640x480 PSDF workload's candidate blocks
 // 38 % update no voxel, and cost about a third of one that does; a thread here
 // drops two thirds of those, and the update takes 771 us with this pass instead
-// of 884 us (320x240 at 6 mm: 163 and 186 us).  A bit for each warp's two layers
+// of 884 us (322x238 at 8 mm: 163 and 186 us).  A bit for each warp's two layers
 // dropped another tenth of the warps and took as much longer itself.
 //
 // The bound is the voxels' box in the camera's axes (cTw may be any matrix) and

@@ -77,7 +77,7 @@ __device__ __forceinline__ unsigned claim_slots(const Dev &d, uint32_t *cw, unsi
 // and that has a voxel which is not non-negative in it or in a block above
 // (otherwise no cube in it is cut).  One thread per candidate, warp-ballot
 // compaction; the blocks above are looked up by eight lanes a candidate.  The
-// mesh pass of a 320x240 PSDF frame at 6 mm takes 119 us with this test and 137
+// mesh pass of a 322x238 PSDF frame at 8 mm takes 119 us with this test and 137
 // us without: most blocks past the gate are observed free space.
 __device__ __forceinline__ void mc_select_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
@@ -148,7 +148,7 @@ __device__ __forceinline__ void mc_end_body(const Dev &d) {
 // block may share too go through the owner's claim word, all slots of an owner
 // with one atomic, and each warp takes its places in the work list at once.  An
 // atomicCAS a cube and edge and an atomicAdd a vertex, one after the other, took
-// 41 us against 18 us for a 320x240 PSDF frame at 6 mm (cold).  What is left is
+// 41 us against 18 us for a 322x238 PSDF frame at 8 mm (cold).  What is left is
 // the latency of a block's chain: candidate, hash, tile, pages, claims.
 __device__ __forceinline__ void mc_cubes_body(const Dev &d, Share sh) {
   __shared__ uint8_t tile[729];
@@ -333,7 +333,7 @@ __device__ __forceinline__ size_t voxel_index(int block, int x, int y, int z) {
 // (GetSpatialValue, :23-66), summed in the reference's order.  Bound by the
 // latency of dependent loads: a thread a vertex, with seven samples one after
 // the other and a hash lookup for every corner in another block, took 52 us
-// against 17 us for a 320x240 PSDF frame at 6 mm (cold).
+// against 17 us for a 322x238 PSDF frame at 8 mm (cold).
 __device__ __forceinline__ void mc_vertices_body(const Dev &d, Share sh) {
   const int n = min(*reinterpret_cast<volatile int *>(&d.ctr->vwork_count), d.vwork_capacity);
   const int per_cta = blockDim.x / 8, stride = sh.stride * per_cta;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(512) k_mc_triangles_b(const Scene *t, int n) {
 // Both passes read a page's slots as vectors, all of them before the first is
 // looked at: what bounds them is the latency of one load after the other.  A
 // slot at a time, and the triangle slots again for each page's end, took 15 and
-// 17 us against 11 and 7 us for a 320x240 PSDF frame at 6 mm (cold).
+// 17 us against 11 and 7 us for a 322x238 PSDF frame at 8 mm (cold).
 __device__ __forceinline__ void mc_recycle_tri_body(const Dev &d, Share sh) {
   constexpr int N = MH_BLOCK_VOXELS * 5 / 4 / MC_RECYCLE_THREADS;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->mesh_list_count);
