@@ -35,7 +35,7 @@ __global__ void k_gc_life_b(const Scene *t, int n) {
 
 // CollectLowSurfelBlocksKernel, second half (recycle.cu:102-113).  Eight lanes a
 // candidate, six with a neighbour each: one after the other the six dependent
-// lookups took 22 us against 9 us for a 322x238 PSDF frame at 8 mm (cold).
+// lookups took 18 us against 10 us for a 322x238 PSDF frame at 8 mm (cold).
 __device__ __forceinline__ void gc_flag_body(const Dev &d, Share sh) {
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->cand_count);
   const int j = threadIdx.x & 7, per_cta = blockDim.x / 8;

@@ -148,7 +148,7 @@ __device__ __forceinline__ void mc_end_body(const Dev &d) {
 // block may share too go through the owner's claim word, all slots of an owner
 // with one atomic, and each warp takes its places in the work list at once.  An
 // atomicCAS a cube and edge and an atomicAdd a vertex, one after the other, took
-// 41 us against 18 us for a 322x238 PSDF frame at 8 mm (cold).  What is left is
+// 141 us against 55 us for a 322x238 PSDF frame at 8 mm (cold).  What is left is
 // the latency of a block's chain: candidate, hash, tile, pages, claims.
 __device__ __forceinline__ void mc_cubes_body(const Dev &d, Share sh) {
   __shared__ uint8_t tile[729];
@@ -332,8 +332,8 @@ __device__ __forceinline__ size_t voxel_index(int block, int x, int y, int z) {
 // spatial_query.h:68-97) and each of eight one corner of the radius
 // (GetSpatialValue, :23-66), summed in the reference's order.  Bound by the
 // latency of dependent loads: a thread a vertex, with seven samples one after
-// the other and a hash lookup for every corner in another block, took 52 us
-// against 17 us for a 322x238 PSDF frame at 8 mm (cold).
+// the other and a hash lookup for every corner in another block, took 78 us
+// against 52 us for a 322x238 PSDF frame at 8 mm (cold).
 __device__ __forceinline__ void mc_vertices_body(const Dev &d, Share sh) {
   const int n = min(*reinterpret_cast<volatile int *>(&d.ctr->vwork_count), d.vwork_capacity);
   const int per_cta = blockDim.x / 8, stride = sh.stride * per_cta;
@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(512) k_mc_triangles_b(const Scene *t, int n) {
 // ------------------------------------------------------------------ recycle
 // Both passes read a page's slots as vectors, all of them before the first is
 // looked at: what bounds them is the latency of one load after the other.  A
-// slot at a time, and the triangle slots again for each page's end, took 15 and
-// 17 us against 11 and 7 us for a 322x238 PSDF frame at 8 mm (cold).
+// slot at a time, and the triangle slots again for each page's end, took 17 and
+// 20 us against 12 and 8 us for a 322x238 PSDF frame at 8 mm (cold).
 __device__ __forceinline__ void mc_recycle_tri_body(const Dev &d, Share sh) {
   constexpr int N = MH_BLOCK_VOXELS * 5 / 4 / MC_RECYCLE_THREADS;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->mesh_list_count);
