@@ -297,6 +297,9 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
   if (!b || !depth || !wTc || tv_iterations < 0 || (tv_iterations > 0 && !(tv_lambda > 0.0f))) return MH_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
   const int n = b->n;
+  // a step that is refused leaves every scene as it was
+  for (int i = 0; i < n; ++i)
+    if ((!active || active[i]) && !depth[i]) return MH_ERR_INVALID;
   const int p = b->step & 1;
   // the block of two steps ago must have been consumed before it is rewritten
   if (b->block_used[p]) MH_CUDA_TRY(cudaEventSynchronize(b->block_free[p]));
@@ -328,7 +331,6 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
     sc.recycle = sc.starve = 0;
     if (!act) continue;
     const size_t np = (size_t)v->hp.width * v->hp.height;
-    if (!depth[i]) return MH_ERR_INVALID;
     if (depth_on_device) {
       sc.src = depth[i];
     } else {
@@ -337,16 +339,14 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
     }
     // MainEngine's frame counter: recycle every 10 frames, starvation
     // (simple update) at frame 14 of every 15 (main_engine.cc:163-191)
-    v->frames += 1;
-    sc.recycle = v->frames % 10 == 0;
-    sc.starve = !v->hp.enable_bayesian_update && v->frames % 15 == 14;
+    const int frame = v->frames + 1;
+    sc.recycle = frame % 10 == 0;
+    sc.starve = !v->hp.enable_bayesian_update && frame % 15 == 14;
     FrameConst &fc = fcs[i];
     memcpy(fc.wTc, wTc + 16 * i, sizeof(float) * 16);
     inverse4(fc.wTc, fc.cTw);
     memcpy(fc.rc_cTw, fc.cTw, sizeof(float) * 16);
     inverse4(fc.rc_cTw, fc.rc_wTc);
-    v->fc_host = fc;
-    v->has_frame = true;
     if (b->raycast) sc.d.grid = ray_grid_for(v->hp, fc.rc_wTc, v->grid);
   }
   const bool host_depth = !depth_on_device;
@@ -375,6 +375,14 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
   } else {
     const int r = enqueue(b, p, host_depth, tv_iterations, tv_lambda, tuning, s);
     if (r != MH_OK) return r;
+  }
+  for (int i = 0; i < n; ++i) {
+    if (!tab[i].active) continue;
+    mh_volume *v = b->vols[i];
+    v->frames += 1;
+    v->fc_host = fcs[i];
+    v->has_frame = true;
+    ray_grid_enqueued(v->grid, tab[i].d.grid);
   }
   MH_CUDA_TRY(cudaEventRecord(b->block_free[p], s));
   b->block_used[p] = true;

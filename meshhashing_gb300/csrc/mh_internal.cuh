@@ -23,6 +23,7 @@
 
 #include "../../include/meshhash.h"
 #include "mh_div.h"
+#include "mh_ray_grid.h"
 
 #define MH_BLOCK_SIDE 8
 #define MH_BLOCK_VOXELS 512
@@ -97,29 +98,6 @@ struct DevParams {
   float min_raycast_depth, max_raycast_depth, raycast_step, sample_sdf_threshold, sdf_threshold;
   int enable_gradients, enable_bayesian;
   int compat;  // evaluate the reference's formulas as written
-};
-
-// The cells of a raycast's view: a bit per cell of U = 2 << shift voxels in
-// the view's bounding box.  A word holds 4 x 4 x 2 cells, so with U = 2 two
-// words hold a block (mh_raycast.cu).
-#define MH_GRID_BIAS 49152.0f        // 1.5 * 2^15: a float there has 8 bits of fraction
-#define MH_GRID_MAX_WORDS (1u << 25) // 128 MB
-struct RayGrid {
-  unsigned *bits;            // null: no grid, every sample is evaluated
-  int cx, cy, cz;            // first cell on each axis (a multiple of 4), in cells from the world's origin
-  unsigned nx, ny, nz;       // words on each axis
-  unsigned words;            // nx * ny * nz
-  int shift;                 // U = 2 << shift
-  float ox, oy, oz;          // world position of the first cell's lower corner
-  float inv_cell;            // 1 / (U voxel sizes)
-  // The blocks of the same box: entry (z bny + y) bnx + x holds tag | block
-  // index for a block that exists, anything with another top byte otherwise.
-  unsigned *blocks;          // null: blocks are looked up in the hash table
-  int bx, by, bz;            // first block on each axis
-  unsigned bnx, bny, bnz;
-  unsigned tag;              // this raycast's top byte, 1 .. 255
-  unsigned clear;            // the tags start over: entries to clear first (all that the buffer has), else 0
-  bool filled;               // the buffers hold this grid already
 };
 
 // Everything a kernel needs, passed by value (pointers + params).

@@ -19,16 +19,6 @@ int launch_predict_inlier(const Dev &d, cudaStream_t s);
 
 int launch_mesh(const Dev &d, cudaStream_t s);
 
-// A volume's buffers for its view's grid: sizes for any view, and the grid of
-// the view from wTc in them (their next tag).
-struct RayGridBuf {
-  unsigned *bits = nullptr, *blocks = nullptr;
-  unsigned words = 0, entries = 0;
-  unsigned tag = 0;
-};
-void ray_grid_sizes(const mh_params &P, RayGridBuf &b);
-RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf &b, double margin = 0.0);
-bool ray_grid_covers(const mh_params &P, const float wTc[16], const RayGrid &g);
 int launch_raycast(const Dev &d, float *depth, float *vert4, float *norm4, cudaStream_t s);
 int launch_count_flags(const uint8_t *flags, int n, int *out, cudaStream_t s);
 

@@ -544,7 +544,10 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
   const size_t n = (size_t)v->hp.rc_width * v->hp.rc_height;
   if (on_device) {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
-    return launch_raycast(with_ray_grid(v), depth, vert4, norm4, s);
+    const Dev d = with_ray_grid(v);
+    TRY(launch_raycast(d, depth, vert4, norm4, s));
+    ray_grid_enqueued(v->grid, d.grid);
+    return MH_OK;
   }
   float *dd = depth ? v->rc_stage : nullptr;
   // vertices and normals are written as float4: they start on such a boundary
@@ -552,7 +555,9 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
   float *dn = norm4 ? v->rc_stage + (n + 3) / 4 * 4 + 4 * n : nullptr;
   {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
-    TRY(launch_raycast(with_ray_grid(v), dd, dv, dn, s));
+    const Dev d = with_ray_grid(v);
+    TRY(launch_raycast(d, dd, dv, dn, s));
+    ray_grid_enqueued(v->grid, d.grid);
   }
   if (depth) MH_CUDA_TRY(cudaMemcpyAsync(depth, dd, n * sizeof(float), cudaMemcpyDeviceToHost, s));
   if (vert4) MH_CUDA_TRY(cudaMemcpyAsync(vert4, dv, n * 4 * sizeof(float), cudaMemcpyDeviceToHost, s));

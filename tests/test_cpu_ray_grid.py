@@ -1,0 +1,88 @@
+"""The view grid's host side (csrc/mh_ray_grid.h), compiled for the host.
+
+A grid asks for the block array's clear when the memory is new or its tags have
+started over.  A caller may drop a grid before anything of it is enqueued; the
+clear has to stay due until it is.
+"""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from meshhashing_gb300 import config, scene
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SRC = '''
+#include "mh_ray_grid.h"
+static mh_params P;
+static RayGridBuf B;
+static unsigned memory[1];
+extern "C" void set_up(const mh_params *p) {
+  P = *p;
+  B = RayGridBuf{};
+  ray_grid_sizes(P, B);
+  B.bits = B.blocks = memory;  // not written here
+}
+extern "C" unsigned entries() { return B.entries; }
+extern "C" void draw(const float *wTc, int enqueue, unsigned *tag, unsigned *clear) {
+  const RayGrid g = ray_grid_for(P, wTc, B);
+  *tag = g.tag >> 24;
+  *clear = g.clear;
+  if (enqueue) ray_grid_enqueued(B, g);
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("grid")
+    (d / "g.cpp").write_text(SRC)
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-I",
+                           os.path.join(ROOT, "meshhashing_gb300", "csrc"), str(d / "g.cpp"), "-o", str(d / "g.so")])
+    return C.CDLL(str(d / "g.so"))
+
+
+def _draws(lib, enqueued):
+    wl = scene.full_spline(2, width=36, height=28)
+    p = config.params_for(wl, voxel_size=0.008, truncation=0.024, value_capacity=1 << 16)
+    lib.set_up(C.byref(p))
+    T = np.ascontiguousarray(np.asarray(wl.pose(1), np.float32).reshape(16))
+    out = []
+    for ok in enqueued:
+        tag, clear = C.c_uint(), C.c_uint()
+        lib.draw(T.ctypes.data_as(C.c_void_p), int(ok), C.byref(tag), C.byref(clear))
+        out.append((tag.value, clear.value))
+    assert lib.entries() > 0
+    return out, lib.entries()
+
+
+def _stale_read(lib, enqueued):
+    """Whether a raycast that was enqueued finds entries with its tag that an
+    earlier raycast, or the memory's last owner, left."""
+    draws, entries = _draws(lib, enqueued)
+    left = set(range(256))               # tags that the array may hold
+    for (tag, clear), ok in zip(draws, enqueued):
+        assert 1 <= tag <= 255 and clear in (0, entries)
+        if not ok:
+            continue
+        if clear:
+            left = set()
+        if tag in left:
+            return True
+        left.add(tag)
+    return False
+
+
+@pytest.mark.parametrize("lost", [[], [0], [0, 1], [254], [255], [253, 254, 255, 256], [0, 254, 255, 509, 510, 511],
+                                  list(range(0, 800, 3))])
+def test_clear_stays_due(lib, lost):
+    assert not _stale_read(lib, [k not in lost for k in range(800)])
+
+
+def test_a_clear_is_asked_for_once(lib):
+    draws, entries = _draws(lib, [True] * 600)
+    clears = [k for k, (_, clear) in enumerate(draws) if clear]
+    assert clears[0] == 0 and len(clears) == 3 and all(b - a >= 250 for a, b in zip(clears, clears[1:]))
