@@ -382,7 +382,7 @@ int mh_batch_step(mh_batch *b, const float *const *depth, int depth_on_device, c
     v->frames += 1;
     v->fc_host = fcs[i];
     v->has_frame = true;
-    ray_grid_enqueued(v->grid, tab[i].d.grid);
+    ray_grid_sent(v, tab[i].d.grid, s);
   }
   MH_CUDA_TRY(cudaEventRecord(b->block_free[p], s));
   b->block_used[p] = true;

@@ -20,6 +20,9 @@ int launch_predict_inlier(const Dev &d, cudaStream_t s);
 int launch_mesh(const Dev &d, cudaStream_t s);
 
 int launch_raycast(const Dev &d, float *depth, float *vert4, float *norm4, cudaStream_t s);
+// the same for a stream that is being captured; `table`: one entry, device
+int launch_raycast_replayed(const Dev &d, const mh_params &P, const RayGridBuf &b, Scene *table, float *depth,
+                            float *vert4, float *norm4, cudaStream_t s);
 int launch_count_flags(const uint8_t *flags, int n, int *out, cudaStream_t s);
 
 int launch_gc_low_surfel(const Dev &d, cudaStream_t s);

@@ -252,7 +252,7 @@ int mh_raycast_backward(mh_volume *v, const float cTw[16], const float *dL_ddept
   if (cudaMemsetAsync(v->acc, 0, sizeof(double) * 32, s) != cudaSuccess) return MH_ERR_CUDA;
   const Dev d = with_ray_grid(v);
   if ((r = launch_raycast_grad(d, 0, dL_ddepth, dL_dnormal4, grad_sdf, nullptr, 0.0f, v->acc, s)) != MH_OK) return r;
-  ray_grid_enqueued(v->grid, d.grid);
+  ray_grid_sent(v, d.grid, s);
   double h[6];
   if (cudaMemcpyAsync(h, v->acc, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
@@ -289,7 +289,7 @@ static int raycast_normal_equations(mh_volume *v, const float cTw[16], const flo
   if (kept && ray_grid_covers(v->hp, rc_wTc, *kept)) d.grid = *kept;
   else d.grid = ray_grid_for(v->hp, rc_wTc, v->grid, kept ? kKeptMargin * v->hp.max_raycast_depth : 0.0);
   if ((r = launch_raycast_grad(d, 1, nullptr, nullptr, nullptr, obs, max_residual, v->acc, s)) != MH_OK) return r;
-  ray_grid_enqueued(v->grid, d.grid);
+  ray_grid_sent(v, d.grid, s);
   if (kept) {
     *kept = d.grid;
     kept->filled = true;

@@ -1,17 +1,25 @@
 // mh_ray_grid.h -- the grid of a raycast's view: where its cells and blocks lie,
-// and the buffers that hold them.  Host arithmetic only; mh_raycast.cu fills and
-// reads the grid.
+// and the buffers that hold them.  mh_raycast.cu fills and reads the grid.  The
+// host makes it from the pose that it uploads; a raycast that a graph replays
+// makes it on the device from the pose that it finds there.
 #pragma once
 #include <algorithm>
 #include <cmath>
 
 #include "../../include/meshhash.h"
 
+#if defined(__CUDACC__)
+#define MH_GRID_HD __host__ __device__
+#else
+#define MH_GRID_HD
+#endif
+
 // The cells of a raycast's view: a bit per cell of U = 2 << shift voxels in
 // the view's bounding box.  A word holds 4 x 4 x 2 cells, so with U = 2 two
 // words hold a block (mh_raycast.cu).
 #define MH_GRID_BIAS 49152.0f        // 1.5 * 2^15: a float there has 8 bits of fraction
 #define MH_GRID_MAX_WORDS (1u << 25) // 128 MB
+#define MH_GRID_REPLAY_TAG 255u      // top byte of blocks written by replayed raycasts
 struct RayGrid {
   unsigned *bits;            // null: no grid, every sample is evaluated
   int cx, cy, cz;            // first cell on each axis (a multiple of 4), in cells from the world's origin
@@ -25,7 +33,7 @@ struct RayGrid {
   unsigned *blocks;          // null: blocks are looked up in the hash table
   int bx, by, bz;            // first block on each axis
   unsigned bnx, bny, bnz;
-  unsigned tag;              // this raycast's top byte, 1 .. 255
+  unsigned tag;              // this raycast's top byte, 1 .. 254, or MH_GRID_REPLAY_TAG
   unsigned clear;            // entries to clear first (all that the buffer has), 0 where old ones cannot be mistaken
   bool filled;               // the buffers hold this grid already
 };
@@ -41,7 +49,7 @@ struct RayGridBuf {
 // the view's corner rays at z = 1: x and y ranges, and the longest of them
 struct ViewCone {
   double x[2], y[2], len;
-  explicit ViewCone(const mh_params &P) {
+  MH_GRID_HD explicit ViewCone(const mh_params &P) {
     x[0] = (0.0 - P.rc_cx) / P.rc_fx, x[1] = ((double)P.rc_width - 1.0 - P.rc_cx) / P.rc_fx;
     y[0] = (0.0 - P.rc_cy) / P.rc_fy, y[1] = ((double)P.rc_height - 1.0 - P.rc_cy) / P.rc_fy;
     const double mx = std::max(std::fabs(x[0]), std::fabs(x[1])), my = std::max(std::fabs(y[0]), std::fabs(y[1]));
@@ -68,7 +76,7 @@ inline void ray_grid_sizes(const mh_params &P, RayGridBuf &b) {
 // ray, so the box is the hull of the view's eight corners when wTc is rigid;
 // any other matrix gets the ball that holds every ray (their directions are
 // normalised).
-inline bool view_box(const mh_params &P, const float wTc[16], double lo[3], double hi[3]) {
+MH_GRID_HD inline bool view_box(const mh_params &P, const float wTc[16], double lo[3], double hi[3]) {
   const ViewCone v(P);
   bool rigid = true;
   for (int i = 0; i < 3; ++i)
@@ -99,7 +107,7 @@ inline bool view_box(const mh_params &P, const float wTc[16], double lo[3], doub
 
 // The smallest cells (U = 2, 4, ... voxels) for which a box fits the words and
 // the coordinates' rounding (4 units in the last place) stays below 1/128 cell.
-inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], const double hi[3], const RayGridBuf &b) {
+MH_GRID_HD inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], const double hi[3], const RayGridBuf &b) {
   RayGrid g{};
   double far = 0.0;
   for (int a = 0; a < 3; ++a) far = std::max(far, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
@@ -153,10 +161,24 @@ inline RayGrid ray_grid_for(const mh_params &P, const float wTc[16], RayGridBuf 
     if (wide.bits && wide.shift == g.shift && !wide.blocks == !g.blocks) g = wide;
   }
   if (g.blocks) {
-    if (b.tag == 255u) b.tag = 0u, b.dirty = true;
+    if (b.tag + 1u == MH_GRID_REPLAY_TAG) b.tag = 0u, b.dirty = true;
     b.tag += 1u;
     g.tag = b.tag << 24;
     g.clear = b.dirty ? b.entries : 0u;
+  }
+  return g;
+}
+
+// The same for a raycast whose launches a graph replays.  Its tag is that of all
+// replays, so each replay clears the entries of its own box first, and no other
+// raycast uses that tag.
+MH_GRID_HD inline RayGrid ray_grid_replayed(const mh_params &P, const float wTc[16], const RayGridBuf &b) {
+  double lo[3], hi[3];
+  if (!b.bits || !view_box(P, wTc, lo, hi)) return RayGrid{};
+  RayGrid g = ray_grid_of(P, lo, hi, b);
+  if (g.blocks) {
+    g.tag = MH_GRID_REPLAY_TAG << 24;
+    g.clear = g.bnx * g.bny * g.bnz;
   }
   return g;
 }

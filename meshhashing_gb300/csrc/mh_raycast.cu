@@ -816,6 +816,31 @@ int launch_batch_ray_grid(const Scene *t, int n, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 
+// A raycast that a graph replays: the launches are recorded once, the pose and
+// the map are those of each replay, so the grid has to be made on the device.  One
+// thread writes it, with the scene, into a table of one entry, and the batch's
+// kernels run over that table.
+__global__ void k_ray_scene(Scene scene, mh_params P, RayGridBuf b, Scene *table) {
+  scene.d.grid = ray_grid_replayed(P, scene.d.fc->rc_wTc, b);
+  *table = scene;
+}
+int launch_raycast_replayed(const Dev &d, const mh_params &P, const RayGridBuf &b, Scene *table, float *depth,
+                            float *vert4, float *norm4, cudaStream_t s) {
+  Scene scene{};
+  scene.d = d;
+  scene.ray_depth = depth;
+  scene.ray_vert = reinterpret_cast<float4 *>(vert4);
+  scene.ray_norm = reinterpret_cast<float4 *>(norm4);
+  scene.active = 1;
+  k_ray_scene<<<1, 1, 0, s>>>(scene, P, b, table);
+  mh_count_launches(1);
+  const int r = launch_batch_ray_grid(table, 1, s);
+  if (r != MH_OK) return r;
+  int tx, ty;
+  ray_tile_shape(0, tx, ty);
+  return launch_raycast_batch(table, 1, ((P.rc_width + tx - 1) / tx) * ((P.rc_height + ty - 1) / ty), 0, s);
+}
+
 // number of nonzero bytes of flags[0, n) added to *out
 __global__ void k_count_flags(const uint8_t *flags, int n, int *out) {
   int c = 0;

@@ -16,6 +16,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "mh_batch.cuh"
 #include "mh_internal.cuh"
 #include "mh_kernels.h"
 #include "mh_volume.h"
@@ -205,6 +206,15 @@ static Counters read_counters(mh_volume *v) {
     if (_r != MH_OK) return _r;   \
   } while (0)
 
+bool mh_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
+void ray_grid_sent(mh_volume *v, const RayGrid &g, cudaStream_t s) {
+  if (!mh_capturing(s)) ray_grid_enqueued(v->grid, g);
+}
+
 // The volume's device state with the grid of the raycast pose's view.
 Dev with_ray_grid(mh_volume *v) {
   Dev d = v->d;
@@ -380,6 +390,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   ray_grid_sizes(P, v->grid);
   A(dalloc(v, &v->grid.bits, v->grid.words));
   if (v->grid.entries) A(dalloc(v, &v->grid.blocks, v->grid.entries));
+  A(dalloc(v, &v->ray_scene, 1));
   A(dalloc(v, &d.mesh_list, cap));
   A(dalloc(v, &d.cube_list, cap));
   d.upd_list = d.cube_list;
@@ -544,9 +555,10 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
   const size_t n = (size_t)v->hp.rc_width * v->hp.rc_height;
   if (on_device) {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
+    if (mh_capturing(s)) return launch_raycast_replayed(v->d, v->hp, v->grid, v->ray_scene, depth, vert4, norm4, s);
     const Dev d = with_ray_grid(v);
     TRY(launch_raycast(d, depth, vert4, norm4, s));
-    ray_grid_enqueued(v->grid, d.grid);
+    ray_grid_sent(v, d.grid, s);
     return MH_OK;
   }
   float *dd = depth ? v->rc_stage : nullptr;
@@ -557,7 +569,7 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
     StageScope sc(v, MH_STAGE_RAYCAST, s);
     const Dev d = with_ray_grid(v);
     TRY(launch_raycast(d, dd, dv, dn, s));
-    ray_grid_enqueued(v->grid, d.grid);
+    ray_grid_sent(v, d.grid, s);
   }
   if (depth) MH_CUDA_TRY(cudaMemcpyAsync(depth, dd, n * sizeof(float), cudaMemcpyDeviceToHost, s));
   if (vert4) MH_CUDA_TRY(cudaMemcpyAsync(vert4, dv, n * 4 * sizeof(float), cudaMemcpyDeviceToHost, s));

@@ -17,6 +17,7 @@ struct mh_volume {
   float *tv = nullptr;
   float *rc_stage = nullptr;  // device staging for host raycast outputs
   RayGridBuf grid;            // cells and blocks of the raycast's view
+  Scene *ray_scene = nullptr; // device: the scene of a replayed raycast
   double *acc = nullptr;      // reduction target of the raycast gradients (allocated on first use)
   uint8_t *touch = nullptr;   // raycast footprint flags, one per block (allocated on first use)
   mh_pd_state *pd = nullptr;  // Huber-TV state (allocated on first use)
@@ -45,6 +46,10 @@ struct mh_volume {
 // 4x4 inverse by cofactors with the term order of float4x4::getInverse
 // (extern/cuda/matrix.h:964-1086)
 void inverse4(const float *m, float *out);
+// whether work given to s is, or may be, recorded for later replays instead of run
+bool mh_capturing(cudaStream_t s);
+// the work that clears and fills g, the volume's last grid, has been given to s
+void ray_grid_sent(mh_volume *v, const RayGrid &g, cudaStream_t s);
 // the device state with the grid of the raycast pose's view (fc_host.rc_wTc)
 Dev with_ray_grid(mh_volume *v);
 // releases the Huber-TV state of a volume (mh_huber.cu)
