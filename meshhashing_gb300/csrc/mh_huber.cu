@@ -68,8 +68,9 @@ __device__ __forceinline__ bool usable(const Dev &d, const PD &pd, long long g) 
 __device__ __forceinline__ int first_voxel(int t) { return t * 4; }
 
 // The voxels of a block that the masked queries may use, a byte for each row of
-// 8 voxels along x; `stamp` tells that the block's bytes are of this call.
-__global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, unsigned *stamp, unsigned call) {
+// 8 voxels along x; `known` (cleared before) tells that the block's bytes are of
+// this call.
+__global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, uint8_t *known) {
   const int n = cand_count(d), t = threadIdx.x;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int blk = d.cand[c].w;
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, u
     if (w.w >= kEps && m.w == pd.epoch) f |= 8u;
     const unsigned hi = __shfl_down_sync(0xffffffffu, f, 1);
     if (!(t & 1)) use[(size_t)blk * 64 + t / 2] = (uint8_t)(f | hi << 4);
-    if (t == 0) stamp[blk] = call;
+    if (t == 0) known[blk] = 1;
   }
 }
 
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, u
 // reading weights and masks of the faces' voxels, a 32-byte sector each along
 // x, took 250 us for 120 k blocks against 134 us for both passes.
 __global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, const uint8_t *use,
-                                                  const unsigned *stamp, unsigned call, uint16_t *flags) {
+                                                  const uint8_t *known, uint16_t *flags) {
   const int n = cand_count(d), row = threadIdx.x & 63, y = row & 7, z = row >> 3;
   for (int c = blockIdx.x * 2 + (threadIdx.x >> 6); c < n; c += gridDim.x * 2) {
     const int blk = d.cand[c].w;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, 
     auto beyond = [&](int face, int r, unsigned want) -> unsigned {
       const int q = __ldg(nbt + 6 * c + face);
       if (q < 0) return 0u;
-      if (stamp[q] == call) return use[(size_t)q * 64 + r];
+      if (known[q]) return use[(size_t)q * 64 + r];
       unsigned f = 0;
       for (int x = 0; x < 8; ++x)
         if ((want >> x & 1u) && usable(d, pd, (long long)q * MH_BLOCK_VOXELS + r * 8 + x)) f |= 1u << x;
@@ -189,9 +190,10 @@ __device__ __forceinline__ float pd_huber(float n2) {
 // PrimalDualInit: weights from the gradient, the iterate's start.  Bound by the
 // traffic, 36 B a voxel and the faces: 480 us for 120 k blocks.  A thread a voxel
 // took 508 us; without the operators' long ways this form takes 479.
-__global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt) {
+__global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt, unsigned *fresh) {
   __shared__ Tile9 sdf, weight;
   const int n = cand_count(d), t = threadIdx.x;
+  if (blockIdx.x == 0 && t == 0) *fresh = pd.epoch;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int blk = d.cand[c].w;
     if (blk < 0) continue;
@@ -238,14 +240,17 @@ __global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt) {
 // dual read, the dual written; 8 more for the energies) and the faces: 390 us
 // for 120 k blocks.  One thread per entry of
 // a list of usable voxels took 660 us and read 12 B more a voxel; with the
-// operators' divisions this form takes 700 us.
+// operator's divisions this form takes 700 us.  After an init, before the first
+// primal step (fresh), the extrapolated sdf is 0 and so is the new dual: there is
+// nothing to do.  The device knows that, since graphs may replay the calls.
 template <bool kEnergy>
-__global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, const uint16_t *flags, float sigma,
-                                                 double *err) {
+__global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, const uint16_t *flags,
+                                                 const unsigned *fresh, float sigma, double *err) {
   __shared__ Tile9 bar, sdf;
   const int n = cand_count(d), t = threadIdx.x;
   const float h = 1.0f + sigma * kAlpha, rh = 1.0f / h;
   const bool h_ok = h > 0x1p-20f && h < 0x1p20f;
+  if (!kEnergy && h_ok && *fresh == pd.epoch) return;
   float e[2] = {0.0f, 0.0f};
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const unsigned f = flags[(size_t)c * 128 + t];
@@ -305,10 +310,11 @@ __global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, c
 // traffic: 32 B a voxel (the dual, sdf, sdf0 and the weight read, sdf and its
 // extrapolation written) and the faces: 382 us for 120 k blocks, 5.1 TB/s
 // without the faces.
-__global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt, const uint16_t *flags, float lambda,
-                                                   float tau) {
+__global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt, const uint16_t *flags,
+                                                   unsigned *fresh, float lambda, float tau) {
   __shared__ Tile9 tx, ty, tz;
   const int n = cand_count(d), t = threadIdx.x;
+  if (blockIdx.x == 0 && t == 0) *fresh = 0u;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const unsigned f = flags[(size_t)c * 128 + t];
     if (!__syncthreads_or(f)) continue;
@@ -361,9 +367,8 @@ struct mh_pd_state {
   int *nbt = nullptr;   // face-neighbour table of the candidate list (6 per candidate)
   uint16_t *flags = nullptr;  // per-voxel flags of the call (128 words per candidate)
   uint8_t *use = nullptr;     // usable voxels, 64 bytes per pool block
-  unsigned *stamp = nullptr;  // call that wrote a block's bytes
-  unsigned call = 0;
-  bool fresh = false;         // no iteration since the last init: bar and p are 0
+  uint8_t *known = nullptr;   // blocks whose bytes this call wrote
+  unsigned *fresh = nullptr;  // epoch of an init that no primal step has followed: bar and p are 0
 };
 
 static int grid_of(const void *fn, int block = 256) { return mh_resident_grid(fn, block, 2048 / block); }
@@ -381,8 +386,8 @@ static int pd_ensure(mh_volume *v) {
   ok = ok && cudaMalloc((void **)&st->nbt, sizeof(int) * 6 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->flags, sizeof(uint16_t) * 128 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->use, 64 * (size_t)v->hp.value_capacity) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&st->stamp, sizeof(unsigned) * (size_t)v->hp.value_capacity) == cudaSuccess;
-  ok = ok && cudaMemset(st->stamp, 0, sizeof(unsigned) * (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->known, (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->fresh, sizeof(unsigned)) == cudaSuccess;
   ok = ok && cudaMemset(st->pd.mask, 0, sizeof(unsigned) * nv) == cudaSuccess;
   st->pd.epoch = 0;
   st->voxels = nv;
@@ -400,7 +405,7 @@ void mh_pd_free(mh_volume *v) {
   if (!st) return;
   for (void *p : {(void *)st->pd.sdf0, (void *)st->pd.bar, (void *)st->pd.w, (void *)st->pd.px, (void *)st->pd.py,
                   (void *)st->pd.pz, (void *)st->pd.mask, (void *)st->err, (void *)st->nbt,
-                  (void *)st->flags, (void *)st->use, (void *)st->stamp})
+                  (void *)st->flags, (void *)st->use, (void *)st->known, (void *)st->fresh})
     if (p) cudaFree(p);
   delete st;
   v->pd = nullptr;
@@ -416,9 +421,8 @@ int mh_huber_tv_init(mh_volume *v, void *stream) {
   st->pd.epoch += 1;
   cudaStream_t s = (cudaStream_t)stream;
   k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-  k_pd_init<<<grid_of((const void *)k_pd_init, 128), 128, 0, s>>>(v->d, st->pd, st->nbt);
+  k_pd_init<<<grid_of((const void *)k_pd_init, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->fresh);
   mh_count_launches(2);
-  st->fresh = true;
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 
@@ -433,24 +437,23 @@ int mh_huber_tv_iterate(mh_volume *v, float lambda, float sigma, float tau, int 
     // the candidate list may have changed since init: rebuild the face table
     // and the flags of this call (neither pass changes w or the mask)
     k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-    st->call += 1;
-    k_pd_usable<<<grid_of((const void *)k_pd_usable, 128), 128, 0, s>>>(v->d, st->pd, st->use, st->stamp, st->call);
-    k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->use, st->stamp,
-                                                                     st->call, st->flags);
+    MH_CUDA_TRY(cudaMemsetAsync(st->known, 0, (size_t)v->hp.value_capacity, s));
+    k_pd_usable<<<grid_of((const void *)k_pd_usable, 128), 128, 0, s>>>(v->d, st->pd, st->use, st->known);
+    k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->use, st->known,
+                                                                     st->flags);
     MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2, s));
     mh_count_launches(3);
   }
   const int gd = grid_of((const void *)k_pd_dual<false>, 128), ge = grid_of((const void *)k_pd_dual<true>, 128),
             gp = grid_of((const void *)k_pd_primal, 128);
   for (int it = 0; it < iterations; ++it) {
-    // only the last pass's energies are returned; the first dual step after
-    // init leaves p = 0 (bar is 0)
-    const bool last = it + 1 == iterations;
-    if (last) k_pd_dual<true><<<ge, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, sigma, st->err);
-    else if (!st->fresh) k_pd_dual<false><<<gd, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, sigma, nullptr);
-    k_pd_primal<<<gp, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, lambda, tau);
-    mh_count_launches(last || !st->fresh ? 2 : 1);
-    st->fresh = false;
+    // only the last pass's energies are returned
+    if (it + 1 == iterations)
+      k_pd_dual<true><<<ge, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, sigma, st->err);
+    else
+      k_pd_dual<false><<<gd, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, sigma, nullptr);
+    k_pd_primal<<<gp, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, lambda, tau);
+    mh_count_launches(2);
   }
   MH_CUDA_TRY(cudaGetLastError());
   if (energy && iterations > 0) {

@@ -140,3 +140,70 @@ def test_replayed_frame(built, psdf):
     for key in fa:
         np.testing.assert_array_equal(fa[key][ia].view(np.uint32), fb[key][ib].view(np.uint32))
     assert v.stats()["error"] == 0 and u.stats()["error"] == 0
+
+
+def _same_blocks(v, u):
+    (pa, fa), (pb, fb) = v.dump_blocks(), u.dump_blocks()
+    ia, ib = np.lexsort(pa.T), np.lexsort(pb.T)
+    np.testing.assert_array_equal(pa[ia], pb[ib])
+    np.testing.assert_array_equal(fa["sdf"][ia].view(np.uint32), fb["sdf"][ib].view(np.uint32))
+    return fa["sdf"][ia]
+
+
+def _iterate(v, iterations):
+    v._c("mh_huber_tv_iterate", 2.0, 8.0, 0.01, iterations, None, v.stream)   # no energies: nothing waits
+
+
+@pytest.mark.parametrize("iterations", [1, 3])
+def test_replayed_huber_tv(built, iterations):
+    wl = scene.full_spline(6, width=96, height=72)
+    stream = torch.cuda.Stream()
+    p = _params(wl, 0.008)
+    v = Volume(p, stream=stream.cuda_stream)
+    for k in range(6):
+        v.integrate_frame(wl.frame(k), wl.pose(k))
+    v.collect_all_blocks()
+    u = Volume(p, stream=stream.cuda_stream)
+    pos, f = v.dump_blocks()
+    u.load_blocks(pos, f["sdf"], f["w"])
+    w = f["w"]
+    seen = [f["sdf"]]
+
+    def both(call):
+        for x in (v, u):
+            call(x)
+    both(lambda x: x.set_candidates(pos))
+    both(lambda x: x.huber_tv_init())
+    g = _capture(stream, lambda: _iterate(v, iterations))
+
+    def step():
+        g.replay()
+        torch.cuda.synchronize()
+        _iterate(u, iterations)
+        seen.append(_same_blocks(v, u))
+        assert not np.array_equal(seen[-1], seen[-2])
+    step()
+    step()
+    both(lambda x: _iterate(x, 2))       # the volume's own call in between
+    step()
+    # neighbours that are no candidates any more, then with other weights
+    both(lambda x: x.set_candidates(pos[::2]))
+    step()
+    rng = np.random.default_rng(0)
+    some = np.where(rng.random(w.shape) < 0.2, 0.0, w).astype(np.float32)
+    both(lambda x: x.load_blocks(pos[1::2], None, some[1::2]))
+    step()
+    both(lambda x: x.set_candidates(pos[1::2]))
+    step()
+    # init and iterations in one graph
+    both(lambda x: x.set_candidates(pos))
+    h = _capture(stream, lambda: (v.huber_tv_init(), _iterate(v, iterations)))
+    for own in (0, 1, 2):
+        h.replay()
+        torch.cuda.synchronize()
+        u.huber_tv_init()
+        _iterate(u, iterations)
+        _same_blocks(v, u)
+        both(lambda x: _iterate(x, own))
+        _same_blocks(v, u)
+    assert v.stats()["error"] == 0 and u.stats()["error"] == 0
