@@ -334,7 +334,6 @@ __global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt,
     float so[4] = {S.x, S.y, S.z, S.w}, bo[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      bo[k] = 0.0f;
       if (!(f >> k & 1u)) continue;
       float div = 0.0f;
       if (f >> (8 + k) & 1u) {
@@ -349,8 +348,16 @@ __global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt,
       so[k] = s;
       bo[k] = 2.0f * s - prev;
     }
-    // voxels that are not usable keep their sdf; their extrapolation is not read
-    if (f) store4(d.sdf, base, so), store4(pd.bar, base, bo);
+    // voxels that are not usable keep their sdf, and their extrapolation too: a
+    // later call may find them observed again
+    if (f) store4(d.sdf, base, so);
+    if ((f & 15u) == 15u) {
+      store4(pd.bar, base, bo);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (f >> k & 1u) pd.bar[base + k] = bo[k];
+    }
     // a warp holds two layers of the block, as in the fusion kernels
     const unsigned neg = neg_bits(make_float4(so[0], so[1], so[2], so[3]));
     if ((t & 31) == 0) reinterpret_cast<uint16_t *>(d.neg + blk)[t >> 5] = (uint16_t)neg;
