@@ -212,6 +212,8 @@ int mh_batch_create(mh_volume *const *volumes, int count, int raycast, mh_batch 
   for (cudaEvent_t &e : b->sev)
     if (r == MH_OK && cudaEventCreate(&e) != cudaSuccess) r = MH_ERR_CUDA;
   if (r == MH_OK && cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking) != cudaSuccess) r = MH_ERR_CUDA;
+  if (r == MH_OK && b->raycast)
+    for (mh_volume *v : b->vols) ray_grid_ready(v);
   if (r == MH_OK) {
     mh_sm_count();
     batch_warm_occupancy();

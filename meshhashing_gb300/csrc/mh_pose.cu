@@ -284,6 +284,7 @@ static int raycast_normal_equations(mh_volume *v, const float cTw[16], const flo
   if ((r = ensure_acc(v)) != MH_OK) return r;
   if ((r = set_raycast_pose(v, cTw, s)) != MH_OK) return r;
   if (cudaMemsetAsync(v->acc, 0, sizeof(double) * 32, s) != cudaSuccess) return MH_ERR_CUDA;
+  ray_grid_ready(v);
   Dev d = v->d;
   const float *rc_wTc = v->fc_host.rc_wTc;
   if (kept && ray_grid_covers(v->hp, rc_wTc, *kept)) d.grid = *kept;

@@ -38,8 +38,10 @@ struct RayGrid {
   bool filled;               // the buffers hold this grid already
 };
 
-// A volume's buffers for its view's grid, of sizes for any view.
+// A volume's buffers for its view's grid, of sizes for any view.  They come with
+// the first raycast: up to 384 MB, of which a volume that casts no rays has no use.
 struct RayGridBuf {
+  bool reserved = false;
   unsigned *bits = nullptr, *blocks = nullptr;
   unsigned words = 0, entries = 0;
   unsigned tag = 0;    // of the last grid handed out
@@ -69,6 +71,17 @@ inline void ray_grid_sizes(const mh_params &P, RayGridBuf &b) {
   b.words = std::max((unsigned)std::min(words, (double)MH_GRID_MAX_WORDS), 4096u);
   const double entries = blocks * blocks * blocks;
   b.entries = entries <= 67108864.0 && P.value_capacity <= (1u << 24) ? (unsigned)entries : 0u;
+}
+
+// The buffers' memory, from alloc(words) (null: there is none), asked for once.
+// Without the blocks they are looked up in the hash table, without the cells every
+// sample is evaluated: the same images, later.
+template <class Alloc> inline void ray_grid_reserve(const mh_params &P, RayGridBuf &b, Alloc &&alloc) {
+  if (b.reserved) return;
+  b.reserved = true;
+  ray_grid_sizes(P, b);
+  b.bits = alloc(b.words);
+  if (b.bits && b.entries) b.blocks = alloc(b.entries);
 }
 
 // The box around a view, false for a pose that is not finite or far out.  The

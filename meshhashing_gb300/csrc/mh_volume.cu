@@ -215,8 +215,24 @@ void ray_grid_sent(mh_volume *v, const RayGrid &g, cudaStream_t s) {
   if (!mh_capturing(s)) ray_grid_enqueued(v->grid, g);
 }
 
+void ray_grid_ready(mh_volume *v) {
+  ray_grid_reserve(v->hp, v->grid, [&](unsigned words) {
+    // memory may be taken while this or another thread captures a stream
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool swapped = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    unsigned *p = nullptr;
+    if (dalloc(v, &p, words) != MH_OK) {
+      cudaGetLastError();  // the failed allocation must not surface at the next launch check
+      p = nullptr;
+    }
+    if (swapped) cudaThreadExchangeStreamCaptureMode(&mode);
+    return p;
+  });
+}
+
 // The volume's device state with the grid of the raycast pose's view.
 Dev with_ray_grid(mh_volume *v) {
+  ray_grid_ready(v);
   Dev d = v->d;
   d.grid = ray_grid_for(v->hp, v->fc_host.rc_wTc, v->grid);
   return d;
@@ -387,9 +403,6 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   A(dalloc(v, &d.page_of, cap));
   A(dalloc(v, &d.wmax, cap));
   A(dalloc(v, &d.neg, cap));
-  ray_grid_sizes(P, v->grid);
-  A(dalloc(v, &v->grid.bits, v->grid.words));
-  if (v->grid.entries) A(dalloc(v, &v->grid.blocks, v->grid.entries));
   A(dalloc(v, &v->ray_scene, 1));
   A(dalloc(v, &d.mesh_list, cap));
   A(dalloc(v, &d.cube_list, cap));
@@ -555,7 +568,10 @@ static int raycast_impl(mh_volume *v, float *depth, float *vert4, float *norm4, 
   const size_t n = (size_t)v->hp.rc_width * v->hp.rc_height;
   if (on_device) {
     StageScope sc(v, MH_STAGE_RAYCAST, s);
-    if (mh_capturing(s)) return launch_raycast_replayed(v->d, v->hp, v->grid, v->ray_scene, depth, vert4, norm4, s);
+    if (mh_capturing(s)) {
+      ray_grid_ready(v);
+      return launch_raycast_replayed(v->d, v->hp, v->grid, v->ray_scene, depth, vert4, norm4, s);
+    }
     const Dev d = with_ray_grid(v);
     TRY(launch_raycast(d, depth, vert4, norm4, s));
     ray_grid_sent(v, d.grid, s);

@@ -50,6 +50,8 @@ void inverse4(const float *m, float *out);
 bool mh_capturing(cudaStream_t s);
 // the work that clears and fills g, the volume's last grid, has been given to s
 void ray_grid_sent(mh_volume *v, const RayGrid &g, cudaStream_t s);
+// allocates the view's grid if no raycast has yet
+void ray_grid_ready(mh_volume *v);
 // the device state with the grid of the raycast pose's view (fc_host.rc_wTc)
 Dev with_ray_grid(mh_volume *v);
 // releases the Huber-TV state of a volume (mh_huber.cu)

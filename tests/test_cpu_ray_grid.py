@@ -2,7 +2,8 @@
 
 A grid asks for the block array's clear when the memory is new or its tags have
 started over.  A caller may drop a grid before anything of it is enqueued; the
-clear has to stay due until it is.
+clear has to stay due until it is.  Where a buffer cannot be allocated there is a
+grid without it, or none.
 """
 import ctypes as C
 import os
@@ -27,6 +28,17 @@ extern "C" void set_up(const mh_params *p) {
   B.bits = B.blocks = memory;  // not written here
 }
 extern "C" unsigned entries() { return B.entries; }
+// the grid of a volume of which the first `have` buffers could be allocated, the number of buffers asked for
+extern "C" int reserve(const mh_params *p, const float *wTc, int have, int *cells, int *blocks) {
+  RayGridBuf b;
+  int asked = 0;
+  for (int k = 0; k < 2; ++k)
+    ray_grid_reserve(*p, b, [&](unsigned words) { return words && asked++ < have ? memory : (unsigned *)nullptr; });
+  const RayGrid g = ray_grid_for(*p, wTc, b);
+  *cells = g.bits != nullptr;
+  *blocks = g.blocks != nullptr;
+  return asked;
+}
 extern "C" void draw(const float *wTc, int enqueue, unsigned *tag, unsigned *clear) {
   const RayGrid g = ray_grid_for(P, wTc, B);
   *tag = g.tag >> 24;
@@ -86,3 +98,13 @@ def test_a_clear_is_asked_for_once(lib):
     draws, entries = _draws(lib, [True] * 600)
     clears = [k for k, (_, clear) in enumerate(draws) if clear]
     assert clears[0] == 0 and len(clears) == 3 and all(b - a >= 250 for a, b in zip(clears, clears[1:]))
+
+
+@pytest.mark.parametrize("have,cells,blocks,asked", [(0, 0, 0, 1), (1, 1, 0, 2), (2, 1, 1, 2)])
+def test_a_grid_without_memory(lib, have, cells, blocks, asked):
+    wl = scene.full_spline(2, width=36, height=28)
+    p = config.params_for(wl, voxel_size=0.008, truncation=0.024, value_capacity=1 << 16)
+    T = np.ascontiguousarray(np.asarray(wl.pose(1), np.float32).reshape(16))
+    c, b = C.c_int(), C.c_int()
+    n = lib.reserve(C.byref(p), T.ctypes.data_as(C.c_void_p), have, C.byref(c), C.byref(b))
+    assert (c.value, b.value, n) == (cells, blocks, asked)

@@ -55,7 +55,8 @@ def _capture(stream, call):
 
 # cells of 2 voxels and of more, blocks from the dense array and (1 mm) from the hash table
 @pytest.mark.parametrize("w,h,voxel", [(124, 92, 0.008), (52, 44, 0.0047), (40, 28, 0.001), (321, 203, 0.016)])
-def test_replayed_raycast(built, w, h, voxel):
+@pytest.mark.parametrize("first", [False, True])
+def test_replayed_raycast(built, w, h, voxel, first):
     wl = scene.full_spline(6, width=w, height=h)
     stream = torch.cuda.Stream()
     v = Volume(_params(wl, voxel), stream=stream.cuda_stream)
@@ -65,7 +66,8 @@ def test_replayed_raycast(built, w, h, voxel):
     poses = [T, left_update(T, [0.1, -0.07, 0.05, 0.1, 0.2, -0.15]), left_update(T, [3.0, -2.0, 0.4, 0.0, 0.0, 2.5]),
              T @ np.diag([1.2, 0.8, 1.1, 1.0]), left_update(T, [40.0, 40.0, 0.0, 0.0, 0.0, 0.0])]
     out = Images(v)
-    v.raycast(_cTw(T))
+    if not first:                        # else the grid's memory is taken in the capture
+        v.raycast(_cTw(T))
     g = _capture(stream, lambda: v.raycast(_cTw(poses[4]), *out.t))   # a view without the map
     hits = []
     pos, f = v.dump_blocks()
