@@ -270,6 +270,11 @@ int mh_dump_flags(mh_volume *v, int max_n, uint8_t *flags, int *n_out);
  * the count of voxels whose sdf lies in [0, 1e30), counted by this call; the
  * raycast skips samples that read no other voxel. */
 int mh_dump_nonneg_counts(mh_volume *v, int n, const int32_t *pos, int32_t *count);
+/* Introspection, no reference counterpart: per block (all bits if absent) the
+ * mask that the library keeps, which the raycast and the mesh pass skip by: bit
+ * x/2 + 4 (y/2) + 16 (z/2) is set where a voxel of that 2x2x2 group may lie
+ * outside [0, 1e30), and may be set without need. */
+int mh_dump_neg_masks(mh_volume *v, int n, const int32_t *pos, uint64_t *mask);
 
 /* Per-stage GPU time, measured with CUDA events recorded on each stage's
  * stream around its launches (the reference's per-stage Timer and logging,

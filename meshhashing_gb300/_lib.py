@@ -19,6 +19,7 @@ i32p = C.POINTER(C.c_int32)
 f32p = C.POINTER(C.c_float)
 u8p = C.POINTER(C.c_uint8)
 u16p = C.POINTER(C.c_uint16)
+u64p = C.POINTER(C.c_uint64)
 i32 = C.c_int
 MHV = C.c_void_p  # opaque mh_volume*
 
@@ -56,6 +57,7 @@ SIGNATURES = {
     "mh_dump_block_meta": (i32, [MHV, i32, i32p, i32p, i32p, i32p]),
     "mh_dump_flags": (i32, [MHV, i32, u8p, i32p]),
     "mh_dump_nonneg_counts": (i32, [MHV, i32, i32p, i32p]),
+    "mh_dump_neg_masks": (i32, [MHV, i32, i32p, u64p]),
     "mh_raycast_footprint": (i32, [MHV, f32p, i32p, vp]),
     "mh_hash_bucket": (C.c_uint32, [C.c_int32, C.c_int32, C.c_int32, C.c_uint32]),
     "mh_bytes_model": (i32, [MHV, C.POINTER(C.c_double)]),

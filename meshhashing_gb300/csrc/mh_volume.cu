@@ -960,6 +960,19 @@ int mh_dump_nonneg_counts(mh_volume *v, int n, const int32_t *pos, int32_t *coun
   return MH_OK;
 }
 
+int mh_dump_neg_masks(mh_volume *v, int n, const int32_t *pos, uint64_t *mask) {
+  CHECK_VOL(v);
+  if (n < 0 || (n > 0 && (!pos || !mask))) return MH_ERR_INVALID;
+  MH_CUDA_TRY(cudaDeviceSynchronize());
+  std::vector<int> ptr;
+  TRY(find_ptrs(v, n, pos, ptr, false));
+  if (n == 0) return MH_OK;
+  std::vector<unsigned long long> all((size_t)v->d.p.value_capacity);
+  MH_CUDA_TRY(cudaMemcpy(all.data(), v->d.neg, sizeof(all[0]) * all.size(), cudaMemcpyDeviceToHost));
+  for (int i = 0; i < n; ++i) mask[i] = ptr[i] < 0 ? UINT64_MAX : all[ptr[i]];
+  return MH_OK;
+}
+
 int mh_dump_flags(mh_volume *v, int max_n, uint8_t *flags, int *n_out) {
   CHECK_VOL(v);
   MH_CUDA_TRY(cudaDeviceSynchronize());

@@ -423,10 +423,19 @@ class Volume:
         return life, inner, bnd
 
     def nonneg_counts(self, pos):
-        """Per block: the library's count of voxels with sdf in [0, 1e30)."""
+        """Per block: voxels with sdf in [0, 1e30), counted by the call."""
         pos = _i32(pos).reshape(-1, 3)
         out = np.zeros(len(pos), np.int32)
         self._c("mh_dump_nonneg_counts", len(pos), _ptr(pos, C.c_int32), _ptr(out, C.c_int32))
+        return out
+
+    def neg_masks(self, pos):
+        """Per block: the mask (uint64) that the raycast and the mesh pass skip
+        by, bit x/2 + 4 (y/2) + 16 (z/2) set where a voxel of that 2x2x2 group
+        may have its sdf outside [0, 1e30)."""
+        pos = _i32(pos).reshape(-1, 3)
+        out = np.zeros(len(pos), np.uint64)
+        self._c("mh_dump_neg_masks", len(pos), _ptr(pos, C.c_int32), _ptr(out, C.c_uint64))
         return out
 
     def flags(self):
