@@ -24,8 +24,9 @@ MH_DIV_HD float mh_div(float a, float b, float y) {
   return fmaf(fmaf(-b, q, a), y, q);
 }
 // Whether mh_div is exact for these dividends and a divisor within
-// 2^-20 .. 2^20: the residuals are multiples of 2^-48 of the dividend.  (A zero
-// takes the other way, which is right for it too.)
+// 2^-60 .. 2^60, which every length in metres is: quotients stay within
+// 2^-120 .. 2^120, and the residuals are multiples of 2^-48 of the dividend, so
+// of 2^-108.  (A zero takes the other way, which is right for it too.)
 MH_DIV_HD bool mh_div_ok(float a, float b, float c) {
   const float x = fabsf(a), y = fabsf(b), z = fabsf(c);
   return fminf(fminf(x, y), z) > 1e-18f && fmaxf(fmaxf(x, y), z) < 1e18f;
