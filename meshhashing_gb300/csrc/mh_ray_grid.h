@@ -28,6 +28,8 @@ struct RayGrid {
   int shift;                 // U = 2 << shift
   float ox, oy, oz;          // world position of the first cell's lower corner
   float inv_cell;            // 1 / (U voxel sizes)
+  float guard;               // samples' cells are taken this far (in cells) below their position
+  int reach;                 // a group of 2^3 voxels marks the cells down to that of the reach-th group below it
   // The blocks of the same box: entry (z bny + y) bnx + x holds tag | block
   // index for a block that exists, anything with another top byte otherwise.
   unsigned *blocks;          // null: blocks are looked up in the hash table
@@ -118,15 +120,27 @@ MH_GRID_HD inline bool view_box(const mh_params &P, const float wTc[16], double 
   return true;
 }
 
-// The smallest cells (U = 2, 4, ... voxels) for which a box fits the words and
-// the coordinates' rounding (4 units in the last place) stays below 1/128 cell.
+// The smallest cells (U = 2, 4, ... voxels) for which a box fits the words.
+//
+// Roundings move a sample's cell coordinate by e at most: the positions' 4 units
+// in the last place of the coordinates, and 1/128 cell in the grid's arithmetic.
+// A sample is looked up `guard` >= e below its position, so that it is never found
+// above the cell of its first corner; one that is found in cell i then has its
+// first corner below voxel U (i + 1 + guard + e) and reads one voxel more.  The
+// marks have to reach as far down: `reach` groups of two voxels, 1 near the origin
+// with cells of up to 16 voxels.  More than a cell is too far; with U = 2 more
+// than one group is, since the marks of those come from bit masks.
 MH_GRID_HD inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], const double hi[3], const RayGridBuf &b) {
   RayGrid g{};
   double far = 0.0;
   for (int a = 0; a < 3; ++a) far = std::max(far, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
   for (int shift = 0; shift < 12; ++shift) {
-    const double cell = (double)(2 << shift) * (double)P.voxel_size;
-    if (far > cell * 16384.0) continue;
+    const int U = 2 << shift;
+    const double cell = (double)U * (double)P.voxel_size;
+    const double e = far / (cell * 2097152.0) + 0.0078125, guard = e <= 0.015625 ? 0.03125 : e;
+    if (!(guard + e < 1.0)) continue;
+    const int reach = 1 + ((int)(U * (guard + e)) + 1) / 2;
+    if (reach > (1 << shift)) continue;
     int c[3];
     double n[3];  // words
     for (int a = 0; a < 3; ++a) {
@@ -141,6 +155,8 @@ MH_GRID_HD inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], co
     g.shift = shift;
     g.ox = (float)(c[0] * cell), g.oy = (float)(c[1] * cell), g.oz = (float)(c[2] * cell);
     g.inv_cell = (float)(1.0 / cell);
+    g.guard = (float)guard;
+    g.reach = reach;
     break;
   }
   // a block around the box: corners and gradient samples reach past a ray

@@ -302,19 +302,17 @@ __device__ __forceinline__ void block_interval(const DevParams &p, int bx, int b
 // A ray in the cells of the view's grid: cell = MH_GRID_BIAS + cam' + t wd'
 // in a float whose last bits are 1/256 cell, so one multiply-add gives a
 // sample's cell and the low 22 bits of the result hold it with 8 bits of
-// fraction.  Positions are shifted down by 1/32 cell: with at most 1/64 cell
-// of rounding (ray_grid_for keeps the coordinates' part below 1/128), a
-// sample found in cell i has its first corner voxel in [U i, U i + U] for
-// cells of U voxels, never below, and k_ray_grid marks cells for voxels up to
-// U i + U + 1.
+// fraction.  Positions are shifted down by the grid's guard (ray_grid_of): a
+// sample found in cell i has no corner below it, and k_ray_grid marks cell i for
+// all voxels above that the sample may read.
 struct GridRay {
   float ox, oy, oz, dx, dy, dz;
 };
 __device__ __forceinline__ GridRay grid_ray(const RayGrid &g, F3 cam, F3 wd) {
   GridRay r;
-  r.ox = (cam.x - g.ox) * g.inv_cell - 0.03125f + MH_GRID_BIAS;
-  r.oy = (cam.y - g.oy) * g.inv_cell - 0.03125f + MH_GRID_BIAS;
-  r.oz = (cam.z - g.oz) * g.inv_cell - 0.03125f + MH_GRID_BIAS;
+  r.ox = (cam.x - g.ox) * g.inv_cell - g.guard + MH_GRID_BIAS;
+  r.oy = (cam.y - g.oy) * g.inv_cell - g.guard + MH_GRID_BIAS;
+  r.oz = (cam.z - g.oz) * g.inv_cell - g.guard + MH_GRID_BIAS;
   r.dx = wd.x * g.inv_cell, r.dy = wd.y * g.inv_cell, r.dz = wd.z * g.inv_cell;
   return r;
 }
@@ -731,10 +729,10 @@ int launch_raycast_batch(const Scene *t, int n, int total, int shape, cudaStream
 }
 
 // ------------------------------------------------------------------ the view's grid
-// Cells are marked from the blocks' masks of 2^3 voxel groups.  A sample in
-// cell i of U voxels reads voxels U i .. U i + U + 1 (the march's shift and
-// rounding included, see grid_ray), so the group that starts at voxel 2 S
-// marks the 2-voxel cells S and S - 1.  A block's 64 groups give the 64 bits
+// Cells are marked from the blocks' masks of 2^3 voxel groups.  With a reach of
+// 1, a sample in cell i of U voxels reads voxels U i .. U i + U + 1 (the march's
+// shift and rounding included, see ray_grid_of), so the group that starts at voxel
+// 2 S marks the 2-voxel cells S and S - 1.  A block's 64 groups give the 64 bits
 // of its own cells and of the last layers of the seven blocks below it on each
 // axis; with U = 2 those are two words each, set with an atomic where not 0.
 // Bound by the scattered writes and atomics; 640x480, 4 mm, 461 k blocks, half
@@ -755,6 +753,26 @@ __device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
     }
     const unsigned long long m = __ldg(d.neg + i);
     if (!m) continue;
+    if (g.reach > 1) {
+      // large cells, or far from the origin: all cells from the reach below the
+      // block's first marked group to its last, on each axis; at most 27 (U = 4)
+      unsigned p = (unsigned)(m | m >> 32);
+      p = (p | p >> 16) & 0xffffu;  // x and y
+      const unsigned xs = (p | p >> 4 | p >> 8 | p >> 12) & 15u;
+      unsigned ys = p | p >> 1;
+      ys |= ys >> 2;
+      ys = (ys & 1u) | (ys >> 3 & 2u) | (ys >> 6 & 4u) | (ys >> 9 & 8u);
+      const unsigned zs = (m & 0xffffull ? 1u : 0u) | (m >> 16 & 0xffffull ? 2u : 0u) | (m >> 32 & 0xffffull ? 4u : 0u) |
+                          (m >> 48 ? 8u : 0u);
+      const int x0 = ((4 * b.x + __ffs(xs) - 1 - g.reach) >> g.shift) - g.cx, x1 = ((4 * b.x + 31 - __clz(xs)) >> g.shift) - g.cx;
+      const int y0 = ((4 * b.y + __ffs(ys) - 1 - g.reach) >> g.shift) - g.cy, y1 = ((4 * b.y + 31 - __clz(ys)) >> g.shift) - g.cy;
+      const int z0 = ((4 * b.z + __ffs(zs) - 1 - g.reach) >> g.shift) - g.cz, z1 = ((4 * b.z + 31 - __clz(zs)) >> g.shift) - g.cz;
+      for (int z = max(z0, 0); z <= min(z1, 2 * nz - 1); ++z)
+        for (int y = max(y0, 0); y <= min(y1, 4 * ny - 1); ++y)
+          for (int x = max(x0, 0); x <= min(x1, 4 * nx - 1); ++x)
+            atomicOr(g.bits + ((size_t)(z >> 1) * ny + (y >> 2)) * nx + (x >> 2), 1u << ((x & 3) | (y & 3) << 2 | (z & 1) << 4));
+      continue;
+    }
 #pragma unroll 1
     for (int j = 0; j < 8; ++j) {
       // block b - j: along an axis of j, group 0 marks cell 3 of the block
