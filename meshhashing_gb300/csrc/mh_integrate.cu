@@ -14,6 +14,7 @@
 #include "mh_batch.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace {
 
@@ -142,10 +143,17 @@ __global__ void __launch_bounds__(128) k_integrate_simple_b(const Scene *t, int 
              [&](const Scene &c, Share sh) { integrate_simple_body(c.d, sh); });
 }
 
-// What the PSDF update needs of a pixel, once per pixel instead of once per
-// voxel that projects onto it: depth (-inf if invalid), inlier ratio, the
-// measurement's variance and the outlier density (update_bayesian.cu:123-156).
-// Half a warp takes a tile of 4x4 pixels and keeps the depth up to which the
+// What the PSDF update needs of a pixel: depth (-inf if invalid), inlier ratio r,
+// the measurement's variance and the outlier density (update_bayesian.cu:123-156).
+__device__ __forceinline__ float4 pixel_record(const DevParams &p, float depth, float r) {
+  const float tau = (depth - 0.4f) * 0.012f + 0.019f;
+  const bool in_range = depth < p.max_depth_range && depth >= p.min_depth_range;
+  const float out = p.compat ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : (1.0f - r) * 0.204081632653061224f;
+  return make_float4(depth_invalid(p, depth) ? -__int_as_float(0x7f800000) : depth, r, tau * tau, in_range ? out : 1.0f);
+}
+
+// The pixels' records, once per pixel instead of once per voxel that projects onto
+// it.  Half a warp takes a tile of 4x4 pixels and keeps the depth up to which the
 // tile updates voxels, as the bits of a float that is not negative.
 __device__ __forceinline__ void pixels_body(const Dev &d, Share sh) {
   const DevParams &p = d.p;
@@ -157,14 +165,10 @@ __device__ __forceinline__ void pixels_body(const Dev &d, Share sh) {
     unsigned far = 0u;
     if (i < n && x < p.width && y < p.height) {
       const size_t pix = (size_t)y * p.width + x;
-      const float dd = d.depth[pix], r = d.inlier[pix];
-      const float tau = (dd - 0.4f) * 0.012f + 0.019f;
-      const bool in_range = dd < p.max_depth_range && dd >= p.min_depth_range;
-      const float out = p.compat ? (1.0f - r) * 1.0f / (5.0f - 0.1f) : (1.0f - r) * 0.204081632653061224f;
-      const bool invalid = depth_invalid(p, dd);
-      d.pixels[pix] = make_float4(invalid ? -__int_as_float(0x7f800000) : dd, r, tau * tau, in_range ? out : 1.0f);
+      const float dd = d.depth[pix];
+      d.pixels[pix] = pixel_record(p, dd, d.inlier[pix]);
       const float f = dd + truncate_dist(p, dd);
-      if (!invalid) far = f <= 0.0f ? 0u : f < 1e30f ? __float_as_uint(f) : 0x7f800000u;  // NaN: no limit
+      if (!depth_invalid(p, dd)) far = f <= 0.0f ? 0u : f < 1e30f ? __float_as_uint(f) : 0x7f800000u;  // NaN: no limit
     }
     far = __reduce_max_sync(lane_id() < 16 ? 0xffffu : 0xffff0000u, far);
     if (j == 0 && i < n) d.tile_far[i] = far;
@@ -254,18 +258,24 @@ __global__ void __launch_bounds__(256) k_upd_select_b(const Scene *t, int n) {
 // the update is division- and transcendental-bound, not load-bound, so the
 // default form restates it with 4 IEEE divisions (see below); compat mode
 // evaluates the reference's expressions as written.
-__device__ __forceinline__ void integrate_psdf_body(const Dev &d, Share sh) {
+//
+// kPlanned: over the selected candidates and the pixels' records.  Without, over
+// all candidates, with the records made per voxel: where the two passes before
+// cost more than they save (psdf_update_direct).
+template <bool kPlanned> __device__ __forceinline__ void integrate_psdf_body(const Dev &d, Share sh) {
   __shared__ float cTw[16];
   if (threadIdx.x < 16) cTw[threadIdx.x] = d.fc->cTw[threadIdx.x];
   __syncthreads();
   const DevParams &p = d.p;
-  const int n = *reinterpret_cast<volatile int *>(&d.ctr->upd_count);
+  const int n = *reinterpret_cast<volatile int *>(kPlanned ? &d.ctr->upd_count : &d.ctr->cand_count);
+  const int4 *list = kPlanned ? d.upd_list : d.cand;
   const int t = threadIdx.x;
   const int lx = (t & 1) * 4, ly = (t >> 1) & 7, lz = t >> 4;
-  int4 next = sh.first < n ? d.upd_list[sh.first] : make_int4(0, 0, 0, -1);
+  int4 next = sh.first < n ? list[sh.first] : make_int4(0, 0, 0, -1);
   for (int c = sh.first; c < n; c += sh.stride) {
     const int4 cb = next;
-    if (c + sh.stride < n) next = d.upd_list[c + sh.stride];
+    if (c + sh.stride < n) next = list[c + sh.stride];
+    if (!kPlanned && cb.w < 0) continue;
     const int vx0 = cb.x * MH_BLOCK_SIDE + lx, vy = cb.y * MH_BLOCK_SIDE + ly, vz = cb.z * MH_BLOCK_SIDE + lz;
     const float fx0 = (float)vx0, fy = (float)vy, fz = (float)vz;
     float xs[4], rs[4], ts[4], cs[4];
@@ -276,7 +286,7 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d, Share sh) {
       const int pix = pixel_of(p, cam);
       act[k] = false;
       if (pix < 0) continue;
-      const float4 px = __ldg(d.pixels + pix);
+      const float4 px = kPlanned ? __ldg(d.pixels + pix) : pixel_record(p, __ldg(d.depth + pix), __ldg(d.inlier + pix));
       const float x = px.x - cam.z;
       const float tr = truncate_dist(p, px.x);
       if (px.x == -__int_as_float(0x7f800000) || x <= -tr) continue;
@@ -375,10 +385,11 @@ __device__ __forceinline__ void integrate_psdf_body(const Dev &d, Share sh) {
     note_neg(d, cb.w, S);
   }
 }
-__global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body(d, whole_grid()); }
+template <bool kPlanned>
+__global__ void __launch_bounds__(128, 8) k_integrate_psdf(Dev d) { integrate_psdf_body<kPlanned>(d, whole_grid()); }
 __global__ void __launch_bounds__(128, 8) k_integrate_psdf_b(const Scene *t, int n) {
   each_scene(t, n, 1, [&](const Scene &c) { return c.d.p.enable_bayesian ? count_of(c.d, &Counters::upd_count) : 0; },
-             [&](const Scene &c, Share sh) { integrate_psdf_body(c.d, sh); });
+             [&](const Scene &c, Share sh) { integrate_psdf_body<true>(c.d, sh); });
 }
 
 // PredictOutlierRatioKernel (mapping/update_bayesian.cu:36-101).  The
@@ -495,6 +506,22 @@ __global__ void k_preprocess_b(const Scene *t, int n) {
              [&](const Scene &c, Share sh) { preprocess_body(c.d, sh, c.src, nullptr, 0.0f); });
 }
 
+// Whether the PSDF update goes over all candidates and makes the pixels' records
+// per voxel.  The two passes before the other form cost 8 us, and 20 with 640x480
+// pixels; they save about a seventh of the update, which grows with the candidates:
+// with the pixels, up to the blocks that fit the view.  The forms are even, us
+// without / with the passes, at 64x48, 4 mm (88 / 88); 160x120, 8 mm (68 / 69);
+// 240x180, 10 mm (82 / 81); 320x240, 12 mm (80 / 80): 40 pixels for each cubic
+// millimetre of a voxel; and at 12 mm for larger images (640x480: 110 / 111), where
+// 32 k blocks fit the view.  On one side: 32x24, 20 mm: 10 / 17; 160x120, 16 mm: 31 /
+// 37; 640x480, 16 mm: 49 / 67; 640x480, 30 mm: 14 / 43; on the other: 160x120, 4 mm:
+// 166 / 155; 640x480, 10 mm: 166 / 160; 640x480, 4 mm: 884 / 771.
+bool psdf_update_direct(const mh_params &P) {
+  const double v = P.voxel_size, z0 = P.min_depth_range, z1 = P.max_depth_range;
+  const double view = std::fabs(P.width / (double)P.fx * (P.height / (double)P.fy)) * (z1 * z1 * z1 - z0 * z0 * z0) / 3.0;
+  return (double)P.width * P.height <= 4e10 * v * v * v || view <= 32768.0 * 512.0 * v * v * v;
+}
+
 static int grid_persistent(int per_sm) { return mh_sm_count() * per_sm; }
 
 int launch_integrate_simple(const Dev &d, cudaStream_t s) {
@@ -503,9 +530,14 @@ int launch_integrate_simple(const Dev &d, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
 int launch_integrate_psdf(const Dev &d, cudaStream_t s) {
+  if (d.p.psdf_direct) {
+    k_integrate_psdf<false><<<mh_resident_grid((const void *)k_integrate_psdf<false>, 128, 16), 128, 0, s>>>(d);
+    mh_count_launches(1);
+    return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
+  }
   k_pixels<<<std::min((far_tiles_x(d.p) * far_tiles_y(d.p) + 15) / 16, mh_sm_count() * 8), 256, 0, s>>>(d);
   k_upd_select<<<mh_sm_count() * 4, 256, 0, s>>>(d);
-  k_integrate_psdf<<<mh_resident_grid((const void *)k_integrate_psdf, 128, 16), 128, 0, s>>>(d);
+  k_integrate_psdf<true><<<mh_resident_grid((const void *)k_integrate_psdf<true>, 128, 16), 128, 0, s>>>(d);
   mh_count_launches(3);
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }

@@ -98,6 +98,7 @@ struct DevParams {
   float min_raycast_depth, max_raycast_depth, raycast_step, sample_sdf_threshold, sdf_threshold;
   int enable_gradients, enable_bayesian;
   int compat;  // evaluate the reference's formulas as written
+  int psdf_direct;  // the PSDF update takes all candidates in one pass
 };
 
 // Everything a kernel needs, passed by value (pointers + params).

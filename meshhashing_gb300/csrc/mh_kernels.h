@@ -15,6 +15,7 @@ int launch_set_candidates(const Dev &d, const int *pos_dev, const int *ptr_dev, 
 int launch_preprocess(const Dev &d, const float *src, const uint16_t *src16, float range_factor, cudaStream_t s);
 int launch_integrate_simple(const Dev &d, cudaStream_t s);
 int launch_integrate_psdf(const Dev &d, cudaStream_t s);
+bool psdf_update_direct(const mh_params &P);
 int launch_predict_inlier(const Dev &d, cudaStream_t s);
 
 int launch_mesh(const Dev &d, cudaStream_t s);

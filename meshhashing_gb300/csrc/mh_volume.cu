@@ -377,6 +377,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   q.sample_sdf_threshold = P.sample_sdf_threshold, q.sdf_threshold = P.sdf_threshold;
   q.enable_gradients = P.enable_gradients, q.enable_bayesian = P.enable_bayesian_update;
   q.compat = P.compat_arithmetic != 0;
+  q.psdf_direct = psdf_update_direct(P);
 
   const size_t cap = P.value_capacity, nv = cap * MH_BLOCK_VOXELS, npix = (size_t)P.width * P.height;
   const size_t rpix = (size_t)P.rc_width * P.rc_height;
