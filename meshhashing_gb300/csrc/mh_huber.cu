@@ -43,7 +43,7 @@ __device__ __forceinline__ int cand_count(const Dev &d) { return *reinterpret_ca
 // the pool index of the block next to candidate c along axis k, direction
 // s (-1 when absent).  One lookup per thread, so the table costs one pass of
 // independent hash probes instead of a serial probe per block and pass.
-__global__ void __launch_bounds__(256) k_pd_faces(Dev d, int *nbt) {
+__device__ __forceinline__ void find_faces(const Dev &d, int *nbt) {
   const int n = cand_count(d);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 6 * n; t += gridDim.x * blockDim.x) {
     const int c = t / 6, j = t - 6 * c;
@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(256) k_pd_faces(Dev d, int *nbt) {
     nbt[t] = q;
   }
 }
+__global__ void __launch_bounds__(256) k_pd_faces(Dev d, int *nbt) { find_faces(d, nbt); }
 
 // neighbour usable by the masked queries: block exists, voxel observed, mask set
 __device__ __forceinline__ bool usable(const Dev &d, const PD &pd, long long g) {
@@ -69,12 +70,18 @@ __device__ __forceinline__ int first_voxel(int t) { return t * 4; }
 
 // The voxels of a block that the masked queries may use, a byte for each row of
 // 8 voxels along x; `known` (cleared before) tells that the block's bytes are of
-// this call.
-__global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, uint8_t *known) {
+// this call, `active` whether the candidate has such a voxel at all.  The face
+// table is made here too: a launch less in calls of few blocks.
+__global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, int *nbt, uint8_t *use, uint8_t *known,
+                                                   uint8_t *active) {
+  find_faces(d, nbt);
   const int n = cand_count(d), t = threadIdx.x;
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int blk = d.cand[c].w;
-    if (blk < 0) continue;
+    if (blk < 0) {
+      if (t == 0) active[c] = 0;
+      continue;
+    }
     const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
     const float4 w = *reinterpret_cast<const float4 *>(d.w + base);
     const uint4 m = *reinterpret_cast<const uint4 *>(pd.mask + base);
@@ -85,7 +92,60 @@ __global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, u
     if (w.w >= kEps && m.w == pd.epoch) f |= 8u;
     const unsigned hi = __shfl_down_sync(0xffffffffu, f, 1);
     if (!(t & 1)) use[(size_t)blk * 64 + t / 2] = (uint8_t)(f | hi << 4);
-    if (t == 0) known[blk] = 1;
+    const int any = __syncthreads_or(f != 0u);
+    if (t == 0) known[blk] = 1, active[c] = any ? 1 : 0;
+  }
+}
+
+// What a thread needs to know of a candidate before it can load its part of it: the
+// pool block, the voxels' flags and the blocks of the face voxels that it brings in
+// (two of 192 at most; side: the faces' place in the table).
+struct Visit {
+  int c, blk, q[2];
+  unsigned f;
+  __device__ __forceinline__ void load(const Dev &d, const int *nbt, const uint16_t *flags, int side, int cand) {
+    c = cand;
+    if (c < 0) return;
+    const int t = threadIdx.x;
+    blk = d.cand[c].w;
+    f = flags[(size_t)c * 128 + t];
+    q[0] = __ldg(nbt + 6 * c + 2 * (t >> 6) + side);
+    q[1] = t < 64 ? __ldg(nbt + 6 * c + 4 + side) : -1;
+  }
+};
+// Runs visit(Visit) for the active ones of this CTA's candidates, with all 128
+// threads.  Their bytes are read 128 at a time, so the others cost next to nothing,
+// and the next one's Visit is loaded while the last one is worked on.  (With 200 of
+// 49 k candidates initialised, ten iterations take 0.22 ms; with the flags of each
+// candidate read in each pass they took 0.39.)
+template <class F>
+__device__ __forceinline__ void each_active(const Dev &d, const int *nbt, const uint8_t *active, const uint16_t *flags,
+                                            int side, F &&visit) {
+  __shared__ unsigned bits[4];
+  const int n = cand_count(d);
+  for (int first = blockIdx.x; first < n; first += 128 * gridDim.x) {
+    const int c = first + threadIdx.x * gridDim.x;
+    const unsigned b = __ballot_sync(0xffffffffu, c < n && active[c]);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) bits[threadIdx.x >> 5] = b;
+    __syncthreads();
+    int w = 0;
+    unsigned left = bits[0];
+    auto next = [&]() {
+      while (!left && w < 3) left = bits[++w];
+      if (!left) return -1;
+      const int k = 32 * w + __ffs(left) - 1;
+      left &= left - 1u;
+      return first + k * (int)gridDim.x;
+    };
+    Visit v;
+    v.load(d, nbt, flags, side, next());
+    while (v.c >= 0) {
+      Visit after;
+      after.load(d, nbt, flags, side, next());
+      visit(v);
+      v = after;
+    }
   }
 }
 
@@ -96,15 +156,12 @@ __global__ void __launch_bounds__(128) k_pd_usable(Dev d, PD pd, uint8_t *use, u
 // reading weights and masks of the faces' voxels, a 32-byte sector each along
 // x, took 250 us for 120 k blocks against 134 us for both passes.
 __global__ void __launch_bounds__(128) k_pd_flags(Dev d, PD pd, const int *nbt, const uint8_t *use,
-                                                  const uint8_t *known, uint16_t *flags) {
+                                                  const uint8_t *known, const uint8_t *active, uint16_t *flags) {
   const int n = cand_count(d), row = threadIdx.x & 63, y = row & 7, z = row >> 3;
   for (int c = blockIdx.x * 2 + (threadIdx.x >> 6); c < n; c += gridDim.x * 2) {
+    if (!active[c]) continue;
     const int blk = d.cand[c].w;
     unsigned *out = reinterpret_cast<unsigned *>(flags) + (size_t)c * 64 + row;
-    if (blk < 0) {
-      *out = 0u;
-      continue;
-    }
     // row r of the neighbour `face`, the voxels `want` of it
     auto beyond = [&](int face, int r, unsigned want) -> unsigned {
       const int q = __ldg(nbt + 6 * c + face);
@@ -147,6 +204,13 @@ __device__ __forceinline__ void tile_own(Tile9 &s, int t, int off, const float4 
   float *o = s.v + (i & 7) + off + 9 * (((i >> 3) & 7) + off) + 81 * ((i >> 6) + off);
   o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
 }
+// Whether the voxel of the block that faces voxel i of the neighbour's face needs
+// it: the flags (16 bits a thread) of the block's last layer (up) or its first.
+__device__ __forceinline__ bool face_needed(const uint16_t *flags, int i, int k, bool up) {
+  const int a = i & 7, b = i >> 3, in = up ? 7 : 0;
+  const int li = k == 0 ? in + 8 * a + 64 * b : k == 1 ? a + 8 * in + 64 * b : a + 8 * b + 64 * in;
+  return flags[li >> 2] >> ((up ? 4 : 8) + (li & 3)) & 1u;
+}
 // 64 voxels of a neighbour's face of axis k: its first layer (up) or its last
 __device__ __forceinline__ void tile_face(Tile9 &s, int i, int k, bool up, int q, const float *field) {
   if (q < 0) return;  // no voxel here has the neighbour: the flags say so
@@ -188,8 +252,8 @@ __device__ __forceinline__ float pd_huber(float n2) {
 }
 
 // PrimalDualInit: weights from the gradient, the iterate's start.  Bound by the
-// traffic, 36 B a voxel and the faces: 480 us for 120 k blocks.  A thread a voxel
-// took 508 us; without the operators' long ways this form takes 479.
+// traffic, 36 B a voxel and the faces: 480 us for 120 k blocks, where a thread a
+// voxel took 508.
 __global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt, unsigned *fresh) {
   __shared__ Tile9 sdf, weight;
   const int n = cand_count(d), t = threadIdx.x;
@@ -236,36 +300,47 @@ __global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt, u
 }
 
 // Dual step (PrimalDualIteratePass1Kernel), with the energies where they are
-// asked for.  Bound by the traffic: 28 B a voxel (the extrapolated sdf and the
-// dual read, the dual written; 8 more for the energies) and the faces: 390 us
-// for 120 k blocks.  One thread per entry of
-// a list of usable voxels took 660 us and read 12 B more a voxel; with the
-// operator's divisions this form takes 700 us.  After an init, before the first
+// asked for.  28 B a voxel (the extrapolated sdf and the dual read, the dual
+// written; 8 more for the energies) and the faces; bound by the latency of a block's
+// loads, so ten CTAs an SM (48 registers): 361 us for 120 k blocks, 1.45 GB, against
+// 390 us with the registers that the compiler takes.  One thread per entry of a list
+// of usable voxels took 660 us and read 12 B more a voxel; with the operators'
+// divisions this form takes 700 us.  In blocks with few usable voxels the list was
+// better: with 35 of 512 in each of 7 k blocks ten iterations take 0.42 ms, and took
+// 0.25 ms.  After an init, before the first
 // primal step (fresh), the extrapolated sdf is 0 and so is the new dual: there is
 // nothing to do.  The device knows that, since graphs may replay the calls.
 template <bool kEnergy>
-__global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, const uint16_t *flags,
-                                                 const unsigned *fresh, float sigma, double *err) {
+__global__ void __launch_bounds__(128, 10) k_pd_dual(Dev d, PD pd, const int *nbt, const uint8_t *active,
+                                                     const uint16_t *flags, const unsigned *fresh, float sigma,
+                                                     double *err) {
   __shared__ Tile9 bar, sdf;
-  const int n = cand_count(d), t = threadIdx.x;
+  __shared__ uint16_t block_flags[128];
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int t = threadIdx.x;
   const float h = 1.0f + sigma * kAlpha, rh = 1.0f / h;
   const bool h_ok = h > 0x1p-20f && h < 0x1p20f;
   if (!kEnergy && h_ok && *fresh == pd.epoch) return;
   float e[2] = {0.0f, 0.0f};
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
-    const unsigned f = flags[(size_t)c * 128 + t];
-    if (!__syncthreads_or(f)) continue;
-    const int blk = d.cand[c].w;
-    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
-    const float4 B = load4(pd.bar, base), X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
-    float4 S, S0;
-    if (kEnergy) S = load4(d.sdf, base), S0 = load4(pd.sdf0, base);
+  each_active(d, nbt, active, flags, 0, [&](const Visit &v) {
+    const unsigned f = v.f;
+    block_flags[t] = (uint16_t)f;
+    __syncthreads();
+    const size_t base = (size_t)v.blk * MH_BLOCK_VOXELS + first_voxel(t);
+    // a thread without a usable voxel needs none of its own, nor does a neighbour
+    float4 B = none, X = none, Y = none, Z = none, S = none, S0 = none;
+    if (f) {
+      B = load4(pd.bar, base), X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
+      if (kEnergy) S = load4(d.sdf, base), S0 = load4(pd.sdf0, base);
+    }
     tile_own(bar, t, 0, B);
     if (kEnergy) tile_own(sdf, t, 0, S);
-    for (int i = t; i < 192; i += 128) {
-      const int k = i >> 6, q = __ldg(nbt + 6 * c + 2 * k);
-      tile_face(bar, i & 63, k, true, q, pd.bar);
-      if (kEnergy) tile_face(sdf, i & 63, k, true, q, d.sdf);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int i = t + 128 * m, k = i >> 6;
+      if (i >= 192 || !face_needed(block_flags, i & 63, k, true)) continue;
+      tile_face(bar, i & 63, k, true, v.q[m], pd.bar);
+      if (kEnergy) tile_face(sdf, i & 63, k, true, v.q[m], d.sdf);
     }
     __syncthreads();
     const int i0 = first_voxel(t), o0 = (i0 & 7) + 9 * ((i0 >> 3) & 7) + 81 * (i0 >> 6);
@@ -302,32 +377,41 @@ __global__ void __launch_bounds__(128) k_pd_dual(Dev d, PD pd, const int *nbt, c
     }
     if (f) store4(pd.px, base, px), store4(pd.py, base, py), store4(pd.pz, base, pz);
     __syncthreads();
-  }
+  });
   if (kEnergy) cta_sum<2>(e, err);
 }
 
 // Primal step and extrapolation (PrimalDualIteratePass2Kernel).  Bound by the
 // traffic: 32 B a voxel (the dual, sdf, sdf0 and the weight read, sdf and its
-// extrapolation written) and the faces: 382 us for 120 k blocks, 5.1 TB/s
-// without the faces.
-__global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt, const uint16_t *flags,
-                                                   unsigned *fresh, float lambda, float tau) {
+// extrapolation written) and the faces: 309 us for 120 k blocks, 1.84 GB at 6.0 TB/s;
+// 382 us without the limit to 48 registers.
+__global__ void __launch_bounds__(128, 10) k_pd_primal(Dev d, PD pd, const int *nbt, const uint8_t *active,
+                                                       const uint16_t *flags, unsigned *fresh, float lambda,
+                                                       float tau) {
   __shared__ Tile9 tx, ty, tz;
-  const int n = cand_count(d), t = threadIdx.x;
+  __shared__ uint16_t block_flags[128];
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int t = threadIdx.x;
   if (blockIdx.x == 0 && t == 0) *fresh = 0u;
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
-    const unsigned f = flags[(size_t)c * 128 + t];
-    if (!__syncthreads_or(f)) continue;
-    const int blk = d.cand[c].w;
-    const size_t base = (size_t)blk * MH_BLOCK_VOXELS + first_voxel(t);
-    const float4 X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
-    const float4 S = load4(d.sdf, base), S0 = load4(pd.sdf0, base), Wt = load4(pd.w, base);
+  each_active(d, nbt, active, flags, 1, [&](const Visit &v) {
+    const unsigned f = v.f;
+    block_flags[t] = (uint16_t)f;
+    __syncthreads();
+    const size_t base = (size_t)v.blk * MH_BLOCK_VOXELS + first_voxel(t);
+    const float4 S = load4(d.sdf, base);  // all of it, for the block's mask
+    float4 X = none, Y = none, Z = none, S0 = none, Wt = none;
+    if (f) {
+      X = load4(pd.px, base), Y = load4(pd.py, base), Z = load4(pd.pz, base);
+      S0 = load4(pd.sdf0, base), Wt = load4(pd.w, base);
+    }
     tile_own(tx, t, 1, X), tile_own(ty, t, 1, Y), tile_own(tz, t, 1, Z);
-    for (int i = t; i < 192; i += 128) {
-      const int k = i >> 6, q = __ldg(nbt + 6 * c + 2 * k + 1);
-      if (k == 0) tile_face(tx, i & 63, 0, false, q, pd.px);
-      else if (k == 1) tile_face(ty, i & 63, 1, false, q, pd.py);
-      else tile_face(tz, i & 63, 2, false, q, pd.pz);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int i = t + 128 * m, k = i >> 6;
+      if (i >= 192 || !face_needed(block_flags, i & 63, k, false)) continue;
+      if (k == 0) tile_face(tx, i & 63, 0, false, v.q[m], pd.px);
+      else if (k == 1) tile_face(ty, i & 63, 1, false, v.q[m], pd.py);
+      else tile_face(tz, i & 63, 2, false, v.q[m], pd.pz);
     }
     __syncthreads();
     const int i0 = first_voxel(t), o0 = (i0 & 7) + 1 + 9 * (((i0 >> 3) & 7) + 1) + 81 * ((i0 >> 6) + 1);
@@ -360,9 +444,9 @@ __global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt,
     }
     // a warp holds two layers of the block, as in the fusion kernels
     const unsigned neg = neg_bits(make_float4(so[0], so[1], so[2], so[3]));
-    if ((t & 31) == 0) reinterpret_cast<uint16_t *>(d.neg + blk)[t >> 5] = (uint16_t)neg;
+    if ((t & 31) == 0) reinterpret_cast<uint16_t *>(d.neg + v.blk)[t >> 5] = (uint16_t)neg;
     __syncthreads();
-  }
+  });
 }
 
 }  // namespace
@@ -370,11 +454,12 @@ __global__ void __launch_bounds__(128) k_pd_primal(Dev d, PD pd, const int *nbt,
 struct mh_pd_state {
   PD pd;
   size_t voxels = 0;
-  double *err = nullptr;
+  double *err = nullptr;      // the energies, and after them `known`: cleared together
   int *nbt = nullptr;   // face-neighbour table of the candidate list (6 per candidate)
   uint16_t *flags = nullptr;  // per-voxel flags of the call (128 words per candidate)
   uint8_t *use = nullptr;     // usable voxels, 64 bytes per pool block
   uint8_t *known = nullptr;   // blocks whose bytes this call wrote
+  uint8_t *active = nullptr;  // candidates with a usable voxel
   unsigned *fresh = nullptr;  // epoch of an init that no primal step has followed: bar and p are 0
 };
 
@@ -389,11 +474,12 @@ static int pd_ensure(mh_volume *v) {
   bool ok = true;
   for (float **p : f) ok = ok && cudaMalloc((void **)p, sizeof(float) * nv) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->pd.mask, sizeof(unsigned) * nv) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&st->err, sizeof(double) * 2) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->err, sizeof(double) * 2 + (size_t)v->hp.value_capacity) == cudaSuccess;
+  st->known = reinterpret_cast<uint8_t *>(st->err + 2);
   ok = ok && cudaMalloc((void **)&st->nbt, sizeof(int) * 6 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->flags, sizeof(uint16_t) * 128 * (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->use, 64 * (size_t)v->hp.value_capacity) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&st->known, (size_t)v->hp.value_capacity) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&st->active, (size_t)v->hp.value_capacity) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&st->fresh, sizeof(unsigned)) == cudaSuccess;
   ok = ok && cudaMemset(st->pd.mask, 0, sizeof(unsigned) * nv) == cudaSuccess;
   st->pd.epoch = 0;
@@ -412,7 +498,7 @@ void mh_pd_free(mh_volume *v) {
   if (!st) return;
   for (void *p : {(void *)st->pd.sdf0, (void *)st->pd.bar, (void *)st->pd.w, (void *)st->pd.px, (void *)st->pd.py,
                   (void *)st->pd.pz, (void *)st->pd.mask, (void *)st->err, (void *)st->nbt,
-                  (void *)st->flags, (void *)st->use, (void *)st->known, (void *)st->fresh})
+                  (void *)st->flags, (void *)st->use, (void *)st->active, (void *)st->fresh})
     if (p) cudaFree(p);
   delete st;
   v->pd = nullptr;
@@ -443,23 +529,22 @@ int mh_huber_tv_iterate(mh_volume *v, float lambda, float sigma, float tau, int 
   if (iterations > 0) {
     // the candidate list may have changed since init: rebuild the face table
     // and the flags of this call (neither pass changes w or the mask)
-    k_pd_faces<<<grid_of((const void *)k_pd_faces), 256, 0, s>>>(v->d, st->nbt);
-    MH_CUDA_TRY(cudaMemsetAsync(st->known, 0, (size_t)v->hp.value_capacity, s));
-    k_pd_usable<<<grid_of((const void *)k_pd_usable, 128), 128, 0, s>>>(v->d, st->pd, st->use, st->known);
+    MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2 + (size_t)v->hp.value_capacity, s));
+    k_pd_usable<<<grid_of((const void *)k_pd_usable, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->use, st->known,
+                                                                       st->active);
     k_pd_flags<<<grid_of((const void *)k_pd_flags, 128), 128, 0, s>>>(v->d, st->pd, st->nbt, st->use, st->known,
-                                                                     st->flags);
-    MH_CUDA_TRY(cudaMemsetAsync(st->err, 0, sizeof(double) * 2, s));
-    mh_count_launches(3);
+                                                                     st->active, st->flags);
+    mh_count_launches(2);
   }
   const int gd = grid_of((const void *)k_pd_dual<false>, 128), ge = grid_of((const void *)k_pd_dual<true>, 128),
             gp = grid_of((const void *)k_pd_primal, 128);
   for (int it = 0; it < iterations; ++it) {
     // only the last pass's energies are returned
     if (it + 1 == iterations)
-      k_pd_dual<true><<<ge, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, sigma, st->err);
+      k_pd_dual<true><<<ge, 128, 0, s>>>(v->d, st->pd, st->nbt, st->active, st->flags, st->fresh, sigma, st->err);
     else
-      k_pd_dual<false><<<gd, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, sigma, nullptr);
-    k_pd_primal<<<gp, 128, 0, s>>>(v->d, st->pd, st->nbt, st->flags, st->fresh, lambda, tau);
+      k_pd_dual<false><<<gd, 128, 0, s>>>(v->d, st->pd, st->nbt, st->active, st->flags, st->fresh, sigma, nullptr);
+    k_pd_primal<<<gp, 128, 0, s>>>(v->d, st->pd, st->nbt, st->active, st->flags, st->fresh, lambda, tau);
     mh_count_launches(2);
   }
   MH_CUDA_TRY(cudaGetLastError());

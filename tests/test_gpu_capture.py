@@ -179,6 +179,7 @@ def test_replayed_huber_tv(built, iterations):
     g = _capture(stream, lambda: _iterate(v, iterations))
 
     def step():
+        torch.cuda.synchronize()         # the replay is on another stream
         g.replay()
         torch.cuda.synchronize()
         _iterate(u, iterations)
