@@ -453,7 +453,6 @@ __global__ void __launch_bounds__(128, 10) k_pd_primal(Dev d, PD pd, const int *
 
 struct mh_pd_state {
   PD pd;
-  size_t voxels = 0;
   double *err = nullptr;      // the energies, and after them `known`: cleared together
   int *nbt = nullptr;   // face-neighbour table of the candidate list (6 per candidate)
   uint16_t *flags = nullptr;  // per-voxel flags of the call (128 words per candidate)
@@ -467,6 +466,7 @@ static int grid_of(const void *fn, int block = 256) { return mh_resident_grid(fn
 
 static int pd_ensure(mh_volume *v) {
   if (v->pd) return MH_OK;
+  // 120 GB of state beside 69 GB of voxels
   if (v->hp.value_capacity > (1u << 23)) return MH_ERR_INVALID;
   mh_pd_state *st = new mh_pd_state();
   const size_t nv = (size_t)v->hp.value_capacity * MH_BLOCK_VOXELS;
@@ -483,7 +483,6 @@ static int pd_ensure(mh_volume *v) {
   ok = ok && cudaMalloc((void **)&st->fresh, sizeof(unsigned)) == cudaSuccess;
   ok = ok && cudaMemset(st->pd.mask, 0, sizeof(unsigned) * nv) == cudaSuccess;
   st->pd.epoch = 0;
-  st->voxels = nv;
   v->pd = st;
   if (!ok) {
     cudaGetLastError();  // the failed allocation must not surface at the next launch check

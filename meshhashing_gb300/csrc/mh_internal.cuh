@@ -65,7 +65,6 @@ struct Counters {
   int cube_list_count; // candidates the cube pass must tile this pass
   int vtx_list_count;  // candidates owning vertices (inlier prediction)
   int upd_count;       // candidates that the PSDF update may change
-  int ray_next;        // next ray handed out by the raycast
   unsigned long long cand_sum;   // sum of candidate counts over mesh calls
   unsigned long long vwork_sum;  // sum of computed vertices over mesh calls
   unsigned long long cube_blocks_sum;     // blocks the cube pass loaded a tile for
@@ -355,47 +354,45 @@ __device__ __forceinline__ void corner_pair(float p, float off, float vs, float 
 
 // Corner voxels of GetSpatialValue at pos (both of each axis) and the
 // position's fractions.
-struct SampleAt {
+struct Corners {
   int v0x, v0y, v0z, v1x, v1y, v1z;
   float rx, ry, rz;
 };
-__device__ __forceinline__ SampleAt sample_at(const DevParams &p, F3 pos) {
-  SampleAt k;
+__device__ __forceinline__ Corners corners_at(const DevParams &p, F3 pos) {
+  Corners k;
+  const float vs = p.voxel_size;
   const F3 q = in_voxels(p, pos);
   const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
   k.rx = q.x - fx, k.ry = q.y - fy, k.rz = q.z - fz;
-  corner_pair(pos.x, p.voxel_size, p.voxel_size, q.x, fx, k.rx, k.v0x, k.v1x);
-  corner_pair(pos.y, p.voxel_size, p.voxel_size, q.y, fy, k.ry, k.v0y, k.v1y);
-  corner_pair(pos.z, p.voxel_size, p.voxel_size, q.z, fz, k.rz, k.v0z, k.v1z);
+  // corner_pair's test for the three axes together
+  const float half = 0.5f - 1e-6f * (fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) + 1.0f);
+  if (fabsf(k.rx - 0.5f) < half && fabsf(k.ry - 0.5f) < half && fabsf(k.rz - 0.5f) < half) {
+    k.v0x = (int)fx, k.v0y = (int)fy, k.v0z = (int)fz;
+    k.v1x = k.v0x + 1, k.v1y = k.v0y + 1, k.v1z = k.v0z + 1;
+  } else {
+    corner_pair(pos.x, vs, vs, q.x, fx, k.rx, k.v0x, k.v1x);
+    corner_pair(pos.y, vs, vs, q.y, fy, k.ry, k.v0y, k.v1y);
+    corner_pair(pos.z, vs, vs, q.z, fz, k.rz, k.v0z, k.v1z);
+  }
   return k;
 }
 
-// GetSpatialValue (geometry/spatial_query.h:23-66): trilinear sdf (and the
-// interpolated sqrt(1/inv_sigma2) when want_radius); false if any corner
-// block is missing.  The block of corner 0 is looked up first, so a sample
+// GetSpatialValue (geometry/spatial_query.h:23-66): trilinear sdf; false if any
+// corner block is missing.  The block of corner 0 is looked up first, so a sample
 // inside a block already known to be missing costs three divisions and one
 // cache compare; corners in other blocks go through a second cache entry.
-template <bool want_radius>
-__device__ __forceinline__ bool spatial_sample(const Dev &d, BlockCache &bc, F3 pos, float &sdf, float &radius,
+__device__ __forceinline__ bool spatial_sample(const Dev &d, BlockCache &bc, F3 pos, float &sdf,
                                                BlockCache *bc2 = nullptr) {
-  const float off = d.p.voxel_size;
-  const float vs = d.p.voxel_size;
-  const F3 q = in_voxels(d.p, pos);
-  const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
-  const float rx = q.x - fx, ry = q.y - fy, rz = q.z - fz;
-  int v0x, v0y, v0z, v1x, v1y, v1z;
-  corner_pair(pos.x, off, vs, q.x, fx, rx, v0x, v1x);
-  corner_pair(pos.y, off, vs, q.y, fy, ry, v0y, v1y);
-  corner_pair(pos.z, off, vs, q.z, fz, rz, v0z, v1z);
-  const int b0x = vox2blk(v0x), b0y = vox2blk(v0y), b0z = vox2blk(v0z);
+  const Corners k = corners_at(d.p, pos);
+  const int b0x = vox2blk(k.v0x), b0y = vox2blk(k.v0y), b0z = vox2blk(k.v0z);
   const int p0 = bc.get(d, b0x, b0y, b0z);
   if (p0 < 0) return false;
-  float s = 0.0f, rad = 0.0f;
+  float s = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int mx = (i & 4) > 0, my = (i & 2) > 0, mz = (i & 1) > 0;
-    const int vx = mx ? v1x : v0x, vy = my ? v1y : v0y, vz = mz ? v1z : v0z;
-    const float wx = mx ? rx : 1.0f - rx, wy = my ? ry : 1.0f - ry, wz = mz ? rz : 1.0f - rz;
+    const int vx = mx ? k.v1x : k.v0x, vy = my ? k.v1y : k.v0y, vz = mz ? k.v1z : k.v0z;
+    const float wx = mx ? k.rx : 1.0f - k.rx, wy = my ? k.ry : 1.0f - k.ry, wz = mz ? k.rz : 1.0f - k.rz;
     const int bx = vox2blk(vx), by = vox2blk(vy), bz = vox2blk(vz);
     int ptr = p0;
     if (bx != b0x || by != b0y || bz != b0z) {
@@ -407,23 +404,21 @@ __device__ __forceinline__ bool spatial_sample(const Dev &d, BlockCache &bc, F3 
     const size_t gi = (size_t)ptr * MH_BLOCK_VOXELS + li;
     const float w = wx * wy * wz;
     s += w * __ldg(d.sdf + gi);
-    if (want_radius) rad += w * sqrtf(1.0f / __ldg(d.w + gi));
   }
   sdf = s;
-  radius = rad;
   return true;
 }
 
 // GetSpatialSDFGradient (geometry/spatial_query.h:68-97)
 __device__ __forceinline__ bool spatial_gradient(const Dev &d, BlockCache &bc, F3 pos, F3 &g) {
   const float h = 0.5f * d.p.voxel_size;
-  float sp[3], sn[3], r;
+  float sp[3], sn[3];
 #pragma unroll 1
   for (int i = 0; i < 3; ++i) {
     F3 dm = f3(pos.x - (i == 0 ? h : 0.0f), pos.y - (i == 1 ? h : 0.0f), pos.z - (i == 2 ? h : 0.0f));
     F3 dp = f3(pos.x + (i == 0 ? h : 0.0f), pos.y + (i == 1 ? h : 0.0f), pos.z + (i == 2 ? h : 0.0f));
-    if (!spatial_sample<false>(d, bc, dm, sn[i], r)) return false;
-    if (!spatial_sample<false>(d, bc, dp, sp[i], r)) return false;
+    if (!spatial_sample(d, bc, dm, sn[i])) return false;
+    if (!spatial_sample(d, bc, dp, sp[i])) return false;
   }
   const float vs = d.p.voxel_size;
   g = f3((sp[0] - sn[0]) / vs, (sp[1] - sn[1]) / vs, (sp[2] - sn[2]) / vs);

@@ -396,7 +396,7 @@ __device__ __forceinline__ void mc_vertices_body(const Dev &d, Share sh) {
     float rad = 0.0f;
     bool rad_ok;
     {
-      const SampleAt k = sample_at(d.p, pos);
+      const Corners k = corners_at(d.p, pos);
       const bool mx = j & 4, my = j & 2, mz = j & 1;
       const int vx = mx ? k.v1x : k.v0x, vy = my ? k.v1y : k.v0y, vz = mz ? k.v1z : k.v0z;
       const int b = vb.get(d, vx, vy, vz);
@@ -411,7 +411,7 @@ __device__ __forceinline__ void mc_vertices_body(const Dev &d, Share sh) {
     }
     // sample j of the gradient: axis j / 2, minus side first
     const float h = 0.5f * vs, off = j & 1 ? h : -h;
-    const SampleAt k = sample_at(d.p, f3(pos.x + (j >> 1 == 0 ? off : 0.0f), pos.y + (j >> 1 == 1 ? off : 0.0f),
+    const Corners k = corners_at(d.p, f3(pos.x + (j >> 1 == 0 ? off : 0.0f), pos.y + (j >> 1 == 1 ? off : 0.0f),
                                          pos.z + (j >> 1 == 2 ? off : 0.0f)));
     bool ok = true;
     float v[8];

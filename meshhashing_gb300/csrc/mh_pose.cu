@@ -143,9 +143,9 @@ __global__ void __launch_bounds__(256) k_point_to_psdf(Dev d, Pose16 T, int ref_
       BlockCache bc, bc2;
       bc.init();
       bc2.init();
-      float s, r;
+      float s;
       F3 g;
-      if (spatial_sample<false>(d, bc, pw, s, r, &bc2) && spatial_gradient(d, bc, pw, g)) {
+      if (spatial_sample(d, bc, pw, s, &bc2) && spatial_gradient(d, bc, pw, g)) {
         const float J[6] = {g.x, g.y, ref_j ? g.x : g.z, -g.y * pw.z + g.z * pw.y, -g.z * pw.x + g.x * pw.z,
                             -g.x * pw.y + g.y * pw.x};
         int k = 0;

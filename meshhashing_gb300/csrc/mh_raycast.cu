@@ -73,8 +73,6 @@
 // valid one (PH_SCAN).
 namespace {
 
-enum { SM_OK = 0, SM_MISS0 = 1, SM_MISS0_NEW = 2, SM_MISS = 3 };
-
 struct Nbhd {
   static constexpr int LANES = 1;
   int bx, by, bz;    // block of the first corner of the last sample
@@ -113,35 +111,9 @@ template <int G> struct GroupNbhd {
   __device__ __forceinline__ unsigned of(unsigned ballot) const { return (ballot >> base) & ((1u << G) - 1u); }
 };
 
-// Corner voxels of GetSpatialValue at pos (both of each axis) and the
-// position's fractions.
-struct Corners {
-  int v0x, v0y, v0z, v1x, v1y, v1z;
-  float rx, ry, rz;
-};
-__device__ __forceinline__ Corners corners_at(const DevParams &p, F3 pos) {
-  Corners k;
-  const float vs = p.voxel_size;
-  const F3 q = in_voxels(p, pos);
-  const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
-  k.rx = q.x - fx, k.ry = q.y - fy, k.rz = q.z - fz;
-  // corner_pair's test for the three axes together
-  const float half = 0.5f - 1e-6f * (fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) + 1.0f);
-  if (fabsf(k.rx - 0.5f) < half && fabsf(k.ry - 0.5f) < half && fabsf(k.rz - 0.5f) < half) {
-    k.v0x = (int)fx, k.v0y = (int)fy, k.v0z = (int)fz;
-    k.v1x = k.v0x + 1, k.v1y = k.v0y + 1, k.v1z = k.v0z + 1;
-  } else {
-    corner_pair(pos.x, vs, vs, q.x, fx, k.rx, k.v0x, k.v1x);
-    corner_pair(pos.y, vs, vs, q.y, fy, k.ry, k.v0y, k.v1y);
-    corner_pair(pos.z, vs, vs, q.z, fz, k.rz, k.v0z, k.v1z);
-  }
-  return k;
-}
-
 // Block indices of the eight corners, corner i = 4 mx + 2 my + mz (m = 1: the
-// upper voxel of that axis).  SM_OK, SM_MISS0_NEW when the first corner's
-// block is missing (SM_MISS0 when that was known), SM_MISS when another is.
-__device__ __forceinline__ int blocks_at(const Dev &d, DenseNbhd &c, const Corners &k, int (&blk)[8]) {
+// upper voxel of that axis); false when one of the blocks is missing.
+__device__ __forceinline__ bool blocks_at(const Dev &d, DenseNbhd &c, const Corners &k, int (&blk)[8]) {
   const RayGrid &g = d.grid;
   c.bx = k.v0x >> 3, c.by = k.v0y >> 3, c.bz = k.v0z >> 3;
   // every sample of a ray lies inside the box; the clamps keep the loads there
@@ -150,19 +122,17 @@ __device__ __forceinline__ int blocks_at(const Dev &d, DenseNbhd &c, const Corne
   const unsigned z0 = min((unsigned)(c.bz - g.bz), g.bnz - 1u), z1 = min((unsigned)((k.v1z >> 3) - g.bz), g.bnz - 1u);
   const unsigned row[4] = {(z0 * g.bny + y0) * g.bnx, (z1 * g.bny + y0) * g.bnx, (z0 * g.bny + y1) * g.bnx,
                            (z1 * g.bny + y1) * g.bnx};
-  unsigned miss0 = 0, any = 0;
+  unsigned any = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const unsigned e = __ldg(g.blocks + row[i & 3] + ((i & 4) ? x1 : x0)) ^ g.tag;
-    if (i == 0) miss0 = e;
     any |= e;
     blk[i] = (int)(e & 0xffffffu);
   }
-  if (any < 0x1000000u) return SM_OK;
-  return miss0 < 0x1000000u ? SM_MISS : SM_MISS0_NEW;
+  return any < 0x1000000u;
 }
 
-__device__ __forceinline__ int blocks_at(const Dev &d, Nbhd &c, const Corners &k, int (&blk)[8]) {
+__device__ __forceinline__ bool blocks_at(const Dev &d, Nbhd &c, const Corners &k, int (&blk)[8]) {
   // VoxelToBlock: floor division by 8 (geometry_helper.h:82-90)
   const int b0x = k.v0x >> 3, b0y = k.v0y >> 3, b0z = k.v0z >> 3;
   if (b0x != c.bx || b0y != c.by || b0z != c.bz) {
@@ -175,8 +145,7 @@ __device__ __forceinline__ int blocks_at(const Dev &d, Nbhd &c, const Corners &k
   if (ey) need |= need << 2;
   if (ez) need |= need << 4;
   unsigned fresh = need & ~c.looked;
-  const bool b0_fresh = fresh & 1u;
-  if (b0_fresh) {
+  if (fresh & 1u) {
     const int b0 = hash_find(d, b0x, b0y, b0z);
     c.p[0] = b0;
     if (b0 >= 0 && d.touch) d.touch[b0] = 1;
@@ -184,7 +153,7 @@ __device__ __forceinline__ int blocks_at(const Dev &d, Nbhd &c, const Corners &k
     c.looked |= 1u;
     fresh &= ~1u;
   }
-  if (c.miss & 1u) return b0_fresh ? SM_MISS0_NEW : SM_MISS0;
+  if (c.miss & 1u) return false;
   while (fresh) {
     const int n = __ffs(fresh) - 1;
     fresh &= fresh - 1;
@@ -196,7 +165,7 @@ __device__ __forceinline__ int blocks_at(const Dev &d, Nbhd &c, const Corners &k
     if (bn < 0) c.miss |= 1u << n;
   }
   c.looked |= need;
-  if (need & c.miss) return SM_MISS;
+  if (need & c.miss) return false;
   // block of each corner (mx, my, mz): p[(mx & ex) | (my & ey) << 1 | (mz & ez) << 2]
   blk[0] = c.p[0];
   blk[4] = ex ? c.p[1] : blk[0];
@@ -206,18 +175,18 @@ __device__ __forceinline__ int blocks_at(const Dev &d, Nbhd &c, const Corners &k
   blk[5] = ez ? (ex ? c.p[5] : c.p[4]) : blk[4];
   blk[3] = ez ? (ey ? c.p[6] : c.p[4]) : blk[2];
   blk[7] = ez ? (ey ? (ex ? c.p[7] : c.p[6]) : (ex ? c.p[5] : c.p[4])) : blk[6];
-  return SM_OK;
+  return true;
 }
 
 // GetSpatialValue (geometry/spatial_query.h:23-66) with the same corners,
-// weights and summation order as spatial_sample.  Returns SM_OK with the
-// value in s (untouched when want is false), or why the sample is invalid.
+// weights and summation order as spatial_sample: the value in s (untouched when
+// want is false), or false for a sample that is invalid.
 template <class N>
-__device__ __forceinline__ int nb_sample(const Dev &d, N &c, F3 pos, bool want, float &s) {
+__device__ __forceinline__ bool nb_sample(const Dev &d, N &c, F3 pos, bool want, float &s) {
   const Corners k = corners_at(d.p, pos);
   int blk[8];
-  const int r = blocks_at(d, c, k, blk);
-  if (r != SM_OK || !want) return r;
+  if (!blocks_at(d, c, k, blk)) return false;
+  if (!want) return true;
   // local voxel coordinates of the two corners of each axis
   const int l0x = k.v0x & 7, l1x = k.v1x & 7;
   const int yz[4] = {(k.v0y & 7) * 8 + (k.v0z & 7) * 64, (k.v0y & 7) * 8 + (k.v1z & 7) * 64,
@@ -232,12 +201,12 @@ __device__ __forceinline__ int nb_sample(const Dev &d, N &c, F3 pos, bool want, 
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc += wxy[i >> 1] * ((i & 1) ? k.rz : w0z) * v[i];
   s = acc;
-  return SM_OK;
+  return true;
 }
 
 // 8 / G corners a lane; every lane of the group gets the result.
 template <int G>
-__device__ __forceinline__ int nb_sample(const Dev &d, GroupNbhd<G> &c, F3 pos, bool, float &s) {
+__device__ __forceinline__ bool nb_sample(const Dev &d, GroupNbhd<G> &c, F3 pos, bool, float &s) {
   const Corners k = corners_at(d.p, pos);
   const RayGrid &g = d.grid;
   float v[8 / G];
@@ -260,7 +229,7 @@ __device__ __forceinline__ int nb_sample(const Dev &d, GroupNbhd<G> &c, F3 pos, 
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc += __shfl_sync(c.lanes, v[i % (8 / G)], c.base + i / (8 / G));
   s = acc;
-  return ok ? SM_OK : SM_MISS;
+  return ok;
 }
 
 // One axis of a slab test with the direction's reciprocal: narrows [lo, hi]
@@ -538,25 +507,25 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
       if (phase == PH_REFINE) tp = m = l + (ls / (ls - rs)) * (r - l);
       const F3 pos = f3(cam.x + tp * wd.x, cam.y + tp * wd.y, cam.z + tp * wd.z);
       float s = 0.0f;
-      const int res = nb_sample(d, c, pos, phase != PH_SCAN, s);
+      const bool valid = nb_sample(d, c, pos, phase != PH_SCAN, s);
       if constexpr (N::LANES > 1) c.lanes = __ballot_sync(c.lanes, phase == PH_SCAN);
       bool refine = false, resume = false;  // start the regula falsi / go on after the negative sample at t
       if (phase == PH_MARCH) {
-        if (res == SM_OK && s < 0.0f && tl != NI && prev_t != tl) {
+        if (valid && s < 0.0f && tl != NI && prev_t != tl) {
           // negative after a sample that was not evaluated or is invalid
           cur_s = s, x = tl;
           phase = PH_PREV;
-        } else if (res == SM_OK && s < 0.0f && prev_t == tl && prev_sdf > 0.0f) {
+        } else if (valid && s < 0.0f && prev_t == tl && prev_sdf > 0.0f) {
           cur_s = s, l = prev_t, ls = prev_sdf;
           refine = true;
         } else {
-          if (res == SM_OK) prev_sdf = s, prev_t = t;
+          if (valid) prev_sdf = s, prev_t = t;
           tl = t;
           t += step;
           phase = PH_SEARCH;
         }
       } else if (phase == PH_PREV) {
-        if (res == SM_OK) {
+        if (valid) {
           // a crossing needs a positive sample before (ray_caster.cu:87-88)
           if (s > 0.0f) l = x, ls = s, refine = true;
           else resume = true;
@@ -571,7 +540,7 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
           else resume = true;
         }
       } else if (phase == PH_SCAN) {
-        if (res == SM_OK) l = x;
+        if (valid) l = x;
         x = skip_missing(d, c, cam, wd, step, x + step, tl);
         if (!(x < tl)) {
           const float first = prev_t != NI ? prev_t : t_min;
@@ -587,7 +556,7 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
         }
       } else {  // PH_REFINE
         bool last = true, hit = false;
-        if (res == SM_OK) {
+        if (valid) {
           if (ls * s > 0.0f) l = m, ls = s, side |= 1 << k;
           else r = m, rs = s;
           last = ++k == 3;
@@ -626,7 +595,7 @@ __device__ __forceinline__ March ray_march(const Dev &d, bool active, F3 cam, F3
       const float e = (k & 1) ? h : -h;
       const F3 pos = f3(k < 2 ? iso.x + e : iso.x, (k >> 1) == 1 ? iso.y + e : iso.y, k >= 4 ? iso.z + e : iso.z);
       float s = 0.0f;
-      if (nb_sample(d, c, pos, true, s) != SM_OK) out.g_ok = false;
+      if (!nb_sample(d, c, pos, true, s)) out.g_ok = false;
       if (!(k & 1)) {
         ls = s;
       } else {
@@ -929,7 +898,7 @@ struct SampleD {
 template <class N> __device__ __noinline__ bool ray_sample_d(const Dev &d, N &c, F3 pos, SampleD &o) {
   const float vs = d.p.voxel_size;
   const Corners k = corners_at(d.p, pos);
-  if (blocks_at(d, c, k, o.ptr) != SM_OK) return false;
+  if (!blocks_at(d, c, k, o.ptr)) return false;
   const float rx = k.rx, ry = k.ry, rz = k.rz;
   const float w0x = 1.0f - rx, w0y = 1.0f - ry, w0z = 1.0f - rz;
   float s = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
