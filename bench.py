@@ -157,11 +157,12 @@ def peaks():
         return 6800.0, "fallback"
 
 
-def bytes_per_launch(stage, nb, px, rpx, vwork, cube_blocks=0, mesh_blocks=0, predict_blocks=0, ray_blocks=None):
+def bytes_per_launch(stage, nb, px, rpx, vwork, cube_blocks=0, mesh_blocks=0, predict_blocks=0, ray_blocks=None,
+                     update_blocks=None):
     """Algorithmic bytes one launch of a stage must move (per-frame averages of
     the blocks each kernel actually visits, counted on the device)."""
-    if stage == "integrate":       # sdf, inv_sigma2, a, b read+write; depth + inlier images
-        return nb * 512 * 32 + px * 8
+    if stage == "integrate":       # sdf, inv_sigma2, a, b of the blocks it goes over read+write; depth + inlier images
+        return (update_blocks if update_blocks is not None else nb) * 512 * 32 + px * 8
     if stage == "predict":         # vertex slots of blocks with vertices; the inlier image
         return predict_blocks * 512 * 12 + px * 4
     if stage == "raycast":         # 2 KB sdf + 16 B entry per block the rays touch; depth, vertex, normal out
@@ -745,7 +746,8 @@ def main():
     counts = {"cube_blocks": (s1["cube_blocks_sum"] - s0["cube_blocks_sum"]) / passes,
               "mesh_blocks": (s1["mesh_list_sum"] - s0["mesh_list_sum"]) / passes,
               "predict_blocks": (s1["predict_blocks_sum"] - s0["predict_blocks_sum"]) / passes,
-              "ray_blocks": ray_blocks}
+              "ray_blocks": ray_blocks,
+              "update_blocks": ((s1["update_blocks"] - s0["update_blocks"]) % (1 << 32)) / passes}
     px, rpx = Ww * Hh, params.rc_width * params.rc_height
     peak, peak_kind = peaks()
     stage_ms = {k: v[0] for k, v in prof.items()}
@@ -754,19 +756,17 @@ def main():
     per_launch_ms = stage_ms[dom] / calls
     alg = bytes_per_launch(dom, nb, px, rpx, vwork, **counts)
     achieved = alg / (per_launch_ms / 1000.0) / 1e9
-    # DRAM bytes per launch measured by ncu (dram__bytes_read.sum + _write.sum,
-    # --set full) on this workload's 10-frame map (frame 9: 274,742 candidate
-    # blocks, 143,854 of them looked up by rays), scaled to this run by the
-    # units the kernel's traffic follows: blocks the rays look up for the
-    # raycast, candidate blocks for the integrate
-    NCU_TRAFFIC = {"raycast": (116.87e6, 143854.0, "ray_blocks", "blocks looked up by rays"),
-                   "integrate": (1780.52e6, 274742.0, "candidates", "candidate blocks")}
+    # DRAM bytes of the stage's kernels in one frame measured by ncu
+    # (dram__bytes_read.sum + _write.sum) on this workload's 10-frame map (frame 9:
+    # 169,310 blocks in the update, 108,212 blocks looked up by rays;
+    # profiles/dram_psdf640_frame9.md), scaled to this run by those counts
+    NCU_TRAFFIC = {"raycast": (50.85e6, 108212.0, "ray_blocks", "blocks looked up by rays"),
+                   "integrate": (1821.9e6, 169310.0, "update_blocks", "blocks in the update")}
     traffic, traffic_src = None, None
     if dom in NCU_TRAFFIC:
         b0, n0, unit, what = NCU_TRAFFIC[dom]
-        n1 = ray_blocks if unit == "ray_blocks" else nb
-        traffic = b0 * n1 / n0
-        traffic_src = ("ncu DRAM read+write of one launch at %d %s (frame 9 of this workload, 10-frame map), "
+        traffic = b0 * counts[unit] / n0
+        traffic_src = ("ncu DRAM read+write of one frame at %d %s (frame 9 of this workload, 10-frame map), "
                        "scaled by %s" % (int(n0), what, what))
     stages = {}
     for k, (t_ms, c) in prof.items():

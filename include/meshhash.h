@@ -105,6 +105,8 @@ typedef struct mh_stats {
   uint64_t mesh_list_sum;         /* blocks walked by the triangle and recycle passes */
   uint64_t predict_blocks_sum;    /* blocks the inlier prediction read */
   uint32_t mesh_pages_used;       /* mesh pages held by blocks */
+  uint32_t update_blocks;         /* blocks that PSDF updates went over since
+                                     reset, modulo 2^32 */
 } mh_stats;
 
 typedef struct mh_volume mh_volume;

@@ -36,7 +36,7 @@ class MhStats(C.Structure):
         "triangles_allocated", "overflow_used", "frames", "dropped_inserts", "gc_freed_blocks",
         "mesh_passes")] + [(n, C.c_uint64) for n in (
         "candidate_sum", "vertex_work_sum", "cube_blocks_sum", "mesh_list_sum", "predict_blocks_sum")] + [
-        ("mesh_pages_used", _u32)]
+        ("mesh_pages_used", _u32), ("update_blocks", _u32)]
 
     def as_dict(self):
         return {k: getattr(self, k) for k, _ in self._fields_}

@@ -270,6 +270,7 @@ template <bool kPlanned> __device__ __forceinline__ void integrate_psdf_body(con
   const int n = *reinterpret_cast<volatile int *>(kPlanned ? &d.ctr->upd_count : &d.ctr->cand_count);
   const int4 *list = kPlanned ? d.upd_list : d.cand;
   const int t = threadIdx.x;
+  if (sh.first == 0 && t == 0) d.ctr->upd_sum += (unsigned)n;
   const int lx = (t & 1) * 4, ly = (t >> 1) & 7, lz = t >> 4;
   int4 next = sh.first < n ? list[sh.first] : make_int4(0, 0, 0, -1);
   for (int c = sh.first; c < n; c += sh.stride) {

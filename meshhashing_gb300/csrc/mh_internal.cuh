@@ -65,6 +65,7 @@ struct Counters {
   int cube_list_count; // candidates the cube pass must tile this pass
   int vtx_list_count;  // candidates owning vertices (inlier prediction)
   int upd_count;       // candidates that the PSDF update may change
+  unsigned upd_sum;    // blocks that PSDF updates went over, modulo 2^32
   unsigned long long cand_sum;   // sum of candidate counts over mesh calls
   unsigned long long vwork_sum;  // sum of computed vertices over mesh calls
   unsigned long long cube_blocks_sum;     // blocks the cube pass loaded a tile for

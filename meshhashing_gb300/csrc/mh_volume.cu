@@ -697,6 +697,7 @@ int mh_stats_get(mh_volume *v, mh_stats *out, void *stream) {
   out->mesh_list_sum = c.mesh_list_sum;
   out->predict_blocks_sum = c.predict_blocks_sum;
   out->mesh_pages_used = (uint32_t)(v->d.page_capacity - c.page_top);
+  out->update_blocks = c.upd_sum;
   return MH_OK;
 }
 
