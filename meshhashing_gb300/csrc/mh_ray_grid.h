@@ -18,6 +18,7 @@
 // the view's bounding box.  A word holds 4 x 4 x 2 cells, so with U = 2 two
 // words hold a block (mh_raycast.cu).
 #define MH_GRID_BIAS 49152.0f        // 1.5 * 2^15: a float there has 8 bits of fraction
+#define MH_GRID_GUARD 0.03125f       // cells that a sample is looked up below its position, at least
 #define MH_GRID_MAX_WORDS (1u << 25) // 128 MB
 #define MH_GRID_REPLAY_TAG 255u      // top byte of blocks written by replayed raycasts
 struct RayGrid {
@@ -26,10 +27,8 @@ struct RayGrid {
   unsigned nx, ny, nz;       // words on each axis
   unsigned words;            // nx * ny * nz
   int shift;                 // U = 2 << shift
-  float ox, oy, oz;          // world position of the first cell's lower corner
+  float ox, oy, oz;          // world position of the first cell's lower corner, and the guard above MH_GRID_GUARD
   float inv_cell;            // 1 / (U voxel sizes)
-  float guard;               // samples' cells are taken this far (in cells) below their position
-  int reach;                 // a group of 2^3 voxels marks the cells down to that of the reach-th group below it
   // The blocks of the same box: entry (z bny + y) bnx + x holds tag | block
   // index for a block that exists, anything with another top byte otherwise.
   unsigned *blocks;          // null: blocks are looked up in the hash table
@@ -38,6 +37,7 @@ struct RayGrid {
   unsigned tag;              // this raycast's top byte, 1 .. 254, or MH_GRID_REPLAY_TAG
   unsigned clear;            // entries to clear first (all that the buffer has), 0 where old ones cannot be mistaken
   bool filled;               // the buffers hold this grid already
+  short reach;               // a group of 2^3 voxels marks the cells down to that of the reach-th group below it
 };
 
 // A volume's buffers for its view's grid, of sizes for any view.  They come with
@@ -140,7 +140,8 @@ MH_GRID_HD inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], co
   for (int shift = 0; shift < 12; ++shift) {
     const int U = 2 << shift;
     const double cell = (double)U * (double)P.voxel_size;
-    const double e = far / (cell * 2097152.0) + 0.0078125, guard = e <= 0.015625 ? 0.03125 : e;
+    const double e = far / (cell * 2097152.0) + 0.0078125;
+    const double guard = std::max(e, (double)MH_GRID_GUARD);
     if (!(guard + e < 1.0)) continue;
     const int reach = 1 + ((int)(U * (guard + e)) + 1) / 2;
     if (reach > (1 << shift)) continue;
@@ -156,10 +157,10 @@ MH_GRID_HD inline RayGrid ray_grid_of(const mh_params &P, const double lo[3], co
     g.nx = (unsigned)n[0], g.ny = (unsigned)n[1], g.nz = (unsigned)n[2];
     g.words = g.nx * g.ny * g.nz;
     g.shift = shift;
-    g.ox = (float)(c[0] * cell), g.oy = (float)(c[1] * cell), g.oz = (float)(c[2] * cell);
+    const double more = guard - MH_GRID_GUARD;
+    g.ox = (float)((c[0] + more) * cell), g.oy = (float)((c[1] + more) * cell), g.oz = (float)((c[2] + more) * cell);
     g.inv_cell = (float)(1.0 / cell);
-    g.guard = (float)guard;
-    g.reach = reach;
+    g.reach = (short)reach;
     break;
   }
   // a block around the box: corners and gradient samples reach past a ray

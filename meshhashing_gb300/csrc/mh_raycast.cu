@@ -279,9 +279,9 @@ struct GridRay {
 };
 __device__ __forceinline__ GridRay grid_ray(const RayGrid &g, F3 cam, F3 wd) {
   GridRay r;
-  r.ox = (cam.x - g.ox) * g.inv_cell - g.guard + MH_GRID_BIAS;
-  r.oy = (cam.y - g.oy) * g.inv_cell - g.guard + MH_GRID_BIAS;
-  r.oz = (cam.z - g.oz) * g.inv_cell - g.guard + MH_GRID_BIAS;
+  r.ox = (cam.x - g.ox) * g.inv_cell - MH_GRID_GUARD + MH_GRID_BIAS;
+  r.oy = (cam.y - g.oy) * g.inv_cell - MH_GRID_GUARD + MH_GRID_BIAS;
+  r.oz = (cam.z - g.oz) * g.inv_cell - MH_GRID_GUARD + MH_GRID_BIAS;
   r.dx = wd.x * g.inv_cell, r.dy = wd.y * g.inv_cell, r.dz = wd.z * g.inv_cell;
   return r;
 }
@@ -707,8 +707,9 @@ int launch_raycast_batch(const Scene *t, int n, int total, int shape, cudaStream
 // Bound by the scattered writes and atomics; 640x480, 4 mm, 461 k blocks, half
 // of them marked: 41 us (cold), of 390 us for the raycast with it.  Cells of 4
 // voxels cost less here (14 us) and more in the march, which then evaluates 6.4
-// samples a ray instead of 3.4 (507 us in all).
-__device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
+// samples a ray instead of 3.4 (507 us in all).  kFar: a reach above 1, marked cell
+// by cell.
+template <bool kFar> __device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
   const RayGrid &g = d.grid;
   if (!g.bits) return;
   const int n = *reinterpret_cast<volatile int *>(&d.ctr->high_water);
@@ -722,7 +723,7 @@ __device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
     }
     const unsigned long long m = __ldg(d.neg + i);
     if (!m) continue;
-    if (g.reach > 1) {
+    if (kFar) {
       // large cells, or far from the origin: all cells from the reach below the
       // block's first marked group to its last, on each axis; at most 27 (U = 4)
       unsigned p = (unsigned)(m | m >> 32);
@@ -772,10 +773,13 @@ __device__ __forceinline__ void ray_grid_body(const Dev &d, Share sh) {
     }
   }
 }
-__global__ void __launch_bounds__(256) k_ray_grid(Dev d) { ray_grid_body(d, whole_grid()); }
-__global__ void __launch_bounds__(256) k_ray_grid_b(const Scene *t, int n) {
+template <bool kFar> __global__ void __launch_bounds__(256) k_ray_grid(Dev d) { ray_grid_body<kFar>(d, whole_grid()); }
+__global__ void __launch_bounds__(256, 5) k_ray_grid_b(const Scene *t, int n) {
   each_scene(t, n, 256, [&](const Scene &c) { return c.d.grid.bits ? count_of(c.d, &Counters::high_water) : 0; },
-             [&](const Scene &c, Share sh) { ray_grid_body(c.d, sh); });
+             [&](const Scene &c, Share sh) {
+    if (c.d.grid.reach > 1) ray_grid_body<true>(c.d, sh);
+    else ray_grid_body<false>(c.d, sh);
+  });
 }
 __global__ void __launch_bounds__(256) k_ray_grid_clear_b(const Scene *t, int n) {
   each_scene(t, n, 256, [&](const Scene &c) { return c.d.grid.bits ? (int)max(c.d.grid.words, c.d.grid.clear) : 0; },
@@ -792,7 +796,8 @@ static int fill_ray_grid(const Dev &d, cudaStream_t s) {
   MH_CUDA_TRY(cudaMemsetAsync(d.grid.bits, 0, sizeof(unsigned) * (size_t)d.grid.words, s));
   if (d.grid.clear)
     MH_CUDA_TRY(cudaMemsetAsync(d.grid.blocks, 0, sizeof(unsigned) * (size_t)d.grid.clear, s));
-  k_ray_grid<<<mh_sm_count() * 8, 256, 0, s>>>(d);
+  if (d.grid.reach > 1) k_ray_grid<true><<<mh_sm_count() * 8, 256, 0, s>>>(d);
+  else k_ray_grid<false><<<mh_sm_count() * 8, 256, 0, s>>>(d);
   mh_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? MH_OK : MH_ERR_CUDA;
 }
