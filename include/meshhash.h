@@ -164,8 +164,9 @@ int mh_gc_collect_garbage(mh_volume *v, void *stream);
  * point (x, y, z, 1), normal = camera-frame -grad(sdf) / |grad| (x, y, z, 1);
  * misses are -inf.  Width x height = rc_width x rc_height.  A volume's first
  * raycast, of whatever kind, allocates a grid of the view, up to 384 MB by the
- * view's size in voxels (a batch with raycasts: when it is created); without
- * memory for it the raycast is slower, with the same images.  Replays of a
+ * view's size in voxels (a batch with raycasts: when it is created; volumes of 16
+ * times that and more: with the volume); without memory for it the raycast is
+ * slower, with the same images.  Replays of a
  * captured call with device outputs take the volume's pose and map of then. */
 int mh_raycast(mh_volume *v, const float cTw[16], float *depth, float *vertex4,
                float *normal4, int out_on_device, void *stream);

@@ -41,7 +41,8 @@ struct RayGrid {
 };
 
 // A volume's buffers for its view's grid, of sizes for any view.  They come with
-// the first raycast: up to 384 MB, of which a volume that casts no rays has no use.
+// the first raycast, since they are up to 384 MB that a volume without raycasts has
+// no use for, but with the volume where they are a small part of it.
 struct RayGridBuf {
   bool reserved = false;
   unsigned *bits = nullptr, *blocks = nullptr;
@@ -76,6 +77,13 @@ inline void ray_grid_sizes(const mh_params &P, RayGridBuf &b) {
   const double words = std::min(cells / 4.0 * (cells / 4.0) * (cells / 2.0),
                                 (b.entries ? 128.0 : 256.0) * P.rc_width * P.rc_height);
   b.words = std::max((unsigned)std::min(words, (double)MH_GRID_MAX_WORDS), 4096u);
+}
+
+// Whether they take at most a sixteenth of what the voxels take.
+inline bool ray_grid_small(const mh_params &P) {
+  RayGridBuf b;
+  ray_grid_sizes(P, b);
+  return 4.0 * ((double)b.words + b.entries) <= P.value_capacity * 8192.0 / 16.0;
 }
 
 // The buffers' memory, from alloc(words) (null: there is none), asked for once.

@@ -431,6 +431,7 @@ int mh_volume_create(const mh_params *p, mh_volume **out) {
   d.pixels = reinterpret_cast<float4 *>(v->tv);
   d.tile_far = reinterpret_cast<unsigned *>(v->tv + 4 * (size_t)P.width * P.height);
   A(dalloc(v, &v->rc_stage, rpix * 9 + 3));
+  if (r == MH_OK && ray_grid_small(P)) ray_grid_ready(v);
   if (r == MH_OK) r = mh_volume_reset(v, nullptr);
   if (r != MH_OK) {
     mh_volume_destroy(v);

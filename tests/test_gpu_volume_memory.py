@@ -1,4 +1,5 @@
-"""The memory of the view's grid comes with the first raycast.
+"""The memory of the view's grid comes with the first raycast, where it is not a
+small part of the volume's.
 
 Two volumes that differ in the raycast's depth only: the farther view's grid is
 larger by tens of megabytes, which a volume takes when it casts rays, not before,
