@@ -759,7 +759,7 @@ def main():
     # DRAM bytes of the stage's kernels in one frame measured by ncu
     # (dram__bytes_read.sum + _write.sum) on this workload's 10-frame map (frame 9:
     # 169,310 blocks in the update, 108,212 blocks looked up by rays;
-    # profiles/dram_psdf640_frame9.md), scaled to this run by those counts
+    # profiles/frame9_psdf640.md), scaled to this run by those counts
     NCU_TRAFFIC = {"raycast": (50.85e6, 108212.0, "ray_blocks", "blocks looked up by rays"),
                    "integrate": (1821.9e6, 169310.0, "update_blocks", "blocks in the update")}
     traffic, traffic_src = None, None

@@ -252,7 +252,7 @@ __device__ __forceinline__ float pd_huber(float n2) {
 }
 
 // PrimalDualInit: weights from the gradient, the iterate's start.  Bound by the
-// traffic, 36 B a voxel and the faces: 480 us for 120 k blocks, where a thread a
+// traffic, 36 B a voxel and the faces: 490 us for 120 k blocks, where a thread a
 // voxel took 508.
 __global__ void __launch_bounds__(128) k_pd_init(Dev d, PD pd, const int *nbt, unsigned *fresh) {
   __shared__ Tile9 sdf, weight;
