@@ -212,7 +212,7 @@ bool mh_capturing(cudaStream_t s) {
 }
 
 void ray_grid_sent(mh_volume *v, const RayGrid &g, cudaStream_t s) {
-  if (!mh_capturing(s)) ray_grid_enqueued(v->grid, g);
+  if (v->grid.dirty && !mh_capturing(s)) ray_grid_enqueued(v->grid, g);
 }
 
 void ray_grid_ready(mh_volume *v) {
